@@ -21,6 +21,8 @@ EXE = os.path.join(OUT, "mtgpu_cocr_fp")
 
 CU_SOURCES = ["sell.cu", "folded.cu", "cocr.cu", "assemble.cu", "survey.cu", "capi.cu", "capi_assembly.cu",
               "noalloc.cu", "receivers.cu", "adjoint.cu", "smoothing.cu", "regular_mesh.cu", "scan.cu"]
+# the survey solver's kernels, one object per lane count (survey_sp.cu)
+SURVEY_LANES = (32, 16, 8, 4, 2, 1)
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -48,12 +50,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     headers.append(os.path.join(ROOT, "include", "mtgpu.h"))
     objs, jobs = [], []
-    for s in CU_SOURCES:
-        src = os.path.join(CSRC, s)
-        obj = os.path.join(OUT, s.replace(".cu", ".o"))
+    units = [("survey_sp.cu", f"survey_sp{n}.o", [f"-DMTGPU_SURVEY_SP={n}"]) for n in SURVEY_LANES]
+    units += [(s, s.replace(".cu", ".o"), []) for s in CU_SOURCES]
+    for s, o, defs in units:
+        src, obj = os.path.join(CSRC, s), os.path.join(OUT, o)
         objs.append(obj)
         if force or _stale(obj, [src] + headers):
-            jobs.append([nvcc()] + _flags() + ["-c", src, "-o", obj])
+            jobs.append([nvcc()] + _flags() + defs + ["-c", src, "-o", obj])
     with cf.ThreadPoolExecutor(max_workers=max(1, min(len(jobs), os.cpu_count() or 4))) as ex:
         for cmd, res in zip(jobs, ex.map(lambda c: subprocess.run(c, capture_output=True, text=True), jobs)):
             if res.returncode != 0:

@@ -140,5 +140,50 @@ __host__ __device__ __forceinline__ df from_double(double v)
     return df{h, (float)(v - (double)h)};
 }
 
+// ---- sums across threads
+// A partial sum as three FP32 numbers a + b + c.  Adding two of them with
+// two-sums on a and b keeps more than 60 bits (the error is that of c, about
+// 2^-70 of the larger operand), more than FP64's 53, in 21 FP32 operations:
+// GB300 issues an FP64 add of a warp once in 16 cycles, so the FP64 trees
+// over 256 threads that these sums replace took most of a small kernel.
+// FP32's range is the limit of a and not FP64's: sums that could overflow are
+// carried scaled by 2^-64 (float4 form, w = 1).
+struct tf {
+    float a, b, c;
+};
+__device__ __forceinline__ tf tf_add(tf x, tf y)
+{
+    float s, e, t, f, u, g;
+    two_sum(x.a, y.a, s, e);
+    two_sum(x.b, y.b, t, f);
+    two_sum(e, t, u, g);
+    return tf{s, u, __fadd_rn(__fadd_rn(x.c, y.c), __fadd_rn(f, g))};
+}
+__device__ __forceinline__ tf tf_scale(tf x, float s) { return tf{x.a * s, x.b * s, x.c * s}; }
+__device__ __forceinline__ tf tf_of(const acc &x) { return tf{x.h, x.l, 0.f}; }
+__device__ __forceinline__ tf tf_of(double v)
+{
+    const float a = (float)v;
+    const double r = v - (double)a;
+    const float b = (float)r;
+    return tf{a, b, (float)(r - (double)b)};
+}
+constexpr float kTfBig = 0x1p100f, kTfDown = 0x1p-64f;
+__device__ __forceinline__ float4 tf_pack(tf x, float w) { return make_float4(x.a, x.b, x.c, w); }
+__device__ __forceinline__ float4 tf4_add(float4 x, float4 y)
+{
+    tf u{x.x, x.y, x.z}, v{y.x, y.y, y.z};
+    if (x.w != y.w) {
+        if (x.w == 0.f) u = tf_scale(u, kTfDown);
+        else v = tf_scale(v, kTfDown);
+    }
+    return tf_pack(tf_add(u, v), fmaxf(x.w, y.w));
+}
+__device__ __forceinline__ double tf4_double(float4 x)
+{
+    const double v = (double)x.x + ((double)x.y + (double)x.z);
+    return x.w == 0.f ? v : v * 0x1p64;
+}
+
 }  // namespace dfl
 }  // namespace mtgpu

@@ -118,7 +118,7 @@ template <int SP>
 __global__ void __launch_bounds__(MfTile<SP>::NT, 1)
 k_mf_tile(MF M, MfTileGrid G, const float2 *__restrict__ omega, const float4 *__restrict__ s,
           float4 *__restrict__ z,
-          SysState *sys, double *partials, int mode)
+          SysState *sys, float4 *partials, int mode)
 {
     pdl_wait();
     using C = MfTile<SP>;
@@ -373,12 +373,13 @@ k_mf_tile(MF M, MfTileGrid G, const float2 *__restrict__ omega, const float4 *__
     red[tid] = tail.zsr.to_double();
     red[NT + tid] = tail.zsi.to_double();
     __syncthreads();
-    double v[2] = {0.0, 0.0};
+    double d[2] = {0.0, 0.0};
     if (tid < SP) {
         const int u = tid - sys0;
         if (u >= 0 && u < SB)
             for (int n = 0; n < 2; n++)
-                for (int t = u * CPS; t < (u + 1) * CPS; t++) v[n] += red[n * NT + t];
+                for (int t = u * CPS; t < (u + 1) * CPS; t++) d[n] += red[n * NT + t];
     }
+    const tf v[2] = {tf_of(d[0]), tf_of(d[1])};
     SpmvTail::finish_v<SP, NT>(v, sys, partials, mode);
 }

@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(PrecTile<SP>::NT)
 k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__restrict__ da,
             const float4 *__restrict__ s, const float4 *__restrict__ z,
             const float4 *__restrict__ a_in, float4 *__restrict__ a_out, float4 *__restrict__ p,
-            float4 *__restrict__ w, float4 *__restrict__ x, SysState *sys, double *partials)
+            float4 *__restrict__ w, float4 *__restrict__ x, SysState *sys, float4 *partials)
 {
     pdl_wait();
     using C = PrecTile<SP>;
@@ -78,8 +78,8 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
     const int tid = threadIdx.x;
     const int u_me = tid / (TX * TY), ti = tid % TX, tj = (tid / TX) % TY;
     // beta of the block's systems (two at most), selected without indexing
-    const dfc be0 = from_d2(sys[sys0].beta);
-    const dfc be1 = SB > 1 ? from_d2(sys[sys0 + SB - 1].beta) : be0;
+    const dfc be0 = from4(sys[sys0].beta_f);
+    const dfc be1 = SB > 1 ? from4(sys[sys0 + SB - 1].beta_f) : be0;
     auto beta_of = [&](int u) { return u ? be1 : be0; };
 
     // a_new of the edges owned by the nodes of plane P (x, y on P; z of
@@ -141,7 +141,7 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
     const dfc bme = beta_of(u_me);
     // the previous iteration's x += alpha p, as in k_edge
     const bool xpme = sys[kme].xp;
-    const dfc alme = from_d2(sys[kme].alpha);
+    const dfc alme = from4(sys[kme].alpha_f);
     const bool col = i < nx && j < ny && sys[kme].status == kRun;
     acc awr, awi;
     for (int k = k0; k < k1; k++) {
@@ -198,22 +198,23 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
     red[tid] = awr.to_double();
     red[NT + tid] = awi.to_double();
     __syncthreads();
-    double v[2] = {0.0, 0.0};
+    double d[2] = {0.0, 0.0};
     if (tid < SP) {
         const int u = tid - sys0;
         if (u >= 0 && u < SB)
             for (int t = u * TX * TY; t < (u + 1) * TX * TY; t++) {
-                v[0] += red[t];
-                v[1] += red[NT + t];
+                d[0] += red[t];
+                d[1] += red[NT + t];
             }
     }
+    const tf v[2] = {tf_of(d[0]), tf_of(d[1])};
     __shared__ double tot[2][32];
-    if (sys_grid_sum<SP, 2, NT>(v, partials, &sys[0].ticket[1], tot) && threadIdx.x < SP) {
+    if (sys_grid_sum<SP, 2, NT>(v, partials, tot) && threadIdx.x < SP) {
         SysState &q = sys[threadIdx.x];
         if (q.status == kRun) {
             const double2 aw = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
             if (fabs(aw.x) < 1e-40 && fabs(aw.y) < 1e-40) q.status = MTGPU_DIV_BY_ZERO;
-            else q.alpha = cdiv(q.zs, aw);
+            else set_alpha(q, cdiv(q.zs, aw));
         }
     }
 }

@@ -6,12 +6,14 @@ namespace mtgpu {
 
 // per-system state, read and written by the kernels' last blocks
 struct SysState {
+    float4 alpha_f, beta_f;    // alpha and beta as double-float (what the row kernels multiply by)
     double2 zs, alpha, beta;
     double r_old;          // ||b||
     double residual;       // ||s_m|| (MRS-smoothed residual)
     double residual_rel;   // residual / r_old: the reference's stop quantity
     double true_rel;       // ||b - A x|| / ||b|| of the last verification
     double mrs_w;
+    float2 mrs_wf;         // mrs_w as double-float
     double eps_k;          // the inner stop threshold on residual_rel
     double bnorm;          // ||b|| of the system (FP64)
     double rnorm;          // ||b - A x|| of the last FP64 residual evaluation
@@ -93,7 +95,7 @@ struct Survey {
     float4 *a2 = nullptr;
     double2 *b64 = nullptr, *xacc = nullptr;      // FP64 b and accumulated x: [row][SP]
     int *all_on = nullptr;                        // 32 flags, all set
-    double *partials = nullptr;
+    float4 *partials = nullptr;                   // tickets, then block and group partials (sys_grid_sum)
     int pblocks = 0;                              // blocks the partial-sum buffer holds
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
