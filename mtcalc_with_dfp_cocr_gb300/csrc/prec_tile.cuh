@@ -1,7 +1,7 @@
 // The folded preconditioner of the iteration in one kernel on tensor meshes,
 // included by survey.cu after k_node / k_edge.
 //
-// k_node (h = D_S G (z + beta a)) and k_edge (p = s + beta p, a = z + beta a,
+// k_node (h = D_S G (z + beta a)) and k_edge (a = z + beta a,
 // w = D_A a + G^T h, (a, w)) are two passes over the vectors with h in
 // global memory between them.  On a tensor mesh numbered as
 // RegularMeshBuilder numbers it, with every interior node a row of G (in
@@ -10,14 +10,14 @@
 // both: a block owns a tile of TX x TY node columns and marches along z;
 // per plane it stages a_new = z + beta a of the edges owned by the plane's
 // nodes (tile plus a one-node halo), computes h of the plane's nodes (tile
-// plus one on the + side) into shared memory, and produces p, a, w of the
+// plus one on the + side) into shared memory, and produces a, w of the
 // edges owned by the previous plane's nodes.  Every vector crosses HBM once;
 // h never leaves the SM.
 //
 // a is read (a_in) and written (a_out) in different buffers: the halo of a
 // tile reads a neighbour tile's edges.  The sums run in the order of k_node
 // (a node's edges by increasing number: -z, -y, -x, +x, +y, +z) and k_edge
-// (D_A a, then the first node's -1/2 h, then the second's +1/2 h), so p, a
+// (D_A a, then the first node's -1/2 h, then the second's +1/2 h), so a
 // and w equal the two-kernel form's to the last bit; the grid sum (a, w)
 // groups its terms by tile and so rounds differently.
 
@@ -45,9 +45,9 @@ struct PrecGrid {
 template <int SP>
 __global__ void __launch_bounds__(PrecTile<SP>::NT)
 k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__restrict__ da,
-            const float4 *__restrict__ s, const float4 *__restrict__ z,
-            const float4 *__restrict__ a_in, float4 *__restrict__ a_out, float4 *__restrict__ p,
-            float4 *__restrict__ w, float4 *__restrict__ x, SysState *sys, float4 *partials)
+            const float4 *__restrict__ z, const float4 *__restrict__ a_in,
+            float4 *__restrict__ a_out, float4 *__restrict__ w, SysState *sys, float4 *partials,
+            int first)
 {
     pdl_wait();
     using C = PrecTile<SP>;
@@ -138,10 +138,6 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
     const int ii = ti + 1, jj = tj + 1;
     const int i = i0 + ti, j = j0 + tj;
     const int kme = sys0 + u_me;
-    const dfc bme = beta_of(u_me);
-    // the previous iteration's x += alpha p, as in k_edge
-    const bool xpme = sys[kme].xp;
-    const dfc alme = from4(sys[kme].alpha_f);
     const bool col = i < nx && j < ny && sys[kme].status == kRun;
     acc awr, awi;
     for (int k = k0; k < k1; k++) {
@@ -156,7 +152,7 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
             for (int d = 0; d < 3; d++) {
                 if (!(d == 0 ? ex : (d == 1 ? ey : ezp))) continue;
                 const long long idx = (long long)(base + (d == 0 ? 0 : (d == 1 ? ex : ex + ey))) * SP + kme;
-                const float4 srcv = __ldg(s + idx), dav = __ldg(da + idx), pv = p[idx];
+                const float4 dav = __ldg(da + idx);
                 const dfc an = from4(d == 0 ? axy(k, 0, ii, jj, u_me)
                                             : (d == 1 ? axy(k, 1, ii, jj, u_me) : az(k, ii, jj, u_me)));
                 // the edge's nodes: (i, j, k) first, its +d neighbour second;
@@ -168,8 +164,6 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
                 const float4 h0 = hh(k, ii, jj, u_me);
                 const float4 h1 = d == 2 ? hh(k + 1, ii, jj, u_me)
                                          : hh(k, ii + (d == 0), jj + (d == 1), u_me);
-                if (xpme) x[idx] = to4(caxpy(from4(x[idx]), alme, from4(pv)));
-                p[idx] = to4(caxpy(from4(srcv), bme, from4(pv)));
                 a_out[idx] = to4(an);
                 const dfc dv = cmul(an, from4(dav));
                 acc wr, wi;
@@ -211,6 +205,7 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
     __shared__ double tot[2][32];
     if (sys_grid_sum<SP, 2, NT>(v, partials, tot) && threadIdx.x < SP) {
         SysState &q = sys[threadIdx.x];
+        if (first) q.cnt = 0;
         if (q.status == kRun) {
             const double2 aw = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
             if (fabs(aw.x) < 1e-40 && fabs(aw.y) < 1e-40) q.status = MTGPU_DIV_BY_ZERO;

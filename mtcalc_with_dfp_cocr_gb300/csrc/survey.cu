@@ -22,10 +22,10 @@
 // residual ||b - A x|| / ||b|| is computed in FP64 and, if `verify` is set and
 // it is not below eps, the system keeps iterating or restarts on its FP64
 // residual (iterative refinement, FP64 solution).  One iteration is the node
-// gather, the edge gather + (a, w) (with the previous iteration's x += alpha
-// p), the updates + the MRS smoothing, and the SpMV + (z, s) (one kernel for
-// a stored matrix, two for the matrix-free forms), captured in a CUDA graph
-// several iterations at a time; all per-system decisions are taken on the
+// gather, the edge gather + (a, w), the updates + the MRS smoothing, and the
+// SpMV + (z, s) (one kernel for a stored matrix, two for the matrix-free
+// forms), captured in a CUDA graph several iterations at a time, with p and x
+// brought up to date once per group of iterations; all per-system decisions are taken on the
 // device by the block of each kernel that finishes last.
 #include "survey_impl.cuh"
 
@@ -49,10 +49,10 @@ void Survey::release()
     dev_free(da); dev_free(ds);
     dev_free(omega); dev_free(omega64); dev_free(gkg); dev_free(gmg);
     dev_free(sys);
-    dev_free(b); dev_free(x); dev_free(r); dev_free(s); dev_free(p); dev_free(a);
+    dev_free(r); dev_free(s); dev_free(hist); dev_free(p); dev_free(a);
     dev_free(z); dev_free(w); dev_free(sm); dev_free(h); dev_free(a2);
     prec_tile = false;
-    dev_free(b64); dev_free(xacc); dev_free(all_on);
+    dev_free(b64); dev_free(xacc);
     dev_free(uoff); dev_free(ucol); dev_free(lc); dev_free(lr);
     ntiles = 0;
     tiles_built = false;
@@ -215,14 +215,13 @@ __global__ void k_in64(int nb, int S, int SP, const double2 *src, double2 *dst)
     dst[i] = k < S ? src[(long long)k * nb + i / SP] : make_double2(0.0, 0.0);
 }
 
-__global__ void k_out64(int nb, int S, int SP, const double2 *xacc, const float4 *xdf,
-                        double2 *dst)
+__global__ void k_out64(int nb, int S, int SP, const double2 *xacc, double2 *dst)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long long)nb * SP) return;
     const int k = (int)(i % SP);
     if (k >= S) return;
-    dst[(long long)k * nb + i / SP] = x_total(xacc, xdf, i);
+    dst[(long long)k * nb + i / SP] = xacc[i];
 }
 
 // ------------------------------------------------------- conversions
@@ -781,12 +780,12 @@ int matfree_build(Survey &V, const MatFreeMesh &a, const DevMesh &dm, int kuz, i
     k_pattern<<<4 * nsm, kB, 0, V.st>>>(n, V.s);
     V.ch = 4;
     MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
-    MTGPU_SP_DISPATCH(V.SP, spmv_only(V));
+    MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
     MTGPU_TRY(cudaMemcpyAsync(V.w, V.z, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
     V.ch = kMatFree;
     MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
-    MTGPU_SP_DISPATCH(V.SP, spmv_only(V));
+    MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
     MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(unsigned long long) * 2, V.st));
     k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.z, V.w, d_mx);
     note_launches(5);
@@ -821,12 +820,12 @@ int matfree_build(Survey &V, const MatFreeMesh &a, const DevMesh &dm, int kuz, i
         MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
         V.ch = kMatFree;
         MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
-        MTGPU_SP_DISPATCH(V.SP, spmv_only(V));
+        MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
         MTGPU_TRY(cudaMemcpyAsync(V.w, V.z, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
         MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
         V.ch = kMatFree + 3;
         MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
-        MTGPU_SP_DISPATCH(V.SP, spmv_only(V));
+        MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
         V.ch = ch;
         MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
         if ((rc = dev_alloc(&d_mx, 2))) return rc;
@@ -872,12 +871,12 @@ int matfree_tile_check(Survey &V, int nsm)
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
     V.ch = kMatFree;
     MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
-    MTGPU_SP_DISPATCH(V.SP, spmv_only(V));
+    MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
     MTGPU_TRY(cudaMemcpyAsync(V.w, V.z, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
     V.ch = kMatFree + 2;
     MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
-    MTGPU_SP_DISPATCH(V.SP, spmv_only(V));
+    MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
     V.ch = ch;
     MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
     unsigned long long *d_mx = nullptr;
@@ -930,7 +929,7 @@ namespace {
 // allows it: a tensor mesh with the lattice's Dirichlet edges, every
 // interior node a row of G in node order, the compact G^T.  A set-up check
 // runs one step of both forms on the same pseudo-random vectors and keeps
-// the fused one only if p, a and w agree bit for bit.
+// the fused one only if a and w agree bit for bit.
 int prec_tile_setup(Survey &V, int nsm)
 {
     V.prec_tile = false;
@@ -956,32 +955,27 @@ int prec_tile_setup(Survey &V, int nsm)
     }
     float4 *ref = nullptr;
     unsigned long long *d_mx = nullptr;
-    if ((rc = dev_alloc(&ref, (size_t)3 * n)) || (rc = dev_alloc(&d_mx, 2))) {
+    if ((rc = dev_alloc(&ref, (size_t)2 * n)) || (rc = dev_alloc(&d_mx, 2))) {
         dev_free(ref);
         return rc;
     }
-    // the same inputs for both: s, z, a (V.a), p from the pattern, p saved
-    for (float4 *v : {V.s, V.z, V.a, V.p}) k_pattern<<<4 * nsm, kB, 0, V.st>>>(n, v);
-    note_launches(4);
-    MTGPU_TRY(cudaMemcpyAsync(V.a2, V.p, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
+    // the same z and a for both, from the pattern
+    for (float4 *v : {V.z, V.a}) k_pattern<<<4 * nsm, kB, 0, V.st>>>(n, v);
+    note_launches(2);
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
-    // unfused: k_edge updates a in place; keep a's input in ref[2]
-    MTGPU_TRY(cudaMemcpyAsync(ref + 2 * n, V.a, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
+    // unfused: k_edge updates a in place; its input is kept for the fused form
+    MTGPU_TRY(cudaMemcpyAsync(V.p, V.a, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
     MTGPU_SP_DISPATCH(V.SP, precond_step(V, false, V.a, V.a));
-    MTGPU_TRY(cudaMemcpyAsync(ref, V.p, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
-    MTGPU_TRY(cudaMemcpyAsync(ref + n, V.w, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
-    // fused: p restored, a's input back in V.a, a's output into ref[2]'s place after the copy
-    MTGPU_TRY(cudaMemcpyAsync(V.p, V.a2, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
-    MTGPU_TRY(cudaMemcpyAsync(V.a2, V.a, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));   // a (unfused result)
-    MTGPU_TRY(cudaMemcpyAsync(V.a, ref + 2 * n, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
-    MTGPU_TRY(cudaMemcpyAsync(ref + 2 * n, V.a2, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
+    MTGPU_TRY(cudaMemcpyAsync(ref, V.w, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
+    MTGPU_TRY(cudaMemcpyAsync(ref + n, V.a, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
+    // lanes beyond the batch's systems are written by neither
+    MTGPU_TRY(cudaMemcpyAsync(V.a2, V.a, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
-    MTGPU_SP_DISPATCH(V.SP, precond_step(V, true, V.a, V.a2));
+    MTGPU_SP_DISPATCH(V.SP, precond_step(V, true, V.p, V.a2));
     MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(unsigned long long) * 2, V.st));
-    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.p, ref, d_mx);
-    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.w, ref + n, d_mx);
-    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.a2, ref + 2 * n, d_mx);
-    note_launches(6);
+    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.w, ref, d_mx);
+    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.a2, ref + n, d_mx);
+    note_launches(5);
     unsigned long long mx[2] = {1, 1};
     cudaError_t err = cudaGetLastError();
     if (err == cudaSuccess) err = cudaMemcpyAsync(mx, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, V.st);
@@ -1055,21 +1049,23 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
         (rc = dev_alloc(&V.ds, (size_t)mm * V.SP)) || (rc = dev_alloc(&V.gkg, mm)) ||
         (rc = dev_alloc(&V.gmg, mm)) || (rc = dev_alloc(&V.omega, 32)) ||
         (rc = dev_alloc(&V.omega64, 32)) || (rc = dev_alloc(&V.sys, 32)) ||
-        (rc = dev_alloc(&V.b, nv)) || (rc = dev_alloc(&V.x, nv)) || (rc = dev_alloc(&V.r, nv)) ||
-        (rc = dev_alloc(&V.s, nv)) || (rc = dev_alloc(&V.p, nv)) || (rc = dev_alloc(&V.a, nv)) ||
+        (rc = dev_alloc(&V.r, nv)) || (rc = dev_alloc(&V.p, nv)) || (rc = dev_alloc(&V.a, nv)) ||
         (rc = dev_alloc(&V.z, nv)) || (rc = dev_alloc(&V.w, nv)) || (rc = dev_alloc(&V.sm, nv)) ||
         (rc = dev_alloc(&V.h, (size_t)mm * V.SP)) || (rc = dev_alloc(&V.b64, nv)) ||
-        (rc = dev_alloc(&V.xacc, nv)) || (rc = dev_alloc(&V.all_on, 32)) ||
+        (rc = dev_alloc(&V.xacc, nv)) || (rc = dev_alloc(&V.hist, 2 * 32 * kGroupIters)) ||
         (rc = dev_alloc(&V.partials, partial_slots(std::max(gmax, nsm * 32), V.SP))))
         return rc;
     V.pblocks = std::max(gmax, nsm * 32);
+    // the s vectors of a group of iterations: 16, fewer where they would take
+    // more than a quarter of the free memory (1: no more than without groups)
+    size_t mem_free = 0, mem_total = 0;
+    MTGPU_TRY(cudaMemGetInfo(&mem_free, &mem_total));
+    V.group = kGroupIters;
+    while (V.group > 1 && (size_t)(V.group + 1) * nv * sizeof(float4) > mem_free / 4) V.group /= 2;
+    if ((rc = dev_alloc(&V.s, (size_t)(V.group + 1) * nv))) return rc;
     MTGPU_TRY(cudaMemsetAsync(V.partials, 0, sizeof(float4) * kTicketSlots, st));
     MTGPU_TRY(cudaMallocHost((void **)&V.hsys, sizeof(SysState) * 32));
     trace.mark("allocations");
-    {
-        const std::vector<int> ones(32, 1);
-        MTGPU_TRY(cudaMemcpyAsync(V.all_on, ones.data(), sizeof(int) * 32, cudaMemcpyHostToDevice, st));
-    }
     std::vector<float2> omdf(32, make_float2(0.f, 0.f));
     std::vector<double> om64(32, 0.0);
     for (int k = 0; k < S; k++) {
@@ -1324,7 +1320,7 @@ int survey_spmv_timed(Survey &V, int reps, float *ms)
     MTGPU_TRY(cudaEventCreate(&e0));
     MTGPU_TRY(cudaEventCreate(&e1));
     MTGPU_TRY(cudaEventRecord(e0, V.st));
-    for (int q = 0; q < reps; q++) MTGPU_SP_DISPATCH(V.SP, spmv(V, 1));
+    for (int q = 0; q < reps; q++) MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 1));
     note_launches((unsigned long long)reps);
     MTGPU_TRY(cudaEventRecord(e1, V.st));
     MTGPU_TRY(cudaEventSynchronize(e1));
@@ -1361,15 +1357,15 @@ int survey_iter_timed(Survey &V, int reps, float *ms)
     }
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
     const long long nv = (long long)V.nb * V.SP;
-    for (float4 *v : {V.x, V.r, V.s, V.p, V.a, V.z, V.w, V.sm})
+    for (float4 *v : {V.r, V.s, V.p, V.a, V.z, V.w, V.sm})
         k_pattern<<<1024, kB, 0, V.st>>>(nv, v);
     if (V.G.m > 0) k_pattern<<<1024, kB, 0, V.st>>>((long long)V.G.m * V.SP, V.h);
-    note_launches(V.G.m > 0 ? 9 : 8);
+    note_launches(V.G.m > 0 ? 8 : 7);
     cudaEvent_t e0, e1;
     MTGPU_TRY(cudaEventCreate(&e0));
     MTGPU_TRY(cudaEventCreate(&e1));
     MTGPU_TRY(cudaEventRecord(e0, V.st));
-    for (int q = 0; q < reps; q++) MTGPU_SP_DISPATCH(V.SP, iteration(V, q));
+    for (int q = 0; q < reps; q++) MTGPU_SP_DISPATCH(V.SP, iteration(V, q, INT_MAX));
     note_launches((unsigned long long)reps * iteration_launches(V));
     MTGPU_TRY(cudaEventRecord(e1, V.st));
     MTGPU_TRY(cudaEventSynchronize(e1));
@@ -1398,7 +1394,7 @@ int survey_spmv(Survey &V, const double2 *x_sys_major, double2 *y_sys_major)
     const long long tot = (long long)V.nb * V.SP;
     const unsigned ge = (unsigned)((tot + kB - 1) / kB);
     k_in<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, x_sys_major, V.s);
-    MTGPU_SP_DISPATCH(V.SP, spmv_only(V));
+    MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
     k_out<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, V.z, y_sys_major);
     note_launches(2);
     MTGPU_TRY(cudaGetLastError());
@@ -1422,9 +1418,9 @@ int upload_flags(int *d, const std::vector<int> &h, cudaStream_t st)
 
 }  // namespace
 
-// The solution is held as x = xacc (FP64) + x_df (double-float increment);
-// every graph launch folds x_df into xacc (group update), so the rounding of
-// the x updates is relative to the increment, not to x: that keeps the true
+// The solution is accumulated in FP64: a group of iterations adds its
+// double-float increment at its end (k_group), so the rounding of the x
+// updates is relative to the increment, not to x: that keeps the true
 // residual at the FP64 solver's level down to 1e-3 Hz.  The iteration solves
 // A d = b - A x0 with the reference's stop rule relative to ||b||.  When the
 // systems have stopped, their true residuals are evaluated in FP64 from the
@@ -1481,7 +1477,6 @@ int survey_begin(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, do
     k_in64<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, b_sys_major, V.b64);
     k_in64<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, x_sys_major, V.xacc);
     note_launches(2);
-    MTGPU_TRY(cudaMemsetAsync(V.x, 0, sizeof(float4) * (size_t)tot, V.st));
     if ((rc = dev_alloc(&R.d_flag, 32))) return rc;
     // inner right-hand side r0 = b - A x0 (FP64), threshold relative to ||b||
     for (int k = 0; k < 32; k++) R.flag[k] = k < V.S;
@@ -1504,9 +1499,7 @@ int survey_begin(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, do
         cudaGraph_t g;
         MTGPU_TRY(cudaStreamBeginCapture(V.st, cudaStreamCaptureModeThreadLocal));
         // an even count: the fused preconditioner's a is back in V.a after the graph
-        for (int k = 0; k < R.ipl; k++) MTGPU_SP_DISPATCH(V.SP, iteration(V, k));
-        // group update: the double-float increment of x goes into the FP64 x
-        MTGPU_SP_DISPATCH(V.SP, fold(V, V.all_on));
+        for (int k = 0; k < R.ipl; k++) MTGPU_SP_DISPATCH(V.SP, iteration(V, k, R.ipl));
         MTGPU_TRY(cudaStreamEndCapture(V.st, &g));
         cudaError_t e = cudaGraphInstantiate(&V.graph, g, 0);
         cudaGraphDestroy(g);
@@ -1536,7 +1529,7 @@ int survey_launch(Survey &V, SurveyRun &R)
         return MTGPU_ERR_CUDA;
     }
     const unsigned long long kpi = iteration_launches(V);
-    note_launches(kpi * (unsigned long long)R.ipl + 1);
+    note_launches(kpi * (unsigned long long)R.ipl + ceil_div(R.ipl, V.group));
     R.guard += R.ipl;
     // the state arrives with the launch's end (read in survey_collect)
     MTGPU_TRY(cudaMemcpyAsync(V.hsys, V.sys, sizeof(SysState) * 32, cudaMemcpyDeviceToHost, V.st));
@@ -1630,7 +1623,7 @@ int survey_finish(Survey &V, SurveyRun &R, mtgpu_survey_stats *stats, int stat_o
         MTGPU_SP_DISPATCH(V.SP, res64(V, R.d_flag, 0));
         if ((rc = sync_sys(V))) return rc;
     }
-    k_out64<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, V.xacc, V.x, R.x_out);
+    k_out64<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, V.xacc, R.x_out);
     note_launches(1);
     MTGPU_TRY(cudaGetLastError());
     MTGPU_TRY(cudaStreamSynchronize(V.st));

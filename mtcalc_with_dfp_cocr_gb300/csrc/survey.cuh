@@ -19,13 +19,18 @@ struct SysState {
     double rnorm;          // ||b - A x|| of the last FP64 residual evaluation
     double res_next;       // ||s_m|| after this iteration's MRS step (k_update), for the stop test
     int mrs_mode;          // 0 keep s_m, 1 s_m = r, 2 s_m += w (r - s_m): the step the next k_update applies
-    int xp;                // x still lacks alpha p of the last k_update (the next k_edge or the fold adds it)
+    int cnt;               // iterations recorded in the present group (k_group applies them to p and x)
     int status;            // 1 running, else MTGPU_OK / MTGPU_DIV_BY_ZERO / MTGPU_MAXITER / MTGPU_X0_NULL
     int iter;              // the reference's iteration counter
     int checks;            // true-residual verifications
     int maxiter;
     unsigned int ticket[6];  // block-completion counters (system 0 only)
 };
+
+// Iterations per group: p and x are needed by nothing in the iteration, so
+// the group's s vectors, alpha and beta are kept and p = s + beta p, x +=
+// alpha p applied for the whole group by one kernel (k_group)
+constexpr int kGroupIters = 16;
 
 constexpr int kRowVariant = 16;    // + slots in flight: one thread per row, both systems
 constexpr int kMatFree = 32;       // matrix-free SpMV on tensor meshes (+1: two systems per thread)
@@ -83,8 +88,14 @@ struct Survey {
     double *omega64 = nullptr;
     double *gkg = nullptr, *gmg = nullptr;       // FP64 diag(G K G^T), diag(G M G^T)
     SysState *sys = nullptr, *hsys = nullptr;
-    float4 *b = nullptr, *x = nullptr, *r = nullptr, *s = nullptr, *p = nullptr, *a = nullptr,
-           *z = nullptr, *w = nullptr, *sm = nullptr;     // [row][SP]
+    float4 *r = nullptr, *p = nullptr, *a = nullptr, *z = nullptr, *w = nullptr,
+           *sm = nullptr;                         // [row][SP]
+    // s of the group's iterations: slot t is read by iteration t of a group
+    // and slot t + 1 written by it; the group kernel moves the last to slot 0
+    float4 *s = nullptr;                          // [group + 1][row][SP]
+    int group = 1;                                // iterations per group (<= kGroupIters)
+    float4 *hist = nullptr;                       // alpha, beta of the group's iterations: [32][kGroupIters][2]
+    int g_group = 0;                              // k_group's launch grid
     float4 *h = nullptr;                          // [node][SP]
     // the fused preconditioner of tensor meshes (prec_tile.cuh): its launch
     // grid, tiles x, y, z chunks, groups, planes per chunk, and the second
@@ -94,7 +105,6 @@ struct Survey {
     float prec_ms[2] = {};                        // set-up timing: ms per iteration unfused, fused
     float4 *a2 = nullptr;
     double2 *b64 = nullptr, *xacc = nullptr;      // FP64 b and accumulated x: [row][SP]
-    int *all_on = nullptr;                        // 32 flags, all set
     float4 *partials = nullptr;                   // tickets, then block and group partials (sys_grid_sum)
     int pblocks = 0;                              // blocks the partial-sum buffer holds
     cudaGraphExec_t graph = nullptr;

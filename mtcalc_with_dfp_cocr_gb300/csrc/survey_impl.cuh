@@ -421,36 +421,32 @@ inline void host_scalars(SysState &q)
     q.mrs_wf = make_float2(w.h, w.l);
 }
 
-// r = b - A x, s_m = r, ||b||, ||r||: stage 2 and the x0 test
+// s_m = r and ||r|| of the inner system A d = r (d = 0 initially, so its
+// right-hand side is its residual): stage 2 and the x0 test
 template <int SP>
 __global__ void __launch_bounds__(kB)
-k_init(int nb, Mat A, const float2 *__restrict__ omega, const float4 *__restrict__ b,
-       const float4 *__restrict__ x, float4 *__restrict__ r, float4 *__restrict__ sm,
-       SysState *sys, float4 *partials)
+k_init(int nb, const float4 *__restrict__ r, float4 *__restrict__ sm, SysState *sys, float4 *partials)
 {
     const int k = threadIdx.x % SP;
     const bool on = sys[k].status == kRun;
-    const df om = d2f(omega[k]);
-    acc nb2, nr2;
+    acc nr2;
     const int rpb = kB / SP;
     for (int row = blockIdx.x * rpb + threadIdx.x / SP; row < nb; row += gridDim.x * rpb) {
         if (!on) continue;
         const long long i = (long long)row * SP + k;
-        const dfc bv = from4(b[i]);
-        const dfc rv = csubd(bv, spmv_row<SP, 2>(A, row, k, om, x));
-        r[i] = to4(rv);
-        sm[i] = to4(rv);
-        nb2.mac(bv.re, bv.re); nb2.mac(bv.im, bv.im);
+        const float4 v = r[i];
+        const dfc rv = from4(v);
+        sm[i] = v;
         nr2.mac(rv.re, rv.re); nr2.mac(rv.im, rv.im);
     }
-    const tf v[2] = {tf_of(nb2), tf_of(nr2)};
-    __shared__ double tot[2][32];
-    if (sys_grid_sum<SP, 2>(v, partials, tot) && threadIdx.x < SP) {
+    const tf v[1] = {tf_of(nr2)};
+    __shared__ double tot[1][32];
+    if (sys_grid_sum<SP, 1>(v, partials, tot) && threadIdx.x < SP) {
         SysState &q = sys[threadIdx.x];
         if (q.status == kRun) {
-            const double bb = tot[0][threadIdx.x], rr = tot[1][threadIdx.x];
-            q.r_old = bb > 0.0 ? sqrt(bb) : 0.0;
+            const double rr = tot[0][threadIdx.x];
             q.residual = rr > 0.0 ? sqrt(rr) : 0.0;
+            q.r_old = q.residual;
             q.residual_rel = 1.0;
             q.beta = make_double2(0.0, 0.0);
             q.beta_f = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -496,26 +492,23 @@ k_node(int m, const int *__restrict__ gp, const int *__restrict__ gj, const floa
     }
 }
 
-// mode 1: p = s + beta p, a = z + beta a, w = D_A a + G^T h, (a, w) -> alpha
-// mode 0: w = D_A src + G^T h (preconditioner application, no reduction)
-// Every input of an element is loaded before anything is stored.
+// mode 1: a = z + beta a, w = D_A a + G^T h, (a, w) -> alpha; first: the
+// iteration is the first of its group
+// mode 0: w = D_A z + G^T h (preconditioner application, no reduction)
+// Every input of an element is loaded before anything is stored.  p = s +
+// beta p and x += alpha p are k_group's: reading s and p and x here and
+// writing p and x were 5 of this kernel's 11 vector passes.
 template <int SP>
 __global__ void __launch_bounds__(kB)
 k_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj, const float *__restrict__ tv,
        const int2 *__restrict__ tn, const float4 *__restrict__ da, const float4 *__restrict__ h,
-       const float4 *__restrict__ src, const float4 *__restrict__ z, float4 *__restrict__ p,
-       float4 *__restrict__ a, float4 *__restrict__ w, float4 *__restrict__ x, SysState *sys,
-       float4 *partials, int mode, int rev)
+       const float4 *__restrict__ z, float4 *__restrict__ a, float4 *__restrict__ w, SysState *sys,
+       float4 *partials, int mode, int first, int rev)
 {
     pdl_wait();
     const int k = threadIdx.x % SP;
     const bool on = sys[k].status == kRun;
     const dfc be = from4(sys[k].beta_f);
-    // the previous iteration's x += alpha p (mode 1), on the p read here
-    // before it is overwritten; alpha is read before the last block
-    // replaces it
-    const bool xp = mode != 0 && sys[k].xp;
-    const dfc alp = from4(sys[k].alpha_f);
     acc awr, awi;
     const int rpb = kB / SP, stride = gridDim.x * rpb;
     // the compact G^T row of the next element is loaded one element ahead,
@@ -540,14 +533,9 @@ k_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj, const floa
             j0 = __ldg(tp + e);
             j1 = __ldg(tp + e + 1);
         }
-        const float4 srcv = src[idx], dav = __ldg(da + idx);
-        float4 pv = make_float4(0.f, 0.f, 0.f, 0.f), zv = pv, av = pv, xv = pv;
-        if (mode != 0) {
-            pv = p[idx];
-            zv = z[idx];
-            av = a[idx];
-            if (xp) xv = x[idx];
-        }
+        const float4 zv = __ldg(z + idx), dav = __ldg(da + idx);
+        float4 av = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (mode != 0) av = a[idx];
         float4 hv0 = make_float4(0.f, 0.f, 0.f, 0.f), hv1 = hv0;
         float t0 = 0.f, t1 = 0.f;
         if (tn) {
@@ -573,10 +561,8 @@ k_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj, const floa
         }
         dfc an;
         if (mode == 0) {
-            an = from4(srcv);
+            an = from4(zv);
         } else {
-            if (xp) x[idx] = to4(caxpy(from4(xv), alp, from4(pv)));
-            p[idx] = to4(caxpy(from4(srcv), be, from4(pv)));
             an = caxpy(from4(zv), be, from4(av));
             a[idx] = to4(an);
         }
@@ -610,6 +596,7 @@ k_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj, const floa
     __shared__ double tot[2][32];
     if (sys_grid_sum<SP, 2>(v, partials, tot) && threadIdx.x < SP) {
         SysState &q = sys[threadIdx.x];
+        if (first) q.cnt = 0;
         if (q.status == kRun) {
             const double2 aw = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
             if (fabs(aw.x) < 1e-40 && fabs(aw.y) < 1e-40) q.status = MTGPU_DIV_BY_ZERO;
@@ -624,13 +611,14 @@ k_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj, const floa
 // s_m), on the r of that iteration), then the sums for this iteration's
 // weight w = -(s_m, u) / ||u||^2, u = r - s_m, and for ||s_m|| after this
 // iteration's step: ||s_m + w u||^2 = ||s_m||^2 + 2 w (s_m, u) + w^2 ||u||^2,
-// or ||r||^2 (mode 1).  x += alpha p is left to the next k_edge (which reads
-// p) or the group update.  Every input of an element is loaded before
-// anything is stored.
+// or ||r||^2 (mode 1).  The new s goes to the group's next slot and alpha and
+// beta into its record (k_group).  Every input of an element is loaded
+// before anything is stored.
 template <int SP>
 __global__ void __launch_bounds__(kB)
 k_update(int n, const float4 *__restrict__ a, const float4 *__restrict__ w, float4 *__restrict__ sm,
-         float4 *__restrict__ r, float4 *__restrict__ s, SysState *sys, float4 *partials, int rev)
+         float4 *__restrict__ r, const float4 *__restrict__ s_in, float4 *__restrict__ s_out,
+         SysState *sys, float4 *hist, float4 *partials, int rev)
 {
     pdl_wait();
     const int k = threadIdx.x % SP;
@@ -652,7 +640,7 @@ k_update(int n, const float4 *__restrict__ a, const float4 *__restrict__ w, floa
             if (u == 1 && !two) break;
             const long long idx = (long long)sweep(e + u * stride, n, rev) * SP + k;
             v[u][0] = __ldg(a + idx); v[u][1] = __ldg(w + idx);
-            v[u][2] = sm[idx]; v[u][3] = r[idx]; v[u][4] = s[idx];
+            v[u][2] = sm[idx]; v[u][3] = r[idx]; v[u][4] = __ldg(s_in + idx);
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
@@ -672,7 +660,7 @@ k_update(int n, const float4 *__restrict__ a, const float4 *__restrict__ w, floa
             }
             const dfc rn = caxpy(ro, nal, from4(v[u][0]));
             r[idx] = to4(rn);
-            s[idx] = to4(caxpy(from4(v[u][4]), nal, from4(v[u][1])));
+            s_out[idx] = to4(caxpy(from4(v[u][4]), nal, from4(v[u][1])));
             if (pm != 0) sm[idx] = to4(smv);
             const df ur = add(rn.re, neg(smv.re)), ui = add(rn.im, neg(smv.im));
             su.mac(smv.re, ur); su.mac(smv.im, ui);
@@ -701,7 +689,10 @@ k_update(int n, const float4 *__restrict__ a, const float4 *__restrict__ w, floa
                 const double m2 = n_n + 2.0 * wm * s_u + wm * wm * u_u;
                 q.res_next = m2 > 0.0 ? sqrt(m2) : 0.0;
             }
-            q.xp = 1;
+            const int c = min(q.cnt, kGroupIters - 1);
+            hist[2 * (threadIdx.x * kGroupIters + c)] = q.alpha_f;
+            hist[2 * (threadIdx.x * kGroupIters + c) + 1] = q.beta_f;
+            q.cnt = c + 1;
         }
     }
 }
@@ -1830,21 +1821,13 @@ struct Mat64 {
     const double *kc, *mc, *kr;
 };
 
-__device__ __forceinline__ double2 x_total(const double2 *__restrict__ xacc,
-                                           const float4 *__restrict__ xdf, long long i)
-{
-    const double2 a = __ldg(xacc + i);
-    const float4 d = __ldg(xdf + i);
-    return make_double2(a.x + ((double)d.x + (double)d.y), a.y + ((double)d.z + (double)d.w));
-}
-
-// r = b - A(omega) (xacc + x_df) in FP64 for the systems flagged in check;
+// r = b - A(omega) x in FP64 for the systems flagged in check;
 // ||b||, ||r||, true_rel into the system state; write != 0: r also becomes
-// the double-float right-hand side bdf of the next inner solve.
+// the double-float residual rdf that the inner solve starts from.
 template <int SP>
 __global__ void __launch_bounds__(kB)
 k_res64(int nb, Mat64 A, const double *__restrict__ omega64, const double2 *__restrict__ b64,
-        const double2 *__restrict__ xacc, const float4 *__restrict__ xdf, float4 *__restrict__ bdf,
+        const double2 *__restrict__ x, float4 *__restrict__ rdf,
         SysState *sys, const int *__restrict__ check, int write, float4 *partials)
 {
     const int k = threadIdx.x % SP;
@@ -1863,7 +1846,7 @@ k_res64(int nb, Mat64 A, const double *__restrict__ omega64, const double2 *__re
                 const long long t = b0 + (long long)kSlice * q;
                 const int c = __ldg(A.col_c + t);
                 const double kv = __ldg(A.kc + t), mv = __ldg(A.mc + t);
-                const double2 xv = x_total(xacc, xdf, (long long)c * SP + k);
+                const double2 xv = __ldg(x + (long long)c * SP + k);
                 kx += kv * xv.x;
                 ky += kv * xv.y;
                 mx += mv * xv.x;
@@ -1877,7 +1860,7 @@ k_res64(int nb, Mat64 A, const double *__restrict__ omega64, const double2 *__re
                 const long long t = b0 + (long long)kSlice * q;
                 const int c = __ldg(A.col_r + t);
                 const double kv = __ldg(A.kr + t);
-                const double2 xv = x_total(xacc, xdf, (long long)c * SP + k);
+                const double2 xv = __ldg(x + (long long)c * SP + k);
                 kx += kv * xv.x;
                 ky += kv * xv.y;
             }
@@ -1885,7 +1868,7 @@ k_res64(int nb, Mat64 A, const double *__restrict__ omega64, const double2 *__re
         const long long i = (long long)row * SP + k;
         const double2 bv = b64[i];
         const double2 rv = make_double2(bv.x - (kx - om * my), bv.y - (ky + om * mx));
-        if (write) bdf[i] = to4(from_d2(rv));
+        if (write) rdf[i] = to4(from_d2(rv));
         nb2 += bv.x * bv.x + bv.y * bv.y;
         nr2 += rv.x * rv.x + rv.y * rv.y;
     }
@@ -1902,36 +1885,55 @@ k_res64(int nb, Mat64 A, const double *__restrict__ omega64, const double2 *__re
     }
 }
 
-// xacc += x_df and x_df = 0 for the systems flagged in check (FP64 update),
-// x_df first completed by the x += alpha p still pending from the last
-// k_update (a system that stopped, or the graph's last iteration); the last
-// block clears the pending flags
+// p and x of a group of iterations: for each, p = s + beta p and d += alpha p
+// in double-float (d from 0), then x += d in FP64, and the last s to slot 0.
+// The same operations on the same values as one iteration at a time, so the
+// same p and x to the last bit; per iteration 1 + 6 / 16 vector passes instead
+// of the 5.4 of updating p and x in k_edge and folding x every 16 iterations
+// (1.8M edges x 2 systems: k_edge 95 -> 57 us, this kernel 11 us an iteration).
+// Four s values are in flight per thread.
 template <int SP>
-__global__ void k_fold(long long n, double2 *xacc, float4 *xdf, const float4 *__restrict__ p,
-                       const int *__restrict__ check, SysState *sys)
+__global__ void __launch_bounds__(kB)
+k_group(long long n, float4 *__restrict__ s, float4 *__restrict__ p, double2 *__restrict__ x,
+        const float4 *__restrict__ hist, const SysState *sys, int rev)
 {
     pdl_wait();
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = (int)(i % SP);
-    if (i < n && check[k]) {
-        const double2 a = xacc[i];
-        dfc d = from4(xdf[i]);
-        if (sys[k].xp) d = caxpy(d, from4(sys[k].alpha_f), from4(p[i]));
-        xacc[i] = make_double2(a.x + ((double)d.re.h + (double)d.re.l),
-                               a.y + ((double)d.im.h + (double)d.im.l));
-        xdf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __shared__ float4 ab[SP * kGroupIters * 2];
+    for (int i = threadIdx.x; i < SP * kGroupIters * 2; i += kB) ab[i] = hist[i];
+    __syncthreads();
+    const int k = threadIdx.x % SP;
+    const int cnt = sys[k].cnt;
+    if (cnt == 0) return;
+    const float4 *c = ab + 2 * kGroupIters * k;
+    const long long stride = (long long)gridDim.x * kB;
+    for (long long ii = (long long)blockIdx.x * kB + threadIdx.x; ii < n; ii += stride) {
+        // n is a multiple of SP: a backward sweep by rows keeps the lane's system
+        const long long i = rev ? n - SP - (ii - k) + k : ii;
+        dfc pv = from4(p[i]), d{df{0.f, 0.f}, df{0.f, 0.f}};
+        const double2 xv = x[i];
+        int j = 0;
+        for (; j + 4 <= cnt; j += 4) {
+            float4 sv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) sv[u] = s[(j + u) * n + i];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                pv = caxpy(from4(sv[u]), from4(c[2 * (j + u) + 1]), pv);
+                d = caxpy(d, from4(c[2 * (j + u)]), pv);
+            }
+        }
+        for (; j < cnt; j++) {
+            pv = caxpy(from4(s[j * n + i]), from4(c[2 * j + 1]), pv);
+            d = caxpy(d, from4(c[2 * j]), pv);
+        }
+        const float4 last = s[cnt * n + i];
+        x[i] = make_double2(xv.x + ((double)d.re.h + (double)d.re.l),
+                            xv.y + ((double)d.im.h + (double)d.im.l));
+        p[i] = to4(pv);
+        s[i] = last;
     }
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(&sys[0].ticket[4], 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    if (threadIdx.x < SP && check[threadIdx.x]) sys[threadIdx.x].xp = 0;
-    if (threadIdx.x == 0) sys[0].ticket[4] = 0u;
 }
 
-// ---------------------------------------------------------- dispatch
 template <int SP>
 struct Impl {
     static Mat mat(const Survey &V)
@@ -1989,95 +1991,100 @@ struct Impl {
             pdl(k_node<SP>, V.g_node, kB, 0, V.st, V.G.m, V.G.d_gp, V.G.d_gj, V.gv32, V.ds, src, a,
                 V.h, V.sys, use_beta, rv);
     }
-    static void spmv(Survey &V, int mode)
+    static void spmv(Survey &V, int mode, const float4 *s)
     {
         const Mat A = mat(V);
         if (V.ch == kMatFree + 2) {
             const MfTileGrid G{V.mft[0], V.mft[1], V.mft[2], V.mft[3], V.mft[4], V.mft[5], V.mft[6]};
             k_mf_tile<SP><<<V.g_mft, MfTile<SP>::NT, MfTile<SP>::SMEM, V.st>>>(
-                mfd(V), G, V.omega, V.s, V.z, V.sys, V.partials, mode);
+                mfd(V), G, V.omega, s, V.z, V.sys, V.partials, mode);
             return;
         }
         if (V.ch == kMatFree + 3) {
             const MF M = mfd(V);
-            pdl(k_mf_gmarch<SP>, V.g_mfg, kB, 0, V.st, M, gmarch(V), V.s, V.sys, flip(V));
-            pdl(k_mf_edges_g<SP>, V.g_mfe3, kB, 0, V.st, V.nb, M, V.omega, V.s, V.z, V.sys,
+            pdl(k_mf_gmarch<SP>, V.g_mfg, kB, 0, V.st, M, gmarch(V), s, V.sys, flip(V));
+            pdl(k_mf_edges_g<SP>, V.g_mfe3, kB, 0, V.st, V.nb, M, V.omega, s, V.z, V.sys,
                                                        V.partials, mode, flip(V));
             return;
         }
         if (V.ch == kMatFree || V.ch == kMatFree + 1) {
             const MF M = mfd(V);
-            pdl(k_mf_faces<SP>, V.g_mff, kB, 0, V.st, M, V.s, V.sys, flip(V));
+            pdl(k_mf_faces<SP>, V.g_mff, kB, 0, V.st, M, s, V.sys, flip(V));
             if constexpr (SP >= 2) {
                 if (V.ch == kMatFree + 1) {
-                    pdl(k_mf_edges2<SP>, V.g_mfe, kB, 0, V.st, V.nb, M, V.omega, V.s, V.z, V.sys, V.partials, mode, flip(V));
+                    pdl(k_mf_edges2<SP>, V.g_mfe, kB, 0, V.st, V.nb, M, V.omega, s, V.z, V.sys, V.partials, mode, flip(V));
                     return;
                 }
             }
-            pdl(k_mf_edges<SP>, V.g_mfe, kB, 0, V.st, V.nb, M, V.omega, V.s, V.z, V.sys,
+            pdl(k_mf_edges<SP>, V.g_mfe, kB, 0, V.st, V.nb, M, V.omega, s, V.z, V.sys,
                                                     V.partials, mode, flip(V));
             return;
         }
         if (V.ch == 0) {
             k_spmv_t<SP, true><<<V.g_spmv_t, TileCfg<SP>::NT, V.tile_smem, V.st>>>(
-                V.nb, tmat(V), V.omega, V.s, V.z, V.sys, V.partials, mode);
+                V.nb, tmat(V), V.omega, s, V.z, V.sys, V.partials, mode);
             return;
         }
         if (V.ch == 1) {
             k_spmv_t<SP, false><<<V.g_spmv_tx, TileCfg<SP>::NT, V.tile_smem_x, V.st>>>(
-                V.nb, tmat(V), V.omega, V.s, V.z, V.sys, V.partials, mode);
+                V.nb, tmat(V), V.omega, s, V.z, V.sys, V.partials, mode);
             return;
         }
         if constexpr (SP == 2) {
             if (V.ch == kRowVariant + 2) {
-                pdl(k_spmv_r2<2>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, V.s, V.z, V.sys, V.partials, mode);
+                pdl(k_spmv_r2<2>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, s, V.z, V.sys, V.partials, mode);
                 return;
             }
             if (V.ch == kRowVariant + 4) {
-                pdl(k_spmv_r2<4>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, V.s, V.z, V.sys, V.partials, mode);
+                pdl(k_spmv_r2<4>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, s, V.z, V.sys, V.partials, mode);
                 return;
             }
         }
         switch (V.ch) {
-        case 2: pdl(k_spmv<SP, 2>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, V.s, V.z, V.sys, V.partials, mode); break;
-        case 8: pdl(k_spmv<SP, 8>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, V.s, V.z, V.sys, V.partials, mode); break;
-        default: pdl(k_spmv<SP, 4>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, V.s, V.z, V.sys, V.partials, mode); break;
+        case 2: pdl(k_spmv<SP, 2>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, s, V.z, V.sys, V.partials, mode); break;
+        case 8: pdl(k_spmv<SP, 8>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, s, V.z, V.sys, V.partials, mode); break;
+        default: pdl(k_spmv<SP, 4>, V.g_spmv, kB, 0, V.st, V.nb, A, V.omega, s, V.z, V.sys, V.partials, mode); break;
         }
     }
-    // iteration t of a sequence: the fused preconditioner alternates a's
-    // buffers (t even reads a, writes a2; t odd the reverse)
-    static void iteration(Survey &V, int t)
+    // slot t of the group's s vectors
+    static float4 *slot_s(const Survey &V, int t) { return V.s + (size_t)t * V.nb * SP; }
+    static void precond(Survey &V, const float4 *src, float4 *w, int mode, int first)
     {
+        if (V.G.m > 0) node(V, src, V.a, mode);
+        pdl(k_edge<SP>, V.g_edge, kB, 0, V.st, V.nb, V.G.d_tp, V.G.d_tj, V.tv32, V.G.d_tn, V.da, V.h,
+            src, V.a, w, V.sys, V.partials, mode, first, flip(V));
+    }
+    static void prec_tile(Survey &V, const float4 *ain, float4 *aout, int first)
+    {
+        const PrecGrid G{V.pt[0], V.pt[1], V.pt[2], V.pt[3], V.pt[4]};
+        k_prec_tile<SP><<<V.g_pt, PrecTile<SP>::NT, PrecTile<SP>::SMEM, V.st>>>(
+            mfd(V), G, V.ds, V.da, V.z, ain, aout, V.w, V.sys, V.partials, first);
+    }
+    // iteration t of a sequence of n: the fused preconditioner alternates a's
+    // buffers (t even reads a, writes a2; t odd the reverse); p and x follow at
+    // the end of a group of iterations and of the sequence
+    static void iteration(Survey &V, int t, int n)
+    {
+        const int j = t % V.group;
+        float4 *a = V.a;
         if (V.prec_tile) {
-            float4 *ain = (t & 1) ? V.a2 : V.a, *aout = (t & 1) ? V.a : V.a2;
-            const PrecGrid G{V.pt[0], V.pt[1], V.pt[2], V.pt[3], V.pt[4]};
-            k_prec_tile<SP><<<V.g_pt, PrecTile<SP>::NT, PrecTile<SP>::SMEM, V.st>>>(
-                mfd(V), G, V.ds, V.da, V.s, V.z, ain, aout, V.p, V.w, V.x, V.sys, V.partials);
-            pdl(k_update<SP>, V.g_update, kB, 0, V.st, V.nb, aout, V.w, V.sm, V.r, V.s, V.sys,
-                V.partials, flip(V));
-            spmv(V, 1);
-            return;
+            a = (t & 1) ? V.a : V.a2;
+            prec_tile(V, (t & 1) ? V.a2 : V.a, a, j == 0);
+        } else {
+            precond(V, V.z, V.w, 1, j == 0);
         }
-        if (V.G.m > 0)
-            node(V, V.z, V.a, 1);
-        pdl(k_edge<SP>, V.g_edge, kB, 0, V.st, V.nb, V.G.d_tp, V.G.d_tj, V.tv32, V.G.d_tn, V.da, V.h, V.s, V.z,
-                                              V.p, V.a, V.w, V.x, V.sys, V.partials, 1, flip(V));
-        pdl(k_update<SP>, V.g_update, kB, 0, V.st, V.nb, V.a, V.w, V.sm, V.r, V.s, V.sys, V.partials, flip(V));
-        spmv(V, 1);
+        pdl(k_update<SP>, V.g_update, kB, 0, V.st, V.nb, a, V.w, V.sm, V.r, slot_s(V, j),
+            slot_s(V, j + 1), V.sys, V.hist, V.partials, flip(V));
+        spmv(V, 1, slot_s(V, j + 1));
+        if (j == V.group - 1 || t == n - 1)
+            pdl(k_group<SP>, V.g_group, kB, 0, V.st, (long long)V.nb * SP, V.s, V.p, V.xacc, V.hist,
+                V.sys, flip(V));
     }
     // one preconditioner step of the iteration (mode 1), unfused or fused
     static void precond_step(Survey &V, bool fused, float4 *ain, float4 *aout)
     {
-        if (fused) {
-            const PrecGrid G{V.pt[0], V.pt[1], V.pt[2], V.pt[3], V.pt[4]};
-            k_prec_tile<SP><<<V.g_pt, PrecTile<SP>::NT, PrecTile<SP>::SMEM, V.st>>>(
-                mfd(V), G, V.ds, V.da, V.s, V.z, ain, aout, V.p, V.w, V.x, V.sys, V.partials);
-            return;
-        }
-        if (V.G.m > 0)
-            node(V, V.z, ain, 1);
-        pdl(k_edge<SP>, V.g_edge, kB, 0, V.st, V.nb, V.G.d_tp, V.G.d_tj, V.tv32, V.G.d_tn, V.da, V.h,
-                                              V.s, V.z, V.p, ain, V.w, V.x, V.sys, V.partials, 1, flip(V));
+        if (fused) prec_tile(V, ain, aout, 1);
+        else precond(V, V.z, V.w, 1, 1);
     }
     static void prec_grid(Survey &V, int nsm)
     {
@@ -2112,31 +2119,22 @@ struct Impl {
     // p = a = 0, z = A s, (z, s)
     static void start(Survey &V)
     {
-        k_init<SP><<<V.g_init, kB, 0, V.st>>>(V.nb, mat(V), V.omega, V.b, V.x, V.r, V.sm, V.sys,
-                                              V.partials);
-        if (V.G.m > 0)
-            node(V, V.r, V.a, 0);
-        k_edge<SP><<<V.g_edge, kB, 0, V.st>>>(V.nb, V.G.d_tp, V.G.d_tj, V.tv32, V.G.d_tn, V.da, V.h, V.r, V.z,
-                                              V.p, V.a, V.s, V.x, V.sys, V.partials, 0, flip(V));
+        k_init<SP><<<V.g_init, kB, 0, V.st>>>(V.nb, V.r, V.sm, V.sys, V.partials);
+        precond(V, V.r, V.s, 0, 1);
         cudaMemsetAsync(V.p, 0, sizeof(float4) * (size_t)V.nb * SP, V.st);
         cudaMemsetAsync(V.a, 0, sizeof(float4) * (size_t)V.nb * SP, V.st);
-        spmv(V, 0);
+        spmv(V, 0, V.s);
         note_launches(V.G.m > 0 ? 4 : 3);
     }
     static void res64(Survey &V, const int *check, int write)
     {
         const ParamMatrix &P = *V.P;
         const Mat64 A{P.d_wc, P.d_wr, P.d_pc, P.d_pr, P.d_col_c, P.d_col_r, P.d_kc, P.d_mc, P.d_kr};
-        k_res64<SP><<<V.g_true, kB, 0, V.st>>>(V.nb, A, V.omega64, V.b64, V.xacc, V.x, V.b,
+        k_res64<SP><<<V.g_true, kB, 0, V.st>>>(V.nb, A, V.omega64, V.b64, V.xacc, V.r,
                                                V.sys, check, write, V.partials);
         note_launches(1);
     }
-    static void fold(Survey &V, const int *check)
-    {
-        const long long n = (long long)V.nb * SP;
-        pdl(k_fold<SP>, (unsigned)((n + kB - 1) / kB), kB, 0, V.st, n, V.xacc, V.x, V.p, check, V.sys);
-    }
-    static void spmv_only(Survey &V) { spmv(V, 0); }
+    static void spmv_only(Survey &V, int mode) { spmv(V, mode, V.s); }
 
     // launch grids: as many blocks as fit on the device at once (grid-stride
     // loops do the rest), never more than there is work for
@@ -2154,6 +2152,7 @@ struct Impl {
         V.g_node_lat = g((const void *)k_node_lat<SP>, V.grid_nodes);
         V.g_edge = g((const void *)k_edge<SP>, V.grid_rows);
         V.g_update = g((const void *)k_update<SP>, V.grid_rows);
+        V.g_group = g((const void *)k_group<SP>, V.grid_rows);
         V.g_true = g((const void *)k_res64<SP>, V.grid_rows);
         const void *fs = V.ch == 2 ? (const void *)k_spmv<SP, 2>
                          : V.ch == 8 ? (const void *)k_spmv<SP, 8> : (const void *)k_spmv<SP, 4>;
@@ -2249,14 +2248,12 @@ struct Impl {
 // Impl<SP> of one lane count as a table, so that survey.cu instantiates none of it
 struct Ops {
     void (*mfd_into)(const Survey &V, MF &M);
-    void (*spmv)(Survey &V, int mode);
-    void (*iteration)(Survey &V, int t);
+    void (*iteration)(Survey &V, int t, int n);
     void (*precond_step)(Survey &V, bool fused, float4 *ain, float4 *aout);
     void (*prec_grid)(Survey &V, int nsm);
     void (*start)(Survey &V);
     void (*res64)(Survey &V, const int *check, int write);
-    void (*fold)(Survey &V, const int *check);
-    void (*spmv_only)(Survey &V);
+    void (*spmv_only)(Survey &V, int mode);
     void (*grids)(Survey &V, int nsm);
     void (*tile_slices_of)(int *T);
     void (*tile_attr)(Survey &V, cudaError_t *e);
@@ -2266,7 +2263,7 @@ template <int SP>
 Ops make_ops()
 {
     using I = Impl<SP>;
-    return Ops{I::mfd_into, I::spmv, I::iteration, I::precond_step, I::prec_grid, I::start, I::res64, I::fold, I::spmv_only, I::grids, I::tile_slices_of, I::tile_attr, I::node};
+    return Ops{I::mfd_into, I::iteration, I::precond_step, I::prec_grid, I::start, I::res64, I::spmv_only, I::grids, I::tile_slices_of, I::tile_attr, I::node};
 }
 const Ops &ops1();
 const Ops &ops2();
