@@ -95,19 +95,18 @@ __device__ __forceinline__ df mul(df a, df b)
     return t.get();
 }
 
-// complex double-float stored as float4 (re.h, re.l, im.h, im.l)
+// complex double-float; in memory a float4 (re.h, im.h, re.l, im.l), so that
+// the high and the low parts of both components are register pairs for the
+// packed operations below
 struct dfc {
     df re, im;
 };
-
-__device__ __forceinline__ dfc ld(const float4 *p, long long i)
+__device__ __forceinline__ dfc from4(float4 v) { return dfc{df{v.x, v.z}, df{v.y, v.w}}; }
+__host__ __device__ __forceinline__ float4 to4(df re, df im) { return make_float4(re.h, im.h, re.l, im.l); }
+__device__ __forceinline__ float4 to4(dfc v) { return to4(v.re, v.im); }
+__device__ __forceinline__ double2 to_d2(float4 v)
 {
-    const float4 v = p[i];
-    return dfc{df{v.x, v.y}, df{v.z, v.w}};
-}
-__device__ __forceinline__ void st(float4 *p, long long i, dfc v)
-{
-    p[i] = make_float4(v.re.h, v.re.l, v.im.h, v.im.l);
+    return make_double2((double)v.x + (double)v.z, (double)v.y + (double)v.w);
 }
 
 // x + a * y  (complex)
@@ -140,6 +139,191 @@ __host__ __device__ __forceinline__ df from_double(double v)
     return df{h, (float)(v - (double)h)};
 }
 
+// ---- packed pairs
+// Blackwell's f32x2 instructions do one FP32 operation on two registers each:
+// the same rate per value as the scalar ones (measured 125 against 120 values
+// a clock and SM) in half the issue slots.  Both components of a complex
+// value take the same operations wherever the other factor is real, and with
+// one exchange of the components where it is complex, so the row kernels
+// carry (re, im) pairs.  Every result equals the scalar operations' above.
+using u64 = unsigned long long;
+__device__ __forceinline__ u64 pk(float a, float b)
+{
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpk(u64 v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b)
+{
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
+{
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// a * b + 0: written as a plain product, an add of its result would be
+// contracted to one multiply-add (ptxas does so for f32x2 in spite of .rn;
+// a unit test of the accumulators below shows it)
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) { return fma2(a, b, 0ull); }
+// a - b (b times -1 is exact)
+__device__ __forceinline__ u64 sub2(u64 a, u64 b) { return fma2(b, 0xbf800000bf800000ull, a); }
+__device__ __forceinline__ u64 swap2(u64 v)
+{
+    float a, b;
+    unpk(v, a, b);
+    return pk(b, a);
+}
+
+// a complex double-float (or two double-floats): high and low parts
+struct cdf {
+    u64 h, l;
+};
+__device__ __forceinline__ cdf cdf_of(float4 v) { return cdf{pk(v.x, v.y), pk(v.z, v.w)}; }
+__device__ __forceinline__ float4 to4(cdf v)
+{
+    float4 r;
+    unpk(v.h, r.x, r.y);
+    unpk(v.l, r.z, r.w);
+    return r;
+}
+// loads that stay where they are written, before the arithmetic: left to
+// itself the compiler moves a load next to its use among the packed
+// operations, and a row kernel's loads go out one latency after the other
+__device__ __forceinline__ cdf ldn(const float4 *p)      // read-only during the kernel
+{
+    cdf v;
+    asm volatile("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(v.h), "=l"(v.l) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ cdf ldg(const float4 *p)
+{
+    cdf v;
+    asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.h), "=l"(v.l) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ cdf cswap(cdf v) { return cdf{swap2(v.h), swap2(v.l)}; }
+__device__ __forceinline__ cdf czero() { return cdf{0ull, 0ull}; }
+// a real double-float for both components
+__device__ __forceinline__ cdf both(df v) { return cdf{pk(v.h, v.h), pk(v.l, v.l)}; }
+__device__ __forceinline__ df lane0(cdf v)
+{
+    df r;
+    float t;
+    unpk(v.h, r.h, t);
+    unpk(v.l, r.l, t);
+    return r;
+}
+__device__ __forceinline__ df lane1(cdf v)
+{
+    df r;
+    float t;
+    unpk(v.h, t, r.h);
+    unpk(v.l, t, r.l);
+    return r;
+}
+
+// acc for both components
+struct acc2 {
+    u64 h = 0ull, l = 0ull;
+    __device__ __forceinline__ void start(cdf x) { h = x.h; l = x.l; }
+    __device__ __forceinline__ void add(cdf x)
+    {
+        const u64 s = add2(h, x.h), nb = sub2(h, s);
+        const u64 e = add2(sub2(h, add2(s, nb)), add2(x.h, nb));
+        h = s;
+        l = add2(l, add2(e, x.l));
+    }
+    __device__ __forceinline__ void sub(cdf x)
+    {
+        const u64 s = sub2(h, x.h), nb = sub2(h, s);
+        const u64 e = add2(sub2(h, add2(s, nb)), sub2(nb, x.h));
+        h = s;
+        l = add2(l, sub2(e, x.l));
+    }
+    // = x * y, component by component
+    __device__ __forceinline__ void first(cdf x, cdf y)
+    {
+        h = mul2(x.h, y.h);
+        l = err(x, y, sub2(0ull, h));
+    }
+    // += x * y
+    __device__ __forceinline__ void mac(cdf x, cdf y)
+    {
+        const u64 p = mul2(x.h, y.h);
+        const u64 pe = err(x, y, sub2(0ull, p));
+        const u64 s = add2(h, p), b = sub2(s, h);
+        const u64 e = add2(sub2(h, sub2(s, b)), sub2(p, b));
+        h = s;
+        l = add2(l, add2(e, pe));
+    }
+    // -= x * y
+    __device__ __forceinline__ void msub(cdf x, cdf y)
+    {
+        const u64 np = sub2(0ull, mul2(x.h, y.h));
+        const u64 pe = err(x, y, np);
+        const u64 s = add2(h, np), b = sub2(s, h);
+        const u64 e = add2(sub2(h, sub2(s, b)), sub2(np, b));
+        h = s;
+        l = add2(l, sub2(e, pe));
+    }
+    // x * y - p for np = -p, p = fl(x.h y.h)
+    static __device__ __forceinline__ u64 err(cdf x, cdf y, u64 np)
+    {
+        u64 t = fma2(x.h, y.h, np);
+        t = fma2(x.h, y.l, t);
+        return fma2(x.l, y.h, t);
+    }
+    __device__ __forceinline__ cdf get() const
+    {
+        const u64 s = add2(h, l);
+        return cdf{s, sub2(l, sub2(s, h))};
+    }
+};
+__device__ __forceinline__ cdf csub(cdf a, cdf b)
+{
+    acc2 t;
+    t.start(a);
+    t.sub(b);
+    return t.get();
+}
+// a complex factor of many products: (re, re) and (-im, im)
+struct cfac {
+    cdf r, i;
+};
+__device__ __forceinline__ cfac cfac_of(cdf v)
+{
+    const df r = lane0(v), i = lane1(v);
+    return cfac{both(r), cdf{pk(-i.h, i.h), pk(-i.l, i.l)}};
+}
+__device__ __forceinline__ cfac cfac_of(dfc a)
+{
+    return cfac{both(a.re), cdf{pk(-a.im.h, a.im.h), pk(-a.im.l, a.im.l)}};
+}
+// x + a * y
+__device__ __forceinline__ cdf caxpy(cdf x, const cfac &a, cdf y)
+{
+    acc2 t;
+    t.start(x);
+    t.mac(a.r, y);
+    t.mac(a.i, cswap(y));
+    return t.get();
+}
+__device__ __forceinline__ cdf cmul(const cfac &a, cdf y)
+{
+    acc2 t;
+    t.first(a.r, y);
+    t.mac(a.i, cswap(y));
+    return t.get();
+}
+
 // ---- sums across threads
 // A partial sum as three FP32 numbers a + b + c.  Adding two of them with
 // two-sums on a and b keeps more than 60 bits (the error is that of c, about
@@ -161,6 +345,17 @@ __device__ __forceinline__ tf tf_add(tf x, tf y)
 }
 __device__ __forceinline__ tf tf_scale(tf x, float s) { return tf{x.a * s, x.b * s, x.c * s}; }
 __device__ __forceinline__ tf tf_of(const acc &x) { return tf{x.h, x.l, 0.f}; }
+__device__ __forceinline__ tf tf_of(df x) { return tf{x.h, x.l, 0.f}; }
+__device__ __forceinline__ tf tf_neg(tf x) { return tf{-x.a, -x.b, -x.c}; }
+// the sum of both components of an accumulator, and its first minus its second
+__device__ __forceinline__ tf tf_sum(const acc2 &x)
+{
+    return tf_add(tf_of(lane0(cdf{x.h, x.l})), tf_of(lane1(cdf{x.h, x.l})));
+}
+__device__ __forceinline__ tf tf_diff(const acc2 &x)
+{
+    return tf_add(tf_of(lane0(cdf{x.h, x.l})), tf_neg(tf_of(lane1(cdf{x.h, x.l}))));
+}
 __device__ __forceinline__ tf tf_of(double v)
 {
     const float a = (float)v;

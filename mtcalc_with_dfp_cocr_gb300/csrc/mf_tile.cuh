@@ -50,19 +50,6 @@ struct MfTile {
     static_assert(NT * 2 * 8 <= SMEM, "staging fits");
 };
 
-// asynchronous 16-byte copy global -> shared; valid = false writes zeros
-// (source size 0: nothing is read)
-__device__ __forceinline__ void cp_async16_zfill(void *smem_dst, const void *gsrc, bool valid)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    const int n = valid ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gsrc), "r"(n)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
 struct MfTileGrid {
     int tiles_x, tiles_y, zchunks, groups, kz;   // kz planes per chunk
     int tx, ty;   // node columns of a tile: tx * ty <= TX * TY, (tx + 2) (ty + 2) <= NS
@@ -73,10 +60,7 @@ __device__ __forceinline__ float4 f4zero() { return make_float4(0.f, 0.f, 0.f, 0
 // the same sum as k_mf_faces: a + b - c - d, in that order
 __device__ __forceinline__ float4 face_sum(float4 a, float4 b, float4 c, float4 d)
 {
-    acc fr, fi;
-    fr.add(df{a.x, a.y}); fr.add(df{b.x, b.y}); fr.add(neg(df{c.x, c.y})); fr.add(neg(df{d.x, d.y}));
-    fi.add(df{a.z, a.w}); fi.add(df{b.z, b.w}); fi.add(neg(df{c.z, c.w})); fi.add(neg(df{d.z, d.w}));
-    return to4(dfc{fr.get(), fi.get()});
+    return to4(mf_circ(cdf_of(a), cdf_of(b), cdf_of(c), cdf_of(d)));
 }
 
 // one face group of mf_row: sg (wa fm + 2 (wa + wb) f0 + wb fp) into kr, ki
@@ -370,8 +354,8 @@ k_mf_tile(MF M, MfTileGrid G, const float2 *__restrict__ omega, const float4 *__
     // per-system sums in a fixed order (deterministic): thread t's partials
     // staged, then thread u < SB adds those of its system in thread order
     double *const red = reinterpret_cast<double *>(sh);
-    red[tid] = tail.zsr.to_double();
-    red[NT + tid] = tail.zsi.to_double();
+    red[tid] = tf4_double(tf_pack(tail.zsr(), 0.f));
+    red[NT + tid] = tf4_double(tf_pack(tail.zsi(), 0.f));
     __syncthreads();
     double d[2] = {0.0, 0.0};
     if (tid < SP) {

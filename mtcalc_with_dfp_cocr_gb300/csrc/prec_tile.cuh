@@ -123,7 +123,7 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
                     hr.macf(t[m].re, g);
                     hi.macf(t[m].im, g);
                 }
-                out = to4(cmul(dfc{hr.get(), hi.get()}, from4(__ldg(ds + row * SP + sys0 + u))));
+                out = to4(cmul(from4(__ldg(ds + row * SP + sys0 + u)), dfc{hr.get(), hi.get()}));
             }
             hh(P, ii, jj, u) = out;
         }
@@ -165,17 +165,17 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
                 const float4 h1 = d == 2 ? hh(k + 1, ii, jj, u_me)
                                          : hh(k, ii + (d == 0), jj + (d == 1), u_me);
                 a_out[idx] = to4(an);
-                const dfc dv = cmul(an, from4(dav));
+                const dfc dv = cmul(from4(dav), an);
                 acc wr, wi;
                 wr.h = dv.re.h; wr.l = dv.re.l;
                 wi.h = dv.im.h; wi.l = dv.im.l;
                 if (in0) {
-                    wr.macf(df{h0.x, h0.y}, -0.5f);
-                    wi.macf(df{h0.z, h0.w}, -0.5f);
+                    wr.macf(df{h0.x, h0.z}, -0.5f);
+                    wi.macf(df{h0.y, h0.w}, -0.5f);
                 }
                 if (in1) {
-                    wr.macf(df{h1.x, h1.y}, 0.5f);
-                    wi.macf(df{h1.z, h1.w}, 0.5f);
+                    wr.macf(df{h1.x, h1.z}, 0.5f);
+                    wi.macf(df{h1.y, h1.w}, 0.5f);
                 }
                 const dfc wn{wr.get(), wi.get()};
                 w[idx] = to4(wn);

@@ -69,6 +69,8 @@ void MatFree::release()
     dev_free(w);
     dev_free(f);
     dev_free(g);
+    dev_free(dir);
+    ndir = 0;
     on = false;
     lattice = false;
     tiled = false;
@@ -104,10 +106,9 @@ __global__ void k_maxdiff(long long n, const float4 *__restrict__ a, const float
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
         const float4 u = a[i], v = b[i];
-        const double ur = (double)u.x + u.y, ui = (double)u.z + u.w;
-        const double vr = (double)v.x + v.y, vi = (double)v.z + v.w;
-        dm = fmax(dm, fmax(fabs(ur - vr), fabs(ui - vi)));
-        bm = fmax(bm, fmax(fabs(vr), fabs(vi)));
+        const double2 ud = to_d2(u), vd = to_d2(v);
+        dm = fmax(dm, fmax(fabs(ud.x - vd.x), fabs(ud.y - vd.y)));
+        bm = fmax(bm, fmax(fabs(vd.x), fabs(vd.y)));
     }
     atomicMax(out, (unsigned long long)__double_as_longlong(dm));
     atomicMax(out + 1, (unsigned long long)__double_as_longlong(bm));
@@ -126,7 +127,7 @@ __global__ void k_pattern(long long n, float4 *v)
             h ^= h >> 13;
             q[t] = (float)(h & 0xffffffu) / 8388608.0f - 1.0f;
         }
-        v[i] = make_float4(q[0], 0.f, q[2] * (1.f + 0.25f * q[1] * q[3]), 0.f);
+        v[i] = make_float4(q[0], q[2] * (1.f + 0.25f * q[1] * q[3]), 0.f, 0.f);
     }
 }
 
@@ -242,7 +243,7 @@ __global__ void k_in(int nb, int S, int SP, const double2 *src, float4 *dst)
     const int k = (int)(i % SP);
     const long long row = i / SP;
     const double2 v = k < S ? src[(long long)k * nb + row] : make_double2(0.0, 0.0);
-    st(dst, i, from_d2(v));
+    dst[i] = to4(from_d2(v));
 }
 
 __global__ void k_out(int nb, int S, int SP, const float4 *src, double2 *dst)
@@ -251,8 +252,7 @@ __global__ void k_out(int nb, int S, int SP, const float4 *src, double2 *dst)
     if (i >= (long long)nb * SP) return;
     const int k = (int)(i % SP);
     if (k >= S) return;
-    const float4 v = src[i];
-    dst[(long long)k * nb + i / SP] = make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
+    dst[(long long)k * nb + i / SP] = to_d2(src[i]);
 }
 
 // D_A[row][k] = 1 / (K_ii + i omega_k M_ii), computed in FP64
@@ -272,7 +272,7 @@ __global__ void k_diag_a(int nb, int SP, const int *nc, const long long *pc, con
         }
     }
     const double2 inv = cdiv(make_double2(1.0, 0.0), make_double2(kk, omega64[k] * mm));
-    st(da, i, from_d2(inv));
+    da[i] = to4(from_d2(inv));
 }
 
 // D_S[v][k] = 1 / (diag(G K G^T) + i omega_k diag(G M G^T)), in FP64
@@ -284,7 +284,7 @@ __global__ void k_diag_s(int m, int SP, const double *gkg, const double *gmg,
     const int k = (int)(i % SP);
     const int v = (int)(i / SP);
     const double2 inv = cdiv(make_double2(1.0, 0.0), make_double2(gkg[v], omega64[k] * gmg[v]));
-    st(ds, i, from_d2(inv));
+    ds[i] = to4(from_d2(inv));
 }
 
 // diag(G K G^T) and diag(G M G^T), FP64, in the reference's summation order
@@ -703,10 +703,31 @@ int matfree_build(Survey &V, const MatFreeMesh &a, const DevMesh &dm, int kuz, i
     F.nfx = (long long)nx * (ny - 1) * (nz - 1);
     F.nfy = (long long)(nx - 1) * ny * (nz - 1);
     F.nfz = (long long)(nx - 1) * (ny - 1) * nz;
+    // the edges on the outer surface: both transverse coordinates' lines of a
+    // direction that touch it, numbered as mf_edge does
+    std::vector<int> surface;
+    for (int k = 0; k < nz; k++)
+        for (int j = 0; j < ny; j++) {
+            const bool sk = k == 0 || k == nz - 1, sj = j == 0 || j == ny - 1;
+            const int ey = j < ny - 1, ez = k < nz - 1;
+            const int line = k * ((ny - 1) * (3 * nx - 1) + 2 * nx - 1) + j * (ez ? 3 * nx - 1 : 2 * nx - 1);
+            for (int i = 0; i < nx; i++) {
+                const bool si = i == 0 || i == nx - 1;
+                if (!si && !sj && !sk) {          // no surface edge along the rest of the line
+                    i = nx - 2;
+                    continue;
+                }
+                const int ex = i < nx - 1, e = line + i * (1 + ey + ez);
+                if (ex && (sj || sk)) surface.push_back(e);
+                if (ey && (si || sk)) surface.push_back(e + ex);
+                if (ez && (si || sj)) surface.push_back(e + ex + ey);
+            }
+        }
+    F.ndir = (int)surface.size();
     double *d_lines = nullptr;
     int *d_bad = nullptr;
     int rc;
-    if ((rc = dev_alloc(&F.pos, (size_t)P.nb)) ||
+    if ((rc = dev_alloc(&F.pos, (size_t)P.nb)) || (rc = dev_alloc(&F.dir, surface.size())) ||
         (rc = dev_alloc(&F.w, (size_t)6 * ncell)) ||
         (rc = dev_alloc(&F.f, (size_t)(F.nfx + F.nfy + F.nfz) * V.SP)) ||
         (rc = dev_alloc(&F.g, (size_t)(F.nfx + F.nfy + F.nfz) * V.SP)) ||
@@ -717,6 +738,8 @@ int matfree_build(Survey &V, const MatFreeMesh &a, const DevMesh &dm, int kuz, i
     }
     cudaError_t err = cudaMemcpyAsync(d_lines, lines.data(), sizeof(double) * lines.size(),
                                       cudaMemcpyHostToDevice, V.st);
+    if (err == cudaSuccess)
+        err = cudaMemcpyAsync(F.dir, surface.data(), sizeof(int) * surface.size(), cudaMemcpyHostToDevice, V.st);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(d_lines + lines.size(), a.mu.data(), sizeof(double) * nmat,
                               cudaMemcpyHostToDevice, V.st);

@@ -47,12 +47,22 @@ struct MatFree {
     float2 *w = nullptr;             // [6][cells] double-float wF/3 (x, y, z), wM/9 (x, y, z)
     float4 *f = nullptr;             // face circulations [faces][SP]
     float4 *g = nullptr;             // face mass applied to them, F f [faces][SP] (variant 35)
+    int *dir = nullptr;              // the edges on the outer surface
+    int ndir = 0;
     double check = -1.0;             // set-up check: max |A_mf s - A s| / max |A s|
     bool lattice = false;            // Dirichlet edges follow the lattice rule (always, when on)
     bool tiled = false;              // variant 34 equals variant 32 bit for bit
     bool tile_checked = false;       // ... and that was checked (on first request)
     bool gface = false;              // the D^T (F f) form agrees with variant 32 (variant 35)
     void release();
+};
+
+// Work of the marching kernels of variant 35: tiles of ly x lz lines in y
+// and z, per_tile items each (survey_impl.cuh)
+struct March {
+    int ly = 1, lz = 1, lx = 1;   // chunk lengths along y, z, x
+    int ty = 1, tz = 1;           // tiles
+    int per_tile = 0, items = 0;
 };
 
 struct Survey {
@@ -79,6 +89,7 @@ struct Survey {
     int g_mff = 0, g_mfe = 0;                    // matrix-free launch grids (faces, edges)
     int g_mft = 0;                               // tiled matrix-free launch grid (variant 34)
     int g_mfg = 0, g_mfe3 = 0;                   // face-mass and edge grids (variant 35)
+    March mg, me;                                // ... and their work
     int mft[7] = {};                             // its tiles x, y, z chunks, groups, planes per chunk, tile columns x, y
     Folded G;                                    // pattern of G and G^T
     float2 *kc = nullptr, *mc = nullptr, *kr = nullptr;   // double-float K and M per slot

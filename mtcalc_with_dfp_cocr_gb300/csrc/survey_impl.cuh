@@ -268,6 +268,37 @@ __device__ __forceinline__ void pdl_wait()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gsrc) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_wait_all()
+{
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+}
+
+// asynchronous 16-byte copy global -> shared; valid = false writes zeros
+// (source size 0: nothing is read)
+__device__ __forceinline__ void cp_async16_zfill(void *smem_dst, const void *gsrc, bool valid)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+    const int n = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gsrc), "r"(n)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// 8 bytes
+__device__ __forceinline__ void cp_async8(void *smem_dst, const void *gsrc)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gsrc) : "memory");
+}
+
 // Element i of a grid-stride sweep over n elements, forwards or backwards.
 // Consecutive kernels of the iteration sweep in opposite directions, so
 // that each starts on the end of what the previous one streamed, which is
@@ -303,8 +334,6 @@ struct Mat {
 // batch's column indices and matrix values are loaded first, then all its x
 // gathers are issued together, so CH gathers are in flight per thread.
 // Offsets stay 32-bit inside a row; full batches carry no predicates.
-__device__ __forceinline__ dfc from4(float4 v) { return dfc{df{v.x, v.y}, df{v.z, v.w}}; }
-__device__ __forceinline__ float4 to4(dfc v) { return make_float4(v.re.h, v.re.l, v.im.h, v.im.l); }
 
 template <int SP, int CH>
 __device__ __forceinline__ dfc spmv_row(const Mat &A, int row, int k, df om,
@@ -335,7 +364,7 @@ __device__ __forceinline__ dfc spmv_row(const Mat &A, int row, int k, df om,
 #pragma unroll
             for (int j = 0; j < CH; j++) {
                 const df kd = d2f(kv[j]), md = d2f(mv[j]);
-                const df xr{xv[j].x, xv[j].y}, xi{xv[j].z, xv[j].w};
+                const df xr{xv[j].x, xv[j].z}, xi{xv[j].y, xv[j].w};
                 kr_.mac(kd, xr);
                 ki_.mac(kd, xi);
                 mr_.mac(md, xr);
@@ -346,7 +375,7 @@ __device__ __forceinline__ dfc spmv_row(const Mat &A, int row, int k, df om,
             const int c = __ldg(cc + kSlice * q);
             const df kd = d2f(__ldg(kk + kSlice * q)), md = d2f(__ldg(mm + kSlice * q));
             const float4 xv = __ldg(xk + c * SP);
-            const df xr{xv.x, xv.y}, xi{xv.z, xv.w};
+            const df xr{xv.x, xv.z}, xi{xv.y, xv.w};
             kr_.mac(kd, xr);
             ki_.mac(kd, xi);
             mr_.mac(md, xr);
@@ -373,16 +402,16 @@ __device__ __forceinline__ dfc spmv_row(const Mat &A, int row, int k, df om,
 #pragma unroll
             for (int j = 0; j < 2 * CH; j++) {
                 const df kd = d2f(kv[j]);
-                kr_.mac(kd, df{xv[j].x, xv[j].y});
-                ki_.mac(kd, df{xv[j].z, xv[j].w});
+                kr_.mac(kd, df{xv[j].x, xv[j].z});
+                ki_.mac(kd, df{xv[j].y, xv[j].w});
             }
         }
         for (; q < n; q++) {
             const int c = __ldg(cc + kSlice * q);
             const df kd = d2f(__ldg(kk + kSlice * q));
             const float4 xv = __ldg(xk + c * SP);
-            kr_.mac(kd, df{xv.x, xv.y});
-            ki_.mac(kd, df{xv.z, xv.w});
+            kr_.mac(kd, df{xv.x, xv.z});
+            ki_.mac(kd, df{xv.y, xv.w});
         }
     }
     // y = Kx + i omega Mx
@@ -392,10 +421,8 @@ __device__ __forceinline__ dfc spmv_row(const Mat &A, int row, int k, df om,
     return dfc{kr_.get(), ki_.get()};
 }
 
-__device__ __forceinline__ dfc csubd(dfc a, dfc b)
-{
-    return dfc{add(a.re, neg(b.re)), add(a.im, neg(b.im))};
-}
+// t x for t = +-1/2 (exact)
+__device__ __forceinline__ cdf chalf(cdf x, float t) { return cdf{mul2(x.h, pk(t, t)), mul2(x.l, pk(t, t))}; }
 
 // ------------------------------------------------------------ set-up
 // the scalars that the row kernels read, in both forms
@@ -411,7 +438,7 @@ __device__ __forceinline__ void set_mrs_w(SysState &q, double v)
 inline float4 host_c4(double2 v)
 {
     const df r = from_double(v.x), i = from_double(v.y);
-    return make_float4(r.h, r.l, i.h, i.l);
+    return to4(r, i);
 }
 inline void host_scalars(SysState &q)
 {
@@ -429,17 +456,16 @@ k_init(int nb, const float4 *__restrict__ r, float4 *__restrict__ sm, SysState *
 {
     const int k = threadIdx.x % SP;
     const bool on = sys[k].status == kRun;
-    acc nr2;
+    acc2 nr2;
     const int rpb = kB / SP;
     for (int row = blockIdx.x * rpb + threadIdx.x / SP; row < nb; row += gridDim.x * rpb) {
         if (!on) continue;
         const long long i = (long long)row * SP + k;
         const float4 v = r[i];
-        const dfc rv = from4(v);
         sm[i] = v;
-        nr2.mac(rv.re, rv.re); nr2.mac(rv.im, rv.im);
+        nr2.mac(cdf_of(v), cdf_of(v));
     }
-    const tf v[1] = {tf_of(nr2)};
+    const tf v[1] = {tf_sum(nr2)};
     __shared__ double tot[1][32];
     if (sys_grid_sum<SP, 1>(v, partials, tot) && threadIdx.x < SP) {
         SysState &q = sys[threadIdx.x];
@@ -472,23 +498,21 @@ k_node(int m, const int *__restrict__ gp, const int *__restrict__ gj, const floa
     pdl_wait();
     const int k = threadIdx.x % SP;
     if (sys[k].status != kRun) return;
-    const dfc be = from4(sys[k].beta_f);
+    const cfac be = cfac_of(from4(sys[k].beta_f));
     const int rpb = kB / SP;
     for (int vi = blockIdx.x * rpb + threadIdx.x / SP; vi < m; vi += gridDim.x * rpb) {
         const int v = sweep(vi, m, rev);
         const int j0 = __ldg(gp + v), j1 = __ldg(gp + v + 1);
         const float4 dsv = __ldg(ds + (long long)v * SP + k);
-        acc hr, hi;
+        acc2 hv;
         for (int j = j0; j < j1; j++) {
             const long long idx = (long long)__ldg(gj + j) * SP + k;
             const float g = __ldg(gv + j);
-            const float4 zv = __ldg(z + idx);
-            dfc an = from4(zv);
-            if (use_beta) an = caxpy(an, be, from4(__ldg(a + idx)));
-            hr.macf(an.re, g);
-            hi.macf(an.im, g);
+            cdf an = cdf_of(__ldg(z + idx));
+            if (use_beta) an = caxpy(an, be, cdf_of(__ldg(a + idx)));
+            hv.mac(both(df{g, 0.f}), an);
         }
-        h[(long long)v * SP + k] = to4(cmul(dfc{hr.get(), hi.get()}, from4(dsv)));
+        h[(long long)v * SP + k] = to4(cmul(cfac_of(from4(dsv)), hv.get()));
     }
 }
 
@@ -508,8 +532,8 @@ k_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj, const floa
     pdl_wait();
     const int k = threadIdx.x % SP;
     const bool on = sys[k].status == kRun;
-    const dfc be = from4(sys[k].beta_f);
-    acc awr, awi;
+    const cfac be = cfac_of(from4(sys[k].beta_f));
+    acc2 aw1, aw2;     // a w component by component, and a with w's exchanged
     const int rpb = kB / SP, stride = gridDim.x * rpb;
     // the compact G^T row of the next element is loaded one element ahead,
     // so that this element's h gathers issue with its other loads
@@ -520,79 +544,37 @@ k_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj, const floa
         if (!on) break;
         const int e = sweep(ei, n, rev);
         const long long idx = (long long)e * SP + k;
+        const cdf zv = ldn(z + idx), dav = ldn(da + idx);
+        cdf av = czero(), h0 = czero(), h1 = czero();
+        if (mode != 0) av = ldg(a + idx);
+        acc2 wv;
+        cdf an;
         // G^T row: compact (the rows of the edge's two nodes, -1/2 and +1/2
         // in that order) or the CSR of T-matrix meshes
-        int j0, j1;
-        int2 r2 = make_int2(-1, -1);
         if (tn) {
-            r2 = r2n;
+            const int2 r2 = r2n;
+            if (r2.x >= 0) h0 = ldn(h + (long long)r2.x * SP + k);
+            if (r2.y >= 0) h1 = ldn(h + (long long)r2.y * SP + k);
             if (ei + stride < n) r2n = __ldg(tn + sweep(ei + stride, n, rev));
-            j0 = 0;
-            j1 = (r2.x >= 0) + (r2.y >= 0);
+            an = mode != 0 ? caxpy(zv, be, av) : zv;
+            wv.start(cmul(cfac_of(dav), an));
+            // +-1/2 is exact: added instead of multiplied
+            if (r2.x >= 0) wv.sub(chalf(h0, 0.5f));
+            if (r2.y >= 0) wv.add(chalf(h1, 0.5f));
         } else {
-            j0 = __ldg(tp + e);
-            j1 = __ldg(tp + e + 1);
+            an = mode != 0 ? caxpy(zv, be, av) : zv;
+            wv.start(cmul(cfac_of(dav), an));
+            for (int j = __ldg(tp + e); j < __ldg(tp + e + 1); j++)
+                wv.mac(both(df{__ldg(tv + j), 0.f}), ldn(h + (long long)__ldg(tj + j) * SP + k));
         }
-        const float4 zv = __ldg(z + idx), dav = __ldg(da + idx);
-        float4 av = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (mode != 0) av = a[idx];
-        float4 hv0 = make_float4(0.f, 0.f, 0.f, 0.f), hv1 = hv0;
-        float t0 = 0.f, t1 = 0.f;
-        if (tn) {
-            // entries in the CSR's order: the first node's (if any), then the second's
-            const int ra = r2.x >= 0 ? r2.x : r2.y, rb = r2.y;
-            if (j1 > 0) {
-                hv0 = __ldg(h + (long long)ra * SP + k);
-                t0 = r2.x >= 0 ? -0.5f : 0.5f;
-            }
-            if (j1 > 1) {
-                hv1 = __ldg(h + (long long)rb * SP + k);
-                t1 = 0.5f;
-            }
-        } else {
-            if (j1 > j0) {
-                hv0 = __ldg(h + (long long)__ldg(tj + j0) * SP + k);
-                t0 = __ldg(tv + j0);
-            }
-            if (j1 > j0 + 1) {
-                hv1 = __ldg(h + (long long)__ldg(tj + j0 + 1) * SP + k);
-                t1 = __ldg(tv + j0 + 1);
-            }
-        }
-        dfc an;
-        if (mode == 0) {
-            an = from4(zv);
-        } else {
-            an = caxpy(from4(zv), be, from4(av));
-            a[idx] = to4(an);
-        }
-        const dfc dv = cmul(an, from4(dav));
-        acc wr, wi;
-        wr.h = dv.re.h; wr.l = dv.re.l;
-        wi.h = dv.im.h; wi.l = dv.im.l;
-        if (j1 > j0) {
-            wr.macf(df{hv0.x, hv0.y}, t0);
-            wi.macf(df{hv0.z, hv0.w}, t0);
-        }
-        if (j1 > j0 + 1) {
-            wr.macf(df{hv1.x, hv1.y}, t1);
-            wi.macf(df{hv1.z, hv1.w}, t1);
-        }
-        for (int j = j0 + 2; j < j1 && !tn; j++) {       // T-matrix rows only
-            const float4 hv = __ldg(h + (long long)__ldg(tj + j) * SP + k);
-            const float t = __ldg(tv + j);
-            wr.macf(df{hv.x, hv.y}, t);
-            wi.macf(df{hv.z, hv.w}, t);
-        }
-        const dfc wn{wr.get(), wi.get()};
+        const cdf wn = wv.get();
+        if (mode != 0) a[idx] = to4(an);
         w[idx] = to4(wn);
-        awr.mac(an.re, wn.re);
-        awr.mac(neg(an.im), wn.im);
-        awi.mac(an.re, wn.im);
-        awi.mac(an.im, wn.re);
+        aw1.mac(an, wn);
+        aw2.mac(an, cswap(wn));
     }
     if (mode == 0) return;
-    const tf v[2] = {tf_of(awr), tf_of(awi)};
+    const tf v[2] = {tf_diff(aw1), tf_sum(aw2)};
     __shared__ double tot[2][32];
     if (sys_grid_sum<SP, 2>(v, partials, tot) && threadIdx.x < SP) {
         SysState &q = sys[threadIdx.x];
@@ -623,53 +605,52 @@ k_update(int n, const float4 *__restrict__ a, const float4 *__restrict__ w, floa
     pdl_wait();
     const int k = threadIdx.x % SP;
     const bool on = sys[k].status == kRun;
-    const dfc al = from4(sys[k].alpha_f);
-    const dfc nal{neg(al.re), neg(al.im)};
+    dfc al = from4(sys[k].alpha_f);
+    al = dfc{neg(al.re), neg(al.im)};
+    const cfac nal = cfac_of(al);
     const int pm = sys[k].mrs_mode;
-    const df pw = d2f(sys[k].mrs_wf);
-    acc su, uu, nn, rr;
+    const cdf pw = both(d2f(sys[k].mrs_wf));
+    acc2 su, uu, nn, rr;
     const int rpb = kB / SP;
     const int stride = gridDim.x * rpb;
     // two elements per pass, all 10 loads issued before any store
     for (int e = blockIdx.x * rpb + threadIdx.x / SP; e < n; e += 2 * stride) {
         if (!on) break;
         const bool two = e + stride < n;
-        float4 v[2][5];
+        cdf v[2][5];
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             if (u == 1 && !two) break;
             const long long idx = (long long)sweep(e + u * stride, n, rev) * SP + k;
-            v[u][0] = __ldg(a + idx); v[u][1] = __ldg(w + idx);
-            v[u][2] = sm[idx]; v[u][3] = r[idx]; v[u][4] = __ldg(s_in + idx);
+            v[u][0] = ldn(a + idx); v[u][1] = ldn(w + idx);
+            v[u][2] = ldg(sm + idx); v[u][3] = ldg(r + idx); v[u][4] = ldn(s_in + idx);
         }
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             if (u == 1 && !two) break;
             const long long idx = (long long)sweep(e + u * stride, n, rev) * SP + k;
-            const dfc ro = from4(v[u][3]);
-            dfc smv = from4(v[u][2]);
+            const cdf ro = v[u][3];
+            cdf smv = v[u][2];
             if (pm == 1) {
                 smv = ro;
             } else if (pm == 2) {
-                acc tr, ti;
-                tr.h = smv.re.h; tr.l = smv.re.l;
-                ti.h = smv.im.h; ti.l = smv.im.l;
-                tr.mac(pw, add(ro.re, neg(smv.re)));
-                ti.mac(pw, add(ro.im, neg(smv.im)));
-                smv = dfc{tr.get(), ti.get()};
+                acc2 t;
+                t.start(smv);
+                t.mac(pw, csub(ro, smv));
+                smv = t.get();
             }
-            const dfc rn = caxpy(ro, nal, from4(v[u][0]));
+            const cdf rn = caxpy(ro, nal, v[u][0]);
             r[idx] = to4(rn);
-            s_out[idx] = to4(caxpy(from4(v[u][4]), nal, from4(v[u][1])));
+            s_out[idx] = to4(caxpy(v[u][4], nal, v[u][1]));
             if (pm != 0) sm[idx] = to4(smv);
-            const df ur = add(rn.re, neg(smv.re)), ui = add(rn.im, neg(smv.im));
-            su.mac(smv.re, ur); su.mac(smv.im, ui);
-            uu.mac(ur, ur); uu.mac(ui, ui);
-            nn.mac(smv.re, smv.re); nn.mac(smv.im, smv.im);
-            rr.mac(rn.re, rn.re); rr.mac(rn.im, rn.im);
+            const cdf ur = csub(rn, smv);
+            su.mac(smv, ur);
+            uu.mac(ur, ur);
+            nn.mac(smv, smv);
+            rr.mac(rn, rn);
         }
     }
-    const tf v[4] = {tf_of(su), tf_of(uu), tf_of(nn), tf_of(rr)};
+    const tf v[4] = {tf_sum(su), tf_sum(uu), tf_sum(nn), tf_sum(rr)};
     __shared__ double tot[4][32];
     if (sys_grid_sum<SP, 4>(v, partials, tot) && threadIdx.x < SP) {
         SysState &q = sys[threadIdx.x];
@@ -700,19 +681,24 @@ k_update(int n, const float4 *__restrict__ a, const float4 *__restrict__ w, floa
 // Per-row tail of the SpMV kernels: store z = A s and accumulate (z, s).
 // (The MRS smoothing of the residual runs in k_update.)
 struct SpmvTail {
-    acc zsr, zsi;
-    __device__ __forceinline__ void row(long long i, dfc y, float4 sv4, float4 *__restrict__ z)
+    acc2 zs1, zs2;     // z s component by component, and z with s's exchanged
+    __device__ __forceinline__ void row(long long i, cdf y, cdf s, float4 *__restrict__ z)
     {
         z[i] = to4(y);
-        const dfc sv = from4(sv4);
-        zsr.mac(y.re, sv.re); zsr.mac(neg(y.im), sv.im);
-        zsi.mac(y.re, sv.im); zsi.mac(y.im, sv.re);
+        zs1.mac(y, s);
+        zs2.mac(y, cswap(s));
     }
+    __device__ __forceinline__ void row(long long i, dfc y, float4 sv4, float4 *__restrict__ z)
+    {
+        row(i, cdf_of(to4(y)), cdf_of(sv4), z);
+    }
+    __device__ __forceinline__ tf zsr() const { return tf_diff(zs1); }
+    __device__ __forceinline__ tf zsi() const { return tf_sum(zs2); }
     // grid totals -> stop test and beta (the last block only)
     template <int SP, int NT = kB>
     __device__ __forceinline__ void finish(SysState *sys, float4 *partials, int mode)
     {
-        const tf v[2] = {tf_of(zsr), tf_of(zsi)};
+        const tf v[2] = {zsr(), zsi()};
         finish_v<SP, NT>(v, sys, partials, mode);
     }
     // the same from this thread's (z, s) re, im of system threadIdx.x % SP.
@@ -810,7 +796,7 @@ __device__ __forceinline__ void spmv_row_all(const Mat &A, int row, const df (&o
                 const df kd = d2f(kv[j]), md = d2f(mv[j]);
 #pragma unroll
                 for (int k = 0; k < SP; k++) {
-                    const df xr{xv[j][k].x, xv[j][k].y}, xi{xv[j][k].z, xv[j][k].w};
+                    const df xr{xv[j][k].x, xv[j][k].z}, xi{xv[j][k].y, xv[j][k].w};
                     kr_[k].mac(kd, xr);
                     ki_[k].mac(kd, xi);
                     mr_[k].mac(md, xr);
@@ -846,8 +832,8 @@ __device__ __forceinline__ void spmv_row_all(const Mat &A, int row, const df (&o
                 const df kd = d2f(kv[j]);
 #pragma unroll
                 for (int k = 0; k < SP; k++) {
-                    kr_[k].mac(kd, df{xv[j][k].x, xv[j][k].y});
-                    ki_[k].mac(kd, df{xv[j][k].z, xv[j][k].w});
+                    kr_[k].mac(kd, df{xv[j][k].x, xv[j][k].z});
+                    ki_[k].mac(kd, df{xv[j][k].y, xv[j][k].w});
                 }
             }
         }
@@ -895,11 +881,11 @@ k_spmv_r2(int nb, Mat A, const float2 *__restrict__ omega, const float4 *__restr
         }
     }
     const bool odd = threadIdx.x & 1;
-    const acc z0[2] = {tail[0].zsr, tail[0].zsi}, z1[2] = {tail[1].zsr, tail[1].zsi};
+    const tf z0[2] = {tail[0].zsr(), tail[0].zsi()}, z1[2] = {tail[1].zsr(), tail[1].zsi()};
     tf v[2];
 #pragma unroll
     for (int n = 0; n < 2; n++) {
-        const tf mine = tf_of(odd ? z1[n] : z0[n]), give = tf_of(odd ? z0[n] : z1[n]);
+        const tf mine = odd ? z1[n] : z0[n], give = odd ? z0[n] : z1[n];
         v[n] = tf_add(mine, GridSum<SP, 2, kB>::shfl(give, 1));
     }
     SpmvTail::finish_v<SP>(v, sys, partials, mode);
@@ -937,6 +923,8 @@ struct MF {
     const float2 *w;
     float4 *f;
     float4 *g;                 // F f (variant 35)
+    const int *dir;            // the edges on the outer surface (variant 35)
+    int ndir;
 };
 
 // the edge counts and index strides of M from its node lines nx, ny, nz
@@ -1000,11 +988,11 @@ __device__ __forceinline__ int mf_edge_in(const MF &M, int d, int i, int j, int 
 
 // x of the +d edge of node (i, j, kk) for system k, 0 on Dirichlet edges
 template <int SP>
-__device__ __forceinline__ dfc mf_x(const MF &M, const float4 *__restrict__ x, int d, int i, int j,
+__device__ __forceinline__ cdf mf_x(const MF &M, const float4 *__restrict__ x, int d, int i, int j,
                                     int kk, int k)
 {
-    if (mf_dirichlet(M, d, i, j, kk)) return dfc{df{0.f, 0.f}, df{0.f, 0.f}};
-    return from4(__ldg(x + mf_edge_in(M, d, i, j, kk) * SP + k));
+    if (mf_dirichlet(M, d, i, j, kk)) return czero();
+    return cdf_of(__ldg(x + mf_edge_in(M, d, i, j, kk) * SP + k));
 }
 
 // k_node on a lattice mesh whose G rows are its interior nodes in node
@@ -1022,7 +1010,7 @@ k_node_lat(MF M, int m, const float4 *__restrict__ ds, const float4 *__restrict_
     pdl_wait();
     const int k = threadIdx.x % SP;
     if (sys[k].status != kRun) return;
-    const dfc be = from4(sys[k].beta_f);
+    const cfac be = cfac_of(from4(sys[k].beta_f));
     const int ix = M.nx - 2, iy = M.ny - 2;
     const int rpb = kB / SP;
     for (int vi = blockIdx.x * rpb + threadIdx.x / SP; vi < m; vi += gridDim.x * rpb) {
@@ -1030,87 +1018,35 @@ k_node_lat(MF M, int m, const float4 *__restrict__ ds, const float4 *__restrict_
         const int i = v % ix + 1, t = v / ix, j = t % iy + 1, kk = t / iy + 1;
         const int e0 = mf_edge_in(M, 0, i, j, kk);
         const int es[6] = {e0 + 2 - M.plane, e0 + 1 - M.l3, e0 - 3, e0, e0 + 1, e0 + 2};
-        float4 zv[6], av[6];
+        cdf zv[6], av[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++) zv[q] = ldn(z + (long long)es[q] * SP + k);
+#pragma unroll
+        for (int q = 0; q < 6; q++) av[q] = use_beta ? ldn(a + (long long)es[q] * SP + k) : czero();
+        const cdf dsv = ldn(ds + (long long)v * SP + k);
+        // the entries are +-1/2: the sum is halved once (exact, as each product)
+        acc2 hv;
 #pragma unroll
         for (int q = 0; q < 6; q++) {
-            zv[q] = __ldg(z + (long long)es[q] * SP + k);
-            av[q] = use_beta ? __ldg(a + (long long)es[q] * SP + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            cdf an = zv[q];
+            if (use_beta) an = caxpy(an, be, av[q]);
+            if (q == 0) hv.start(an);
+            else if (q < 3) hv.add(an);
+            else hv.sub(an);
         }
-        const float4 dsv = __ldg(ds + (long long)v * SP + k);
-        acc hr, hi;
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-            dfc an = from4(zv[q]);
-            if (use_beta) an = caxpy(an, be, from4(av[q]));
-            const float g = q < 3 ? 0.5f : -0.5f;
-            hr.macf(an.re, g);
-            hi.macf(an.im, g);
-        }
-        h[(long long)v * SP + k] = to4(cmul(dfc{hr.get(), hi.get()}, from4(dsv)));
+        h[(long long)v * SP + k] = to4(cmul(cfac_of(dsv), chalf(hv.get(), 0.5f)));
     }
 }
 
-// face t (faces numbered by normal, then z, y, x) -> normal n and position;
-// 32-bit (the set-up keeps faces x systems below 2^31)
-__device__ __forceinline__ void mf_face_pos(const MF &M, int t, int &n, int &i, int &j, int &kk)
+// the circulation a + b - c - d
+__device__ __forceinline__ cdf mf_circ(cdf a, cdf b, cdf c, cdf d)
 {
-    const int fx = (int)M.nfx, fy = (int)M.nfy;
-    int q = t, a, b;
-    if (q < fx) {
-        n = 0;
-        a = M.nx;
-        b = M.ny - 1;
-    } else if ((q -= fx) < fy) {
-        n = 1;
-        a = M.nx - 1;
-        b = M.ny;
-    } else {
-        q -= fy;
-        n = 2;
-        a = M.nx - 1;
-        b = M.ny - 1;
-    }
-    const int r = q / a;
-    i = q - r * a;
-    kk = r / b;
-    j = r - kk * b;
-}
-
-// the circulation of system k's x around face (n, i, j, kk)
-template <int SP>
-__device__ __forceinline__ dfc mf_face_f(const MF &M, const float4 *__restrict__ x, int n, int i,
-                                         int j, int kk, int k)
-{
-    dfc a, b, c, d;
-    if (n == 0) {
-        a = mf_x<SP>(M, x, 1, i, j, kk, k);
-        b = mf_x<SP>(M, x, 2, i, j + 1, kk, k);
-        c = mf_x<SP>(M, x, 1, i, j, kk + 1, k);
-        d = mf_x<SP>(M, x, 2, i, j, kk, k);
-    } else if (n == 1) {
-        a = mf_x<SP>(M, x, 2, i, j, kk, k);
-        b = mf_x<SP>(M, x, 0, i, j, kk + 1, k);
-        c = mf_x<SP>(M, x, 2, i + 1, j, kk, k);
-        d = mf_x<SP>(M, x, 0, i, j, kk, k);
-    } else {
-        a = mf_x<SP>(M, x, 0, i, j, kk, k);
-        b = mf_x<SP>(M, x, 1, i + 1, j, kk, k);
-        c = mf_x<SP>(M, x, 0, i, j + 1, kk, k);
-        d = mf_x<SP>(M, x, 1, i, j, kk, k);
-    }
-    acc fr, fi;
-    fr.add(a.re); fr.add(b.re); fr.add(neg(c.re)); fr.add(neg(d.re));
-    fi.add(a.im); fi.add(b.im); fi.add(neg(c.im)); fi.add(neg(d.im));
-    return dfc{fr.get(), fi.get()};
-}
-
-// the circulation a + b - c - d in mf_face_f's order
-__device__ __forceinline__ dfc mf_circ(dfc a, dfc b, dfc c, dfc d)
-{
-    acc fr, fi;
-    fr.add(a.re); fr.add(b.re); fr.add(neg(c.re)); fr.add(neg(d.re));
-    fi.add(a.im); fi.add(b.im); fi.add(neg(c.im)); fi.add(neg(d.im));
-    return dfc{fr.get(), fi.get()};
+    acc2 f;
+    f.start(a);
+    f.add(b);
+    f.sub(c);
+    f.sub(d);
+    return f.get();
 }
 
 // f = D s: x(e0) + x(e1) - x(e2) - x(e3) around every face (counterclockwise
@@ -1129,16 +1065,16 @@ k_mf_faces(MF M, const float4 *__restrict__ x, const SysState *sys, int rev)
     const int nx = M.nx, ny = M.ny, nz = M.nz;
     const int nn = nx * ny * nz;
     const int rpb = kB / SP;
-    const dfc zero{df{0.f, 0.f}, df{0.f, 0.f}};
+    const cdf zero = czero();
     for (int ti = blockIdx.x * rpb + threadIdx.x / SP; ti < nn; ti += gridDim.x * rpb) {
         const int v = sweep(ti, nn, rev);
         const int r = v / nx, i = v - r * nx;
         const int kk = r / ny, j = r - kk * ny;
         // the node's +x, +y, +z edges exist below the last line of their axis
         const bool hx = i < nx - 1, hy = j < ny - 1, hz = kk < nz - 1;
-        const dfc ex = hx ? mf_x<SP>(M, x, 0, i, j, kk, k) : zero;
-        const dfc ey = hy ? mf_x<SP>(M, x, 1, i, j, kk, k) : zero;
-        const dfc ez = hz ? mf_x<SP>(M, x, 2, i, j, kk, k) : zero;
+        const cdf ex = hx ? mf_x<SP>(M, x, 0, i, j, kk, k) : zero;
+        const cdf ey = hy ? mf_x<SP>(M, x, 1, i, j, kk, k) : zero;
+        const cdf ez = hz ? mf_x<SP>(M, x, 2, i, j, kk, k) : zero;
         if (hy && hz)
             M.f[(M.fb[0] + (kk * (ny - 1) + j) * nx + i) * SP + k] =
                 to4(mf_circ(ey, mf_x<SP>(M, x, 2, i, j + 1, kk, k), mf_x<SP>(M, x, 1, i, j, kk + 1, k), ez));
@@ -1202,159 +1138,122 @@ __device__ __forceinline__ int mf_mass_edge(const MF &M, const MfRow<D> &r, int 
     return r.e + (a - 1) * M.es[MfRow<D>::T1] + (b - 1) * M.es[MfRow<D>::T2];
 }
 
-// one non-Dirichlet edge of direction D at lattice position p:
-// (K + i omega M) s.  D, and with it the two transverse axes T1 = D+1,
-// T2 = D+2 (mod 3), are compile-time constants: the rows run direction by
-// direction, so warps are uniform.
-template <int SP, int D>
-__device__ __forceinline__ dfc mf_row(const MF &M, Pos p, int k, df om, const float4 *__restrict__ x)
+// (a0 + b0, a1 + b1) of two double-float pairs, packed
+__device__ __forceinline__ cdf pair_add(df a0, df a1, df b0, df b1)
 {
-    constexpr int T1 = (D + 1) % 3, T2 = (D + 2) % 3;
-    const int nc = (int)M.ncell;
-    const MfRow<D> r = mf_rowctx<D>(M, p);
-    // weights of the 4 cells around the edge, offsets (a - 1, b - 1) along (T1, T2)
-    df w1[2][2], w2[2][2], wm[2][2];
-#pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const int cc = r.cell + (a - 1) * M.cs[T1] + (b - 1) * M.cs[T2];
-            w1[a][b] = d2f(__ldg(M.w + T1 * nc + cc));
-            w2[a][b] = d2f(__ldg(M.w + T2 * nc + cc));
-            wm[a][b] = d2f(__ldg(M.w + (3 + D) * nc + cc));
-        }
-    acc kr, ki, mr, mi;
-    // D^T F D: faces of normal T1 through the edge (T2 cells b - 1 = -1: +1,
-    // 0: -1), then faces of normal T2 (T1 cells -1: -1, 0: +1); each face's
-    // F row: wa (f_-1 + 2 f_0) + wb (2 f_0 + f_+1) over the cells before and
-    // after it along the normal
-#pragma unroll
-    for (int b = 0; b < 2; b++) {
-        const int q = r.f1 + (b - 1) * M.fs[T1][T2];
-        const float sg = b == 0 ? 1.f : -1.f;
-        const df wa = w1[0][b], wb = w1[1][b];
-        const dfc fm = from4(__ldg(M.f + (q - M.fs[T1][T1]) * SP + k));
-        const dfc f0 = from4(__ldg(M.f + q * SP + k));
-        const dfc fp = from4(__ldg(M.f + (q + M.fs[T1][T1]) * SP + k));
-        const df ca = scale(wa, sg), cb = scale(wb, sg), c0 = scale(add(wa, wb), 2.f * sg);
-        kr.mac(ca, fm.re); kr.mac(c0, f0.re); kr.mac(cb, fp.re);
-        ki.mac(ca, fm.im); ki.mac(c0, f0.im); ki.mac(cb, fp.im);
-    }
-#pragma unroll
-    for (int a = 0; a < 2; a++) {
-        const int q = r.f2 + (a - 1) * M.fs[T2][T1];
-        const float sg = a == 0 ? -1.f : 1.f;
-        const df wa = w2[a][0], wb = w2[a][1];
-        const dfc fm = from4(__ldg(M.f + (q - M.fs[T2][T2]) * SP + k));
-        const dfc f0 = from4(__ldg(M.f + q * SP + k));
-        const dfc fp = from4(__ldg(M.f + (q + M.fs[T2][T2]) * SP + k));
-        const df ca = scale(wa, sg), cb = scale(wb, sg), c0 = scale(add(wa, wb), 2.f * sg);
-        kr.mac(ca, fm.re); kr.mac(c0, f0.re); kr.mac(cb, fp.re);
-        ki.mac(ca, fm.im); ki.mac(c0, f0.im); ki.mac(cb, fp.im);
-    }
-    // M: the 3 x 3 parallel edges around (grid position (A, B), this edge at
-    // (1, 1)); edge (A, B) lies in the cells (a, b) with a in {A-1, A},
-    // b in {B-1, B}, each contributing its weight times 2 per axis on which
-    // A (B) is the edge's own position: coefficients 4 (w00+w01+w10+w11),
-    // 2 (pair sums) and 1 (corner cells)
-    const df s0_ = add(wm[0][0], wm[0][1]), s1_ = add(wm[1][0], wm[1][1]);
-    const df r0_ = add(wm[0][0], wm[1][0]), r1_ = add(wm[0][1], wm[1][1]);
-    const df cm[3][3] = {{wm[0][0], scale(s0_, 2.f), wm[0][1]},
-                         {scale(r0_, 2.f), scale(add(s0_, s1_), 4.f), scale(r1_, 2.f)},
-                         {wm[1][0], scale(s1_, 2.f), wm[1][1]}};
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) {
-            dfc xe{df{0.f, 0.f}, df{0.f, 0.f}};
-            if (!mf_mass_dir(r, a, b)) xe = from4(__ldg(x + mf_mass_edge(M, r, a, b) * SP + k));
-            mr.mac(cm[a][b], xe.re);
-            mi.mac(cm[a][b], xe.im);
-        }
-    const df mxr = mr.get(), mxi = mi.get();
-    kr.mac(neg(om), mxi);
-    ki.mac(om, mxr);
-    return dfc{kr.get(), ki.get()};
+    acc2 t;
+    t.start(cdf{pk(a0.h, a1.h), pk(a0.l, a1.l)});
+    t.add(cdf{pk(b0.h, b1.h), pk(b0.l, b1.l)});
+    return t.get();
 }
 
-// The same row for two systems (k0, k0 + 1) at once: the index arithmetic,
-// the weights and their combinations are shared; the adjacent systems'
-// values are one contiguous 32-byte pair.
-template <int SP, int D>
-__device__ __forceinline__ void mf_row2(const MF &M, Pos p, int k0, const df (&om)[2],
-                                        const float4 *__restrict__ x, dfc (&y)[2])
+// weights w of the 4 cells around an edge of direction D, offsets (a - 1,
+// b - 1) along (T1, T2)
+template <int D>
+__device__ __forceinline__ void mf_weights(const MF &M, const MfRow<D> &r, int w, df (&out)[2][2])
 {
-    constexpr int T1 = (D + 1) % 3, T2 = (D + 2) % 3;
-    const int nc = (int)M.ncell;
-    const MfRow<D> r = mf_rowctx<D>(M, p);
-    df w1[2][2], w2[2][2], wm[2][2];
+    const int base = w * (int)M.ncell + r.cell;
 #pragma unroll
     for (int a = 0; a < 2; a++)
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const int cc = r.cell + (a - 1) * M.cs[T1] + (b - 1) * M.cs[T2];
-            w1[a][b] = d2f(__ldg(M.w + T1 * nc + cc));
-            w2[a][b] = d2f(__ldg(M.w + T2 * nc + cc));
-            wm[a][b] = d2f(__ldg(M.w + (3 + D) * nc + cc));
-        }
-    acc kr[2], ki[2], mr[2], mi[2];
-#pragma unroll
-    for (int nn = 0; nn < 2; nn++)
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            df wa, wb;
-            float sg;
-            int im, i0, ip;
-            if (nn == 0) {
-                sg = b == 0 ? 1.f : -1.f;
-                wa = w1[0][b];
-                wb = w1[1][b];
-                i0 = r.f1 + (b - 1) * M.fs[T1][T2];
-                im = i0 - M.fs[T1][T1];
-                ip = i0 + M.fs[T1][T1];
-            } else {
-                sg = b == 0 ? -1.f : 1.f;
-                wa = w2[b][0];
-                wb = w2[b][1];
-                i0 = r.f2 + (b - 1) * M.fs[T2][T1];
-                im = i0 - M.fs[T2][T2];
-                ip = i0 + M.fs[T2][T2];
-            }
-            const df ca = scale(wa, sg), cb = scale(wb, sg), c0 = scale(add(wa, wb), 2.f * sg);
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const dfc fm = from4(__ldg(M.f + im * SP + k0 + u));
-                const dfc f0 = from4(__ldg(M.f + i0 * SP + k0 + u));
-                const dfc fp = from4(__ldg(M.f + ip * SP + k0 + u));
-                kr[u].mac(ca, fm.re); kr[u].mac(c0, f0.re); kr[u].mac(cb, fp.re);
-                ki[u].mac(ca, fm.im); ki[u].mac(c0, f0.im); ki[u].mac(cb, fp.im);
-            }
-        }
-    const df s0_ = add(wm[0][0], wm[0][1]), s1_ = add(wm[1][0], wm[1][1]);
-    const df r0_ = add(wm[0][0], wm[1][0]), r1_ = add(wm[0][1], wm[1][1]);
-    const df cm[3][3] = {{wm[0][0], scale(s0_, 2.f), wm[0][1]},
-                         {scale(r0_, 2.f), scale(add(s0_, s1_), 4.f), scale(r1_, 2.f)},
-                         {wm[1][0], scale(s1_, 2.f), wm[1][1]}};
+        for (int b = 0; b < 2; b++)
+            out[a][b] = d2f(__ldg(M.w + base + (a - 1) * M.cs[MfRow<D>::T1] + (b - 1) * M.cs[MfRow<D>::T2]));
+}
+
+// The mass part of a row for U systems k0, k0 + 1, ...: the 3 x 3 parallel
+// edges around (grid position (A, B), this edge at (1, 1)); edge (A, B) lies
+// in the cells (a, b) with a in {A-1, A}, b in {B-1, B}, each contributing its
+// weight times 2 per axis on which A (B) is the edge's own position:
+// coefficients 4 (w00+w01+w10+w11), 2 (pair sums) and 1 (corner cells).
+// Then y = kk + i omega (mass part).  sv: the row's own x.
+template <int SP, int D, int U>
+__device__ __forceinline__ void mf_mass_row(const MF &M, const MfRow<D> &r, int k0, const df (&om)[U],
+                                            const float4 *__restrict__ x, const cdf (&sv)[U],
+                                            acc2 (&kk)[U], cdf (&y)[U])
+{
+    df wm[2][2];
+    mf_weights<D>(M, r, 3 + D, wm);
+    const cdf s = pair_add(wm[0][0], wm[1][0], wm[0][1], wm[1][1]);      // sums over b
+    const cdf q = pair_add(wm[0][0], wm[0][1], wm[1][0], wm[1][1]);      // sums over a
+    const df s0 = lane0(s), s1 = lane1(s), r0 = lane0(q), r1 = lane1(q);
+    const df cm[3][3] = {{wm[0][0], scale(s0, 2.f), wm[0][1]},
+                         {scale(r0, 2.f), scale(add(s0, s1), 4.f), scale(r1, 2.f)},
+                         {wm[1][0], scale(s1, 2.f), wm[1][1]}};
+    acc2 mm[U];
 #pragma unroll
     for (int a = 0; a < 3; a++)
 #pragma unroll
         for (int b = 0; b < 3; b++) {
-            if (mf_mass_dir(r, a, b)) continue;
-            const int e = mf_mass_edge(M, r, a, b);
+            const cdf c = both(cm[a][b]);
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const dfc xe = from4(__ldg(x + e * SP + k0 + u));
-                mr[u].mac(cm[a][b], xe.re);
-                mi[u].mac(cm[a][b], xe.im);
+            for (int u = 0; u < U; u++) {
+                cdf xe = czero();
+                if (a == 1 && b == 1)
+                    xe = sv[u];
+                else if (!mf_mass_dir(r, a, b))
+                    xe = cdf_of(__ldg(x + mf_mass_edge(M, r, a, b) * SP + k0 + u));
+                if (a == 0 && b == 0) mm[u].first(c, xe);
+                else mm[u].mac(c, xe);
             }
         }
 #pragma unroll
-    for (int u = 0; u < 2; u++) {
-        const df mxr = mr[u].get(), mxi = mi[u].get();
-        kr[u].mac(neg(om[u]), mxi);
-        ki[u].mac(om[u], mxr);
-        y[u] = dfc{kr[u].get(), ki[u].get()};
+    for (int u = 0; u < U; u++) {
+        const cdf f{pk(-om[u].h, om[u].h), pk(-om[u].l, om[u].l)};
+        kk[u].mac(f, cswap(mm[u].get()));
+        y[u] = kk[u].get();
     }
+}
+
+// one face group of a row: +- (wa f_-1 + 2 (wa + wb) f_0 + wb f_+1)
+template <int SP, int U, bool PLUS, bool FIRST>
+__device__ __forceinline__ void mf_face_group(const MF &M, int q, int step, int k0, df wa, df wb, df c2,
+                                              acc2 (&kk)[U])
+{
+    const cdf ca = both(wa), c0 = both(scale(c2, 2.f)), cb = both(wb);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const cdf fm = cdf_of(__ldg(M.f + (q - step) * SP + k0 + u));
+        const cdf f0 = cdf_of(__ldg(M.f + q * SP + k0 + u));
+        const cdf fp = cdf_of(__ldg(M.f + (q + step) * SP + k0 + u));
+        if (PLUS) {
+            if (FIRST) kk[u].first(ca, fm);
+            else kk[u].mac(ca, fm);
+            kk[u].mac(c0, f0);
+            kk[u].mac(cb, fp);
+        } else {
+            kk[u].msub(ca, fm);
+            kk[u].msub(c0, f0);
+            kk[u].msub(cb, fp);
+        }
+    }
+}
+
+// one non-Dirichlet edge of direction D at lattice position p for U systems:
+// (K + i omega M) s.  D, and with it the two transverse axes T1 = D+1,
+// T2 = D+2 (mod 3), are compile-time constants: the rows run direction by
+// direction, so warps are uniform.  The adjacent systems' values are
+// contiguous and share the index arithmetic, the weights and their
+// combinations.
+template <int SP, int D, int U>
+__device__ __forceinline__ void mf_row(const MF &M, Pos p, int k0, const df (&om)[U],
+                                       const float4 *__restrict__ x, const cdf (&sv)[U], cdf (&y)[U])
+{
+    constexpr int T1 = (D + 1) % 3, T2 = (D + 2) % 3;
+    const MfRow<D> r = mf_rowctx<D>(M, p);
+    df w1[2][2], w2[2][2];
+    mf_weights<D>(M, r, T1, w1);
+    mf_weights<D>(M, r, T2, w2);
+    // D^T F D: faces of normal T1 through the edge (T2 cells b - 1 = -1: +1,
+    // 0: -1), then faces of normal T2 (T1 cells -1: -1, 0: +1); each face's
+    // F row over the cells before and after it along the normal
+    acc2 kk[U];
+    const cdf c1 = pair_add(w1[0][0], w1[0][1], w1[1][0], w1[1][1]);
+    mf_face_group<SP, U, true, true>(M, r.f1 - M.fs[T1][T2], M.fs[T1][T1], k0, w1[0][0], w1[1][0], lane0(c1), kk);
+    mf_face_group<SP, U, false, false>(M, r.f1, M.fs[T1][T1], k0, w1[0][1], w1[1][1], lane1(c1), kk);
+    const cdf c2 = pair_add(w2[0][0], w2[1][0], w2[0][1], w2[1][1]);
+    mf_face_group<SP, U, false, false>(M, r.f2 - M.fs[T2][T1], M.fs[T2][T2], k0, w2[0][0], w2[0][1], lane0(c2), kk);
+    mf_face_group<SP, U, true, false>(M, r.f2, M.fs[T2][T2], k0, w2[1][0], w2[1][1], lane1(c2), kk);
+    mf_mass_row<SP, D, U>(M, r, k0, om, x, sv, kk, y);
 }
 
 // The matrix-free SpMV with two systems per thread (variant 33, SP >= 2):
@@ -1389,17 +1288,17 @@ k_mf_edges2(int nb, MF M, const float2 *__restrict__ omega, const float4 *__rest
             const Pos p{(int)(c & 1023u), (int)((c >> 10) & 1023u), (int)((c >> 20) & 1023u)};
             const int e = mf_edge(M, d, p.x, p.y, p.z);
             const long long i = (long long)e * SP + k0;
-            const float4 sv[2] = {__ldg(s + i), __ldg(s + i + 1)};
-            dfc y[2];
+            const cdf sv[2] = {cdf_of(__ldg(s + i)), cdf_of(__ldg(s + i + 1))};
+            cdf y[2];
             if (mf_dirichlet(M, d, p.x, p.y, p.z)) {
-                y[0] = from4(sv[0]);
-                y[1] = from4(sv[1]);
+                y[0] = sv[0];
+                y[1] = sv[1];
             } else if (d == 0) {
-                mf_row2<SP, 0>(M, p, k0, om, s, y);
+                mf_row<SP, 0, 2>(M, p, k0, om, s, sv, y);
             } else if (d == 1) {
-                mf_row2<SP, 1>(M, p, k0, om, s, y);
+                mf_row<SP, 1, 2>(M, p, k0, om, s, sv, y);
             } else {
-                mf_row2<SP, 2>(M, p, k0, om, s, y);
+                mf_row<SP, 2, 2>(M, p, k0, om, s, sv, y);
             }
 #pragma unroll
             for (int u = 0; u < 2; u++)
@@ -1412,11 +1311,11 @@ k_mf_edges2(int nb, MF M, const float2 *__restrict__ omega, const float4 *__rest
     const int lane = threadIdx.x & 31;
     const bool up = lane & H;
     const int from = (lane & ~(SP - 1)) | ((lane & 1) ? H : 0) | ((lane % SP) >> 1);
-    const acc z0[2] = {tail[0].zsr, tail[0].zsi}, z1[2] = {tail[1].zsr, tail[1].zsi};
+    const tf z0[2] = {tail[0].zsr(), tail[0].zsi()}, z1[2] = {tail[1].zsr(), tail[1].zsi()};
     tf v[2];
 #pragma unroll
     for (int n = 0; n < 2; n++) {
-        const tf mine = tf_of(up ? z1[n] : z0[n]), give = tf_of(up ? z0[n] : z1[n]);
+        const tf mine = up ? z1[n] : z0[n], give = up ? z0[n] : z1[n];
         const tf q = tf_add(mine, GridSum<SP, 2, kB>::shfl(give, H));
         v[n] = tf{__shfl_sync(0xffffffffu, q.a, from), __shfl_sync(0xffffffffu, q.b, from),
                   __shfl_sync(0xffffffffu, q.c, from)};
@@ -1434,7 +1333,7 @@ k_mf_edges(int nb, MF M, const float2 *__restrict__ omega, const float4 *__restr
     pdl_wait();
     const int k = threadIdx.x % SP;
     const bool on = sys[k].status == kRun;
-    const df om = d2f(omega[k]);
+    const df om[1] = {d2f(omega[k])};
     SpmvTail tail;
     const int rpb = kB / SP, stride = gridDim.x * rpb;
     // the next row's position is loaded one row ahead
@@ -1448,17 +1347,17 @@ k_mf_edges(int nb, MF M, const float2 *__restrict__ omega, const float4 *__restr
         const Pos p{(int)(c & 1023u), (int)((c >> 10) & 1023u), (int)((c >> 20) & 1023u)};
         const int e = mf_edge(M, d, p.x, p.y, p.z);
         const long long i = (long long)e * SP + k;
-        const float4 sv4 = __ldg(s + i);
-        dfc y;
+        const cdf sv[1] = {cdf_of(__ldg(s + i))};
+        cdf y[1];
         if (mf_dirichlet(M, d, p.x, p.y, p.z))
-            y = from4(sv4);
+            y[0] = sv[0];
         else if (d == 0)
-            y = mf_row<SP, 0>(M, p, k, om, s);
+            mf_row<SP, 0, 1>(M, p, k, om, s, sv, y);
         else if (d == 1)
-            y = mf_row<SP, 1>(M, p, k, om, s);
+            mf_row<SP, 1, 1>(M, p, k, om, s, sv, y);
         else
-            y = mf_row<SP, 2>(M, p, k, om, s);
-        tail.row(i, y, sv4, z);
+            mf_row<SP, 2, 1>(M, p, k, om, s, sv, y);
+        tail.row(i, y[0], sv[0], z);
     }
     tail.finish<SP>(sys, partials, mode);
 }
@@ -1473,189 +1372,282 @@ k_mf_edges(int nb, MF M, const float2 *__restrict__ omega, const float4 *__restr
 // whose position along the normal is interior (the faces of non-Dirichlet
 // edges); the others get 0.
 
-// g = F f straight from x, each circulation formed once (variant 35):
-// y- and z-normal faces by columns along the normal — a thread owns a
-// column (its transverse position; neighbouring threads, neighbouring
-// columns) and a chunk of kMarch positions, computes the circulations of
-// the chunk and of its two neighbours and keeps the last two in registers
-// while it marches; x-normal faces, whose neighbours along the normal are
-// the adjacent faces of the same row, one per thread with the two
-// neighbours' circulations formed from the same cached loads.  Every
-// circulation is k_mf_faces' sum and every g the same three multiply-adds
-// in the same order whichever thread forms it, so g does not depend on the
+// g = F f straight from x, each circulation formed once (variant 35): a
+// thread owns a column of faces along their normal and a chunk of len
+// positions, computes the circulations of the chunk and of its two neighbours
+// and keeps the last two in registers while it marches.  Every circulation
+// is k_mf_faces' sum and every g the same three multiply-adds in the same
+// order whichever thread forms it, so g does not depend on the
 // decomposition; no face array is written.
-constexpr int kMarch = 16;
+//
+// z = A s from g: a thread owns a line of parallel edges (direction D) along
+// one transverse axis Q and marches a chunk of len of them; R is the other
+// transverse axis.
+// Curl-curl part: the signed sum of g over the row's 4 faces; the R-normal
+// face shared with the row before stays in registers.
+// Mass part: m (x) m with m = [2 1; 1 2] per cell is applied first along R,
+// P_a(m) = 2 x(0, m) + x(+-1, m) for the cells a on either side, once per
+// line position and kept for the three rows that use it; a row then is the sum
+// over its 4 cells of w (2 P_a(m) + P_a(m +- 1)): 6 additions and 4
+// multiply-adds instead of 9 multiply-adds whose coefficients (sums of the
+// weights) have to be formed, and 8 loads a row (3 x, 3 g, 2 weights) instead
+// of 17.
+//
+// The rows on the outer surface (the identity) come from a list of their own.
+//
+// The edge kernel's next positions are copied to shared memory
+// asynchronously, kStages ahead, each thread into slots of its own: with
+// loads straight to registers the march was bound by their latency (27 % of
+// the issue slots used, 4 warps a scheduler for the registers).  Work is
+// ordered in tiles of ly x lz lines and columns in y and z, all
+// directions of a tile together, so that the vectors' cache lines, which hold
+// the three edges of a node, are used while they are in L2 (300 -> 160 MB of
+// DRAM traffic on 1.8M edges x 2 systems).
+constexpr int kStages = 2;
 
-struct GMarch {
-    int xitems, yitems;    // x-normal faces; y-normal column chunks (z-normal after)
-    int ycols, zcols;      // columns per chunk row: (nx-1) for both
-    int ych, zch;          // chunks per column
+// slots [stage][value][thread]
+template <int V>
+struct Ring {
+    float4 *base;
+    __device__ __forceinline__ float4 *at(int stage, int v) const
+    {
+        return base + (stage * V + v) * kB + threadIdx.x;
+    }
 };
 
-template <int SP>
-__device__ __forceinline__ dfc mf_g(const MF &M, int n, int cb, int ca, dfc fm, dfc f0, dfc fp)
+__device__ __forceinline__ cdf mf_g(df wa, df wb, cdf fm, cdf f0, cdf fp)
 {
-    const int nc = (int)M.ncell;
-    const df wa = d2f(__ldg(M.w + n * nc + cb)), wb = d2f(__ldg(M.w + n * nc + ca));
-    const df c0 = scale(add(wa, wb), 2.f);
-    acc gr, gi;
-    gr.mac(wa, fm.re); gr.mac(c0, f0.re); gr.mac(wb, fp.re);
-    gi.mac(wa, fm.im); gi.mac(c0, f0.im); gi.mac(wb, fp.im);
-    return dfc{gr.get(), gi.get()};
+    acc2 g;
+    g.first(both(wa), fm);
+    g.mac(both(scale(add(wa, wb), 2.f)), f0);
+    g.mac(both(wb), fp);
+    return g.get();
+}
+
+// the faces of normal N at c (c[N]: the chunk's first position) that are off
+// the outer surface; no edge row reads those on it
+template <int SP, int N>
+__device__ __forceinline__ void mf_face_march(const MF &M, int len, const int (&c)[3],
+                                              const float4 *__restrict__ x, int k)
+{
+    constexpr int A = (N + 1) % 3, B = (N + 2) % 3;        // transverse axes
+    const int ext[3] = {M.nx, M.ny, M.nz};
+    const int last = ext[N] - 1, p0 = max(c[N], 1), p1 = min(c[N] + len, last);
+    if (p0 >= p1) return;
+    // Dirichlet edges of the column's faces: a-edges at b = 0 and b + 1 on the
+    // far side, b-edges at a = 0 and a + 1 on the far side
+    const bool a0 = c[B] == 0, a1 = c[B] + 1 == ext[B] - 1, b0 = c[A] == 0, b1 = c[A] + 1 == ext[A] - 1;
+    const int es = M.es[N] * SP, ea = M.es[A] * SP, eb = M.es[B] * SP;
+    const float4 *__restrict__ xk = x + k;
+    // the circulation at the position of edge index i; 0 on the surface
+    auto fat = [&](int p, int i) {
+        if (p <= 0 || p >= last) return czero();
+        const cdf va = a0 ? czero() : ldn(xk + i + A * SP);
+        const cdf vb = b1 ? czero() : ldn(xk + i + ea + B * SP);
+        const cdf vc = a1 ? czero() : ldn(xk + i + eb + A * SP);
+        const cdf vd = b0 ? czero() : ldn(xk + i + B * SP);
+        return mf_circ(va, vb, vc, vd);
+    };
+    int e = (c[A] * M.es[A] + c[B] * M.es[B] + p0 * M.es[N]) * SP;
+    int face = (M.fb[N] + c[A] * M.fs[N][A] + c[B] * M.fs[N][B] + p0 * M.fs[N][N]) * SP + k;
+    int cell = N * (int)M.ncell + c[A] * M.cs[A] + c[B] * M.cs[B] + p0 * M.cs[N];
+    cdf fm = fat(p0 - 1, e - es), f0 = fat(p0, e);
+    df wa = d2f(__ldg(M.w + cell - M.cs[N]));
+    for (int p = p0; p < p1; p++) {
+        e += es;
+        const df wb = d2f(__ldg(M.w + cell));
+        const cdf fp = fat(p + 1, e);
+        M.g[face] = to4(mf_g(wa, wb, fm, f0, fp));
+        face += M.fs[N][N] * SP;
+        cell += M.cs[N];
+        wa = wb;
+        fm = f0;
+        f0 = fp;
+    }
 }
 
 template <int SP>
-__global__ void __launch_bounds__(kB)
-k_mf_gmarch(MF M, GMarch G, const float4 *__restrict__ x, const SysState *sys, int rev)
+__global__ void __launch_bounds__(kB, 4)
+k_mf_gmarch(MF M, March G, const float4 *__restrict__ x, const SysState *sys, int rev)
 {
     pdl_wait();
     const int k = threadIdx.x % SP;
     if (sys[k].status != kRun) return;
-    const dfc zero{df{0.f, 0.f}, df{0.f, 0.f}};
-    const int nx = M.nx, ny = M.ny, nz = M.nz;
-    auto cell = [&](int a, int b, int c) { return (c * (ny - 1) + b) * (nx - 1) + a; };
-    const int zitems = G.zcols * (ny - 1) * G.zch;
-    const int nitems = G.xitems + G.yitems + zitems;
-    const int rpb = kB / SP;
-    for (int qi = blockIdx.x * rpb + threadIdx.x / SP; qi < nitems; qi += gridDim.x * rpb) {
-        const int q = sweep(qi, nitems, rev);
-        if (q < G.xitems) {
-            // x-normal face t = (kk (ny-1) + j) nx + i: neighbours i -+ 1
-            int n, i, j, kk;
-            mf_face_pos(M, q, n, i, j, kk);
-            dfc out = zero;
-            if (i >= 1 && i < nx - 1) {
-                const dfc fm = mf_face_f<SP>(M, x, 0, i - 1, j, kk, k);
-                const dfc f0 = mf_face_f<SP>(M, x, 0, i, j, kk, k);
-                const dfc fp = mf_face_f<SP>(M, x, 0, i + 1, j, kk, k);
-                out = mf_g<SP>(M, 0, cell(i - 1, j, kk), cell(i, j, kk), fm, f0, fp);
-            }
-            M.g[(long long)q * SP + k] = to4(out);
-            continue;
-        }
-        // a column chunk: y-normal (column (i, kk), positions j) or z-normal
-        // (column (i, j), positions kk)
-        int n, i, c2, p0, L;
-        if (q < G.xitems + G.yitems) {
-            const int r = q - G.xitems;
-            n = 1;
-            i = r % G.ycols;
-            const int t = r / G.ycols;
-            c2 = t % (nz - 1);              // kk
-            p0 = (t / (nz - 1)) * kMarch;   // j
-            L = ny - 1;
+    const int rpb = kB / SP, nyz = G.ly * G.lz, cx = M.nx - 1;
+    for (int qi = blockIdx.x * rpb + threadIdx.x / SP; qi < G.items; qi += gridDim.x * rpb) {
+        const int q = sweep(qi, G.items, rev);
+        const int tile = q / G.per_tile, r = q - tile * G.per_tile;
+        const int tz = tile / G.ty, y0 = (tile - tz * G.ty) * G.ly, z0 = tz * G.lz;
+        const int line = r / cx, i = r - line * cx;
+        if (line < G.lz) {
+            // y-normal columns (i, z)
+            const int c[3] = {i, y0, z0 + line};
+            if (c[2] < M.nz - 1) mf_face_march<SP, 1>(M, G.ly, c, x, k);
+        } else if (line < G.lz + G.ly) {
+            // z-normal columns (i, y)
+            const int c[3] = {i, y0 + line - G.lz, z0};
+            if (c[1] < M.ny - 1) mf_face_march<SP, 2>(M, G.lz, c, x, k);
         } else {
-            const int r = q - G.xitems - G.yitems;
-            n = 2;
-            i = r % G.zcols;
-            const int t = r / G.zcols;
-            c2 = t % (ny - 1);              // j
-            p0 = (t / (ny - 1)) * kMarch;   // kk
-            L = nz - 1;
-        }
-        const int p1 = min(p0 + kMarch, L + 1);
-        auto fat = [&](int p) {
-            return n == 1 ? mf_face_f<SP>(M, x, 1, i, p, c2, k) : mf_face_f<SP>(M, x, 2, i, c2, p, k);
-        };
-        auto face = [&](int p) -> long long {
-            return n == 1 ? M.nfx + ((long long)c2 * ny + p) * (nx - 1) + i
-                          : M.nfx + M.nfy + ((long long)p * (ny - 1) + c2) * (nx - 1) + i;
-        };
-        dfc fm = p0 >= 1 ? fat(p0 - 1) : zero;
-        dfc f0 = fat(p0);
-        for (int p = p0; p < p1; p++) {
-            const dfc fp = p + 1 <= L ? fat(p + 1) : zero;
-            dfc out = zero;
-            if (p >= 1 && p < L) {
-                const int cb = n == 1 ? cell(i, p - 1, c2) : cell(i, c2, p - 1);
-                const int ca = n == 1 ? cell(i, p, c2) : cell(i, c2, p);
-                out = mf_g<SP>(M, n, cb, ca, fm, f0, fp);
-            }
-            M.g[face(p) * SP + k] = to4(out);
-            fm = f0;
-            f0 = fp;
+            // x-normal columns (y, z), chunks along x
+            const int s = r - (G.lz + G.ly) * cx, ch = s / nyz, t = s - ch * nyz, jz = t / G.ly;
+            const int c[3] = {ch * G.lx, y0 + t - jz * G.ly, z0 + jz};
+            if (c[1] < M.ny - 1 && c[2] < M.nz - 1) mf_face_march<SP, 0>(M, G.lx, c, x, k);
         }
     }
 }
 
-// one non-Dirichlet edge of direction D at lattice position p: the signed
-// sum of g over its 4 faces (the signs of mf_row's groups) plus the mass
-// part of mf_row
+constexpr int kEdgeValues = 7;    // x at R - 1, 0, R + 1; g of three faces; two weights
+// the edges of direction D at c (c[Q]: the chunk's first position)
 template <int SP, int D>
-__device__ __forceinline__ dfc mf_row_g(const MF &M, Pos p, int k, df om, const float4 *__restrict__ x)
+__device__ __forceinline__ void mf_edge_march(const MF &M, int len, const int (&c)[3], df om, int k,
+                                              const float4 *__restrict__ x, float4 *__restrict__ z,
+                                              SpmvTail &tail, Ring<kEdgeValues> ring)
 {
-    constexpr int T1 = (D + 1) % 3, T2 = (D + 2) % 3;
-    const int nc = (int)M.ncell;
-    const MfRow<D> r = mf_rowctx<D>(M, p);
-    df wm[2][2];
+    constexpr int Q = D == 2 ? 1 : 2, R = 3 - D - Q;
+    constexpr bool FLIP = D == 1;                        // Q is D + 1 and not D + 2
+    const int ext[3] = {M.nx, M.ny, M.nz};
+    const int last = ext[Q] - 1, a = max(c[Q], 1), b = min(c[Q] + len, last);
+    if (a >= b || c[R] == 0 || c[R] == ext[R] - 1) return;
+    const float4 *__restrict__ xk = x + k;
+    {
+        const bool lo = c[R] == 1, hi = c[R] == ext[R] - 2;
+        const int es = M.es[Q] * SP, er = M.es[R] * SP;
+        // row m = a: its edge, the weight of the cell (R, a), the R-normal
+        // face (R, a) and the Q-normal face (R, a)
+        int e = (c[2] * M.plane + c[1] * M.l3 + 3 * c[0] + D) * SP + (a - c[Q]) * es;
+        const int cell0 = (3 + D) * (int)M.ncell + c[R] * M.cs[R] + c[D] * M.cs[D];
+        const int fr0 = (M.fb[R] + c[R] * M.fs[R][R] + c[D] * M.fs[R][D]) * SP + k, frq = M.fs[R][Q] * SP;
+        const int fq0 = (M.fb[Q] + c[R] * M.fs[Q][R] + c[D] * M.fs[Q][D]) * SP + k, fqq = M.fs[Q][Q] * SP;
+        const int fqr = M.fs[Q][R] * SP;
+        // copies for row m (at edge i): line position m + 1, the faces and weights of row m
+        auto copy = [&](int m, int i, int stage) {
+            const bool in = m + 1 < last;
+            const int j = in ? i + es : i;
+            cp_async16_zfill(ring.at(stage, 0), xk + (in && !lo ? j - er : j), in && !lo);
+            cp_async16_zfill(ring.at(stage, 1), xk + j, in);
+            cp_async16_zfill(ring.at(stage, 2), xk + (in && !hi ? j + er : j), in && !hi);
+            cp_async16(ring.at(stage, 3), M.g + fr0 + m * frq);
+            cp_async16(ring.at(stage, 4), M.g + fq0 + m * fqq - fqr);
+            cp_async16(ring.at(stage, 5), M.g + fq0 + m * fqq);
+            float2 *w = reinterpret_cast<float2 *>(ring.at(stage, 6));
+            cp_async8(w, M.w + cell0 + m * M.cs[Q] - M.cs[R]);
+            cp_async8(w + 1, M.w + cell0 + m * M.cs[Q]);
+        };
+        int next = a, en = e, st_in = 0, st = 0;
 #pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int b = 0; b < 2; b++)
-            wm[a][b] = d2f(__ldg(M.w + (3 + D) * nc + r.cell + (a - 1) * M.cs[T1] + (b - 1) * M.cs[T2]));
-    const dfc g1a = from4(__ldg(M.g + (r.f1 - M.fs[T1][T2]) * SP + k));
-    const dfc g1b = from4(__ldg(M.g + r.f1 * SP + k));
-    const dfc g2a = from4(__ldg(M.g + (r.f2 - M.fs[T2][T1]) * SP + k));
-    const dfc g2b = from4(__ldg(M.g + r.f2 * SP + k));
-    acc kr, ki;
-    kr.add(g1a.re); kr.add(neg(g1b.re)); kr.add(neg(g2a.re)); kr.add(g2b.re);
-    ki.add(g1a.im); ki.add(neg(g1b.im)); ki.add(neg(g2a.im)); ki.add(g2b.im);
-    acc mr, mi;
-    const df s0_ = add(wm[0][0], wm[0][1]), s1_ = add(wm[1][0], wm[1][1]);
-    const df r0_ = add(wm[0][0], wm[1][0]), r1_ = add(wm[0][1], wm[1][1]);
-    const df cm[3][3] = {{wm[0][0], scale(s0_, 2.f), wm[0][1]},
-                         {scale(r0_, 2.f), scale(add(s0_, s1_), 4.f), scale(r1_, 2.f)},
-                         {wm[1][0], scale(s1_, 2.f), wm[1][1]}};
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) {
-            dfc xe{df{0.f, 0.f}, df{0.f, 0.f}};
-            if (!mf_mass_dir(r, a, b)) xe = from4(__ldg(x + mf_mass_edge(M, r, a, b) * SP + k));
-            mr.mac(cm[a][b], xe.re);
-            mi.mac(cm[a][b], xe.im);
+        for (int s = 0; s < kStages - 1; s++) {
+            if (next < b) copy(next, en, st_in);
+            cp_async_commit();
+            next++;
+            en += es;
+            st_in++;
         }
-    const df mxr = mr.get(), mxi = mi.get();
-    kr.mac(neg(om), mxi);
-    ki.mac(om, mxr);
-    return dfc{kr.get(), ki.get()};
+        // P_lo and P_hi of a line position (0 on the surface)
+        auto sums = [&](cdf xc, cdf xl, cdf xh, acc2 &plo, acc2 &phi) {
+            const cdf x2{add2(xc.h, xc.h), add2(xc.l, xc.l)};
+            plo.start(x2);
+            plo.add(xl);
+            phi.start(x2);
+            phi.add(xh);
+        };
+        auto line = [&](int i, acc2 &plo, acc2 &phi) {
+            const cdf xc = cdf_of(__ldg(xk + i));
+            sums(xc, lo ? czero() : cdf_of(__ldg(xk + i - er)), hi ? czero() : cdf_of(__ldg(xk + i + er)),
+                 plo, phi);
+            return xc;
+        };
+        acc2 pl0, ph0, pl1, ph1;
+        if (a > 1) line(e - es, pl0, ph0);
+        cdf x1 = line(e, pl1, ph1);
+        df wl0 = d2f(__ldg(M.w + cell0 + (a - 1) * M.cs[Q] - M.cs[R])),
+           wh0 = d2f(__ldg(M.w + cell0 + (a - 1) * M.cs[Q]));
+        cdf gr = cdf_of(__ldg(M.g + fr0 + (a - 1) * frq));
+        const cdf fom{pk(-om.h, om.h), pk(-om.l, om.l)};
+        for (int m = a; m < b; m++) {
+            if (next < b) copy(next, en, st_in);
+            cp_async_commit();
+            next++;
+            en += es;
+            st_in = st_in == kStages - 1 ? 0 : st_in + 1;
+            cp_async_wait<kStages - 1>();
+            auto value = [&](int v) { return cdf_of(*ring.at(st, v)); };
+            const cdf x2 = value(1);
+            acc2 pl2, ph2;
+            sums(x2, value(0), value(2), pl2, ph2);
+            const float4 w = *ring.at(st, 6);
+            const df wl1{w.x, w.y}, wh1{w.z, w.w};
+            // the mass part: 2 P(m) + P(m - 1) and 2 P(m) + P(m + 1)
+            acc2 mm;
+            auto cells = [&](const acc2 &p0, const acc2 &p1, const acc2 &p2, df w0, df w1, bool first) {
+                const cdf d{add2(p1.h, p1.h), add2(p1.l, p1.l)};
+                acc2 u, v;
+                u.start(d);
+                u.add(cdf{p0.h, p0.l});
+                v.start(d);
+                v.add(cdf{p2.h, p2.l});
+                if (first) mm.first(both(w0), cdf{u.h, u.l});
+                else mm.mac(both(w0), cdf{u.h, u.l});
+                mm.mac(both(w1), cdf{v.h, v.l});
+            };
+            cells(pl0, pl1, pl2, wl0, wl1, true);
+            cells(ph0, ph1, ph2, wh0, wh1, false);
+            const cdf gn = value(3), ga = value(4), gb = value(5);
+            acc2 kk;
+            kk.start(FLIP ? gn : gr);
+            kk.sub(FLIP ? gr : gn);
+            kk.sub(FLIP ? gb : ga);
+            kk.add(FLIP ? ga : gb);
+            kk.mac(fom, cswap(mm.get()));
+            tail.row(e + k, kk.get(), x1, z);
+            st = st == kStages - 1 ? 0 : st + 1;
+            e += es;
+            gr = gn;
+            pl0 = pl1; ph0 = ph1;
+            pl1 = pl2; ph1 = ph2;
+            wl0 = wl1; wh0 = wh1;
+            x1 = x2;
+        }
+    }
 }
 
-// z = A s in the D^T (F f) form, with the SpMV tail of k_spmv
 template <int SP>
-__global__ void __launch_bounds__(kB)
-k_mf_edges_g(int nb, MF M, const float2 *__restrict__ omega, const float4 *__restrict__ s,
-             float4 *__restrict__ z,
-             SysState *sys, float4 *partials, int mode, int rev)
+__global__ void __launch_bounds__(kB, 2)
+k_mf_edges_g(MF M, March E, const float2 *__restrict__ omega, const float4 *__restrict__ s,
+             float4 *__restrict__ z, SysState *sys, float4 *partials, int mode, int rev)
 {
     pdl_wait();
+    extern __shared__ __align__(16) float4 ring_smem[];
     const int k = threadIdx.x % SP;
     const bool on = sys[k].status == kRun;
     const df om = d2f(omega[k]);
+    const Ring<kEdgeValues> ring{ring_smem};
     SpmvTail tail;
-    const int rpb = kB / SP, stride = gridDim.x * rpb;
-    // the next row's position is loaded one row ahead
-    const int r0 = blockIdx.x * rpb + threadIdx.x / SP;
-    unsigned cn = on && r0 < nb ? __ldg(M.pos + sweep(r0, nb, rev)) : 0u;
-    for (int ri = r0; ri < nb; ri += stride) {
+    const int rpb = kB / SP;
+    for (int qi = blockIdx.x * rpb + threadIdx.x / SP; qi < E.items; qi += gridDim.x * rpb) {
         if (!on) break;
-        const unsigned c = cn;
-        if (ri + stride < nb) cn = __ldg(M.pos + sweep(ri + stride, nb, rev));
-        const int d = (int)(c >> 30);
-        const Pos p{(int)(c & 1023u), (int)((c >> 10) & 1023u), (int)((c >> 20) & 1023u)};
-        const int e = mf_edge(M, d, p.x, p.y, p.z);
-        const long long i = (long long)e * SP + k;
-        const float4 sv4 = __ldg(s + i);
-        dfc y;
-        if (mf_dirichlet(M, d, p.x, p.y, p.z))
-            y = from4(sv4);
-        else if (d == 0)
-            y = mf_row_g<SP, 0>(M, p, k, om, s);
-        else if (d == 1)
-            y = mf_row_g<SP, 1>(M, p, k, om, s);
-        else
-            y = mf_row_g<SP, 2>(M, p, k, om, s);
-        tail.row(i, y, sv4, z);
+        const int q = sweep(qi, E.items, rev);
+        const int tile = q / E.per_tile, r = q - tile * E.per_tile;
+        const int tz = tile / E.ty;
+        const int line = r / (M.nx - 1);
+        int c[3] = {r - line * (M.nx - 1), (tile - tz * E.ty) * E.ly, tz * E.lz};
+        // x- and y-edges: lines (x, y) along z; z-edges: lines (x, z) along y
+        if (line < E.ly) {
+            c[1] += line;
+            if (c[1] < M.ny - 1) mf_edge_march<SP, 0>(M, E.lz, c, om, k, s, z, tail, ring);
+        } else if (line < 2 * E.ly) {
+            c[1] += line - E.ly;
+            if (c[1] < M.ny - 1) mf_edge_march<SP, 1>(M, E.lz, c, om, k, s, z, tail, ring);
+        } else {
+            c[2] += line - 2 * E.ly;
+            if (c[2] < M.nz - 1) mf_edge_march<SP, 2>(M, E.ly, c, om, k, s, z, tail, ring);
+        }
+    }
+    // the rows on the outer surface are the identity
+    for (int qi = blockIdx.x * rpb + threadIdx.x / SP; qi < M.ndir; qi += gridDim.x * rpb) {
+        if (!on) break;
+        const long long i = (long long)__ldg(M.dir + qi) * SP + k;
+        const cdf sv = cdf_of(__ldg(s + i));
+        tail.row(i, sv, sv, z);
     }
     tail.finish<SP>(sys, partials, mode);
 }
@@ -1680,17 +1672,6 @@ struct TileMat {
     const int *uoff, *ucol;
     int T, ntiles, nslices;
 };
-
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gsrc) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all()
-{
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
 
 // shared-memory bytes of a tile: x segments, then K, M, K_real, local indices
 __host__ __device__ __forceinline__ long long tile_bytes(int nu, int SP, long long nc, long long nr)
@@ -1775,7 +1756,7 @@ k_spmv_t(int nb, TileMat A, const float2 *__restrict__ omega, const float4 *__re
                     const int t2 = b + 32 * q;
                     const float4 xv = xs[ldv(slc + t2, MAT) * SP + k];
                     const df kd = d2f(ldv(skc + t2, MAT)), md = d2f(ldv(smc + t2, MAT));
-                    const df xr{xv.x, xv.y}, xi{xv.z, xv.w};
+                    const df xr{xv.x, xv.z}, xi{xv.y, xv.w};
                     kr_.mac(kd, xr);
                     ki_.mac(kd, xi);
                     mr_.mac(md, xr);
@@ -1789,8 +1770,8 @@ k_spmv_t(int nb, TileMat A, const float2 *__restrict__ omega, const float4 *__re
                     const int t2 = b + 32 * q;
                     const float4 xv = xs[ldv(slr + t2, MAT) * SP + k];
                     const df kd = d2f(ldv(skr + t2, MAT));
-                    kr_.mac(kd, df{xv.x, xv.y});
-                    ki_.mac(kd, df{xv.z, xv.w});
+                    kr_.mac(kd, df{xv.x, xv.z});
+                    ki_.mac(kd, df{xv.y, xv.w});
                 }
             }
             const df mxr = mr_.get(), mxi = mi_.get();
@@ -1909,26 +1890,26 @@ k_group(long long n, float4 *__restrict__ s, float4 *__restrict__ p, double2 *__
     for (long long ii = (long long)blockIdx.x * kB + threadIdx.x; ii < n; ii += stride) {
         // n is a multiple of SP: a backward sweep by rows keeps the lane's system
         const long long i = rev ? n - SP - (ii - k) + k : ii;
-        dfc pv = from4(p[i]), d{df{0.f, 0.f}, df{0.f, 0.f}};
+        cdf pv = ldg(p + i), d = czero();
         const double2 xv = x[i];
         int j = 0;
         for (; j + 4 <= cnt; j += 4) {
-            float4 sv[4];
+            cdf sv[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) sv[u] = s[(j + u) * n + i];
+            for (int u = 0; u < 4; u++) sv[u] = ldg(s + (j + u) * n + i);
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                pv = caxpy(from4(sv[u]), from4(c[2 * (j + u) + 1]), pv);
-                d = caxpy(d, from4(c[2 * (j + u)]), pv);
+                pv = caxpy(sv[u], cfac_of(from4(c[2 * (j + u) + 1])), pv);
+                d = caxpy(d, cfac_of(from4(c[2 * (j + u)])), pv);
             }
         }
         for (; j < cnt; j++) {
-            pv = caxpy(from4(s[j * n + i]), from4(c[2 * j + 1]), pv);
-            d = caxpy(d, from4(c[2 * j]), pv);
+            pv = caxpy(cdf_of(s[j * n + i]), cfac_of(from4(c[2 * j + 1])), pv);
+            d = caxpy(d, cfac_of(from4(c[2 * j])), pv);
         }
         const float4 last = s[cnt * n + i];
-        x[i] = make_double2(xv.x + ((double)d.re.h + (double)d.re.l),
-                            xv.y + ((double)d.im.h + (double)d.im.l));
+        const double2 dv = to_d2(to4(d));
+        x[i] = make_double2(xv.x + dv.x, xv.y + dv.y);
         p[i] = to4(pv);
         s[i] = last;
     }
@@ -1948,18 +1929,38 @@ struct Impl {
                        V.uoff, V.ucol, V.tile_T, V.ntiles, P.nslices};
     }
     static void mfd_into(const Survey &V, MF &M) { M = mfd(V); }
-    // the work items of k_mf_gmarch
-    static GMarch gmarch(const Survey &V)
+    // The work of the marching kernels.  Chunk lengths: an item costs its
+    // positions plus about 3 for its start (the neighbours' values, the first
+    // loads' latency), so the length is the one with the least rounds of
+    // resident threads times that cost: 16 on large problems, down to 1 where
+    // longer ones would leave the chip idle.  Axes are cut evenly (41 cells
+    // into 3 chunks of 14, not 2 of 16 and one of 9).
+    static March march(const Survey &V, bool faces, long long threads)
     {
-        const MatFree &F = V.mf;
-        GMarch G;
-        G.ycols = G.zcols = F.nx - 1;
-        G.ych = ceil_div(F.ny, kMarch);
-        G.zch = ceil_div(F.nz, kMarch);
-        G.xitems = (int)F.nfx;
-        G.yitems = G.ycols * (F.nz - 1) * G.ych;
-        return G;
+        const int cx = V.mf.nx - 1, cy = V.mf.ny - 1, cz = V.mf.nz - 1;
+        March best;
+        long long cost = -1;
+        for (int len = 16; len >= 1; len--) {
+            March G;
+            G.ty = ceil_div(cy, len);
+            G.tz = ceil_div(cz, len);
+            G.ly = ceil_div(cy, G.ty);
+            G.lz = ceil_div(cz, G.tz);
+            G.lx = ceil_div(cx, ceil_div(cx, len));
+            G.ty = ceil_div(cy, G.ly);
+            G.tz = ceil_div(cz, G.lz);
+            G.per_tile = faces ? (G.lz + G.ly) * cx + ceil_div(cx, G.lx) * G.ly * G.lz : (2 * G.ly + G.lz) * cx;
+            G.items = G.ty * G.tz * G.per_tile;
+            const long long c = ((long long)G.items * SP + threads - 1) / threads *
+                                (std::max({G.ly, G.lz, faces ? G.lx : 1}) + 3);
+            if (cost < 0 || c < cost) {
+                cost = c;
+                best = G;
+            }
+        }
+        return best;
     }
+    static constexpr int kEdgeSmem = kStages * kEdgeValues * kB * 16;
     static MF mfd(const Survey &V)
     {
         const MatFree &F = V.mf;
@@ -1976,6 +1977,8 @@ struct Impl {
         M.w = F.w;
         M.f = F.f;
         M.g = F.g;
+        M.dir = F.dir;
+        M.ndir = F.ndir;
         return M;
     }
     // h = D_S G (src + beta a): the lattice form where G is the lattice's
@@ -2002,9 +2005,9 @@ struct Impl {
         }
         if (V.ch == kMatFree + 3) {
             const MF M = mfd(V);
-            pdl(k_mf_gmarch<SP>, V.g_mfg, kB, 0, V.st, M, gmarch(V), s, V.sys, flip(V));
-            pdl(k_mf_edges_g<SP>, V.g_mfe3, kB, 0, V.st, V.nb, M, V.omega, s, V.z, V.sys,
-                                                       V.partials, mode, flip(V));
+            pdl(k_mf_gmarch<SP>, V.g_mfg, kB, 0, V.st, M, V.mg, s, V.sys, flip(V));
+            pdl(k_mf_edges_g<SP>, V.g_mfe3, kB, kEdgeSmem, V.st, M, V.me, V.omega, s, V.z, V.sys,
+                V.partials, mode, flip(V));
             return;
         }
         if (V.ch == kMatFree || V.ch == kMatFree + 1) {
@@ -2077,8 +2080,10 @@ struct Impl {
             slot_s(V, j + 1), V.sys, V.hist, V.partials, flip(V));
         spmv(V, 1, slot_s(V, j + 1));
         if (j == V.group - 1 || t == n - 1)
+            // (the iteration's sweep directions, and with them its sums, do not
+            // depend on the group's length)
             pdl(k_group<SP>, V.g_group, kB, 0, V.st, (long long)V.nb * SP, V.s, V.p, V.xacc, V.hist,
-                V.sys, flip(V));
+                V.sys, V.dir ^ 1);
     }
     // one preconditioner step of the iteration (mode 1), unfused or fused
     static void precond_step(Survey &V, bool fused, float4 *ain, float4 *aout)
@@ -2162,14 +2167,18 @@ struct Impl {
             V.g_mff = g((const void *)k_mf_faces<SP>, (int)std::min<long long>(
                                                           (nn + kB / SP - 1) / (kB / SP), INT_MAX));
             V.g_mfe = g((const void *)k_mf_edges<SP>, V.grid_rows);
-            {
-                const GMarch G = gmarch(V);
-                const long long items = (long long)G.xitems + G.yitems +
-                                        (long long)G.zcols * (V.mf.ny - 1) * G.zch;
-                V.g_mfg = g((const void *)k_mf_gmarch<SP>, (int)std::min<long long>(
-                                                               (items + kB / SP - 1) / (kB / SP), INT_MAX));
-            }
-            V.g_mfe3 = g((const void *)k_mf_edges_g<SP>, V.grid_rows);
+            auto gs = [&](const void *f, int smem, bool faces, March &G) {
+                int b = 0;
+                if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kB, smem) != cudaSuccess || b < 1) {
+                    cudaGetLastError();
+                    b = 1;
+                }
+                G = march(V, faces, (long long)b * nsm * kB);
+                return std::max(1, std::min(b * nsm, ceil_div(G.items, kB / SP)));
+            };
+            V.g_mfg = gs((const void *)k_mf_gmarch<SP>, 0, true, V.mg);
+            V.g_mfe3 = gs((const void *)k_mf_edges_g<SP>, kEdgeSmem, false, V.me);
             if constexpr (SP >= 2) {
                 if (V.ch == kMatFree + 1)
                     V.g_mfe = g((const void *)k_mf_edges2<SP>,
