@@ -202,14 +202,5 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
             }
     }
     const tf v[2] = {tf_of(d[0]), tf_of(d[1])};
-    __shared__ double tot[2][32];
-    if (sys_grid_sum<SP, 2, NT>(v, partials, tot) && threadIdx.x < SP) {
-        SysState &q = sys[threadIdx.x];
-        if (first) q.cnt = 0;
-        if (q.status == kRun) {
-            const double2 aw = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
-            if (fabs(aw.x) < 1e-40 && fabs(aw.y) < 1e-40) q.status = MTGPU_DIV_BY_ZERO;
-            else set_alpha(q, cdiv(q.zs, aw));
-        }
-    }
+    finish_alpha<SP, NT>(v, sys, partials, first);
 }

@@ -17,7 +17,7 @@ struct SysState {
     double eps_k;          // the inner stop threshold on residual_rel
     double bnorm;          // ||b|| of the system (FP64)
     double rnorm;          // ||b - A x|| of the last FP64 residual evaluation
-    double res_next;       // ||s_m|| after this iteration's MRS step (k_update), for the stop test
+    double res2_next;      // ||s_m||^2 after this iteration's MRS step (k_update), for the stop test; mode 0: as before
     int mrs_mode;          // 0 keep s_m, 1 s_m = r, 2 s_m += w (r - s_m): the step the next k_update applies
     int cnt;               // iterations recorded in the present group (k_group applies them to p and x)
     int status;            // 1 running, else MTGPU_OK / MTGPU_DIV_BY_ZERO / MTGPU_MAXITER / MTGPU_X0_NULL

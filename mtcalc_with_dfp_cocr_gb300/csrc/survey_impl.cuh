@@ -120,12 +120,27 @@ struct GridSum {
         return tf{__shfl_xor_sync(0xffffffffu, x.a, o), __shfl_xor_sync(0xffffffffu, x.b, o),
                   __shfl_xor_sync(0xffffffffu, x.c, o)};
     }
-    // the totals of `rows` partials in threads t < W
+    // the totals of `rows` partials in threads t < W: up to 12 loads a thread
+    // in flight, added pairwise (one load latency for 456 blocks x 2 systems;
+    // a loop of dependent adds took 4,300 cycles)
     static __device__ __forceinline__ float4 rows(const float4 *part, int rows, float4 *sm)
     {
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-        for (int i = threadIdx.x; i < rows * W; i += NT) s = tf4_add(s, __ldcg(part + i));
+        constexpr int U = 12;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 s = zero;
+        for (int i0 = 0; i0 < rows * W; i0 += U * NT) {
+            float4 v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int i = i0 + u * NT + threadIdx.x;
+                v[u] = i < rows * W ? __ldcg(part + i) : zero;
+            }
+#pragma unroll
+            for (int h = 1; h < U; h <<= 1)
+#pragma unroll
+                for (int u = 0; u + h < U; u += 2 * h) v[u] = tf4_add(v[u], v[u + h]);
+            s = i0 == 0 ? v[0] : tf4_add(s, v[0]);
+        }
         __syncthreads();
         return block_rows(s, sm);
     }
@@ -165,12 +180,12 @@ __device__ bool sys_grid_sum(const tf (&v)[N], float4 *partials, double (*tot)[3
         if (threadIdx.x < W) __stcg(dst + threadIdx.x, s);
         __syncthreads();
         if (threadIdx.x == 0) {
-            __threadfence();      // the block's stores, ordered by the barrier
-            last = atomicAdd(ticket, 1u) == n - 1;
-            if (last) {
-                *ticket = 0u;
-                __threadfence();
-            }
+            // release: the block's stores, which the barrier ordered before
+            // this thread; acquire: those of the blocks counted before
+            unsigned int seen;
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(ticket) : "memory");
+            last = seen == n - 1;
+            if (last) *ticket = 0u;
         }
         __syncthreads();
         return last;
@@ -488,6 +503,36 @@ k_init(int nb, const float4 *__restrict__ r, float4 *__restrict__ sm, SysState *
     }
 }
 
+// a / b of FP64 values that come from FP32 sums: |b|^2 is far inside FP64's
+// range, so the quotient is formed from it directly, one divide deep instead
+// of the two of a division scaled against overflow
+__device__ __forceinline__ double2 cquot(double2 a, double2 b)
+{
+    const double d = b.x * b.x + b.y * b.y;
+    return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
+}
+
+// (a, w) -> alpha, by the block that finishes last.  Here and in the other
+// finishers the state is read before the sum, so that its latency passes
+// behind the sum's, and independent FP64 chains (a divide or a square root is
+// 500 cycles) run side by side.
+template <int SP, int NT>
+__device__ __forceinline__ void finish_alpha(const tf (&v)[2], SysState *sys, float4 *partials, int first)
+{
+    __shared__ double tot[2][32];
+    SysState &q = sys[threadIdx.x % SP];
+    const double2 zs = q.zs;
+    const int status = q.status;
+    if (sys_grid_sum<SP, 2, NT>(v, partials, tot) && threadIdx.x < SP) {
+        if (first) q.cnt = 0;
+        if (status == kRun) {
+            const double2 aw = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
+            if (fabs(aw.x) < 1e-40 && fabs(aw.y) < 1e-40) q.status = MTGPU_DIV_BY_ZERO;
+            else set_alpha(q, cquot(zs, aw));
+        }
+    }
+}
+
 // h = D_S G (z + beta a); use_beta = 0: h = D_S G z
 template <int SP>
 __global__ void __launch_bounds__(kB)
@@ -523,7 +568,7 @@ k_node(int m, const int *__restrict__ gp, const int *__restrict__ gj, const floa
 // beta p and x += alpha p are k_group's: reading s and p and x here and
 // writing p and x were 5 of this kernel's 11 vector passes.
 template <int SP>
-__global__ void __launch_bounds__(kB)
+__global__ void __launch_bounds__(kB, 4)
 k_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj, const float *__restrict__ tv,
        const int2 *__restrict__ tn, const float4 *__restrict__ da, const float4 *__restrict__ h,
        const float4 *__restrict__ z, float4 *__restrict__ a, float4 *__restrict__ w, SysState *sys,
@@ -575,16 +620,7 @@ k_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj, const floa
     }
     if (mode == 0) return;
     const tf v[2] = {tf_diff(aw1), tf_sum(aw2)};
-    __shared__ double tot[2][32];
-    if (sys_grid_sum<SP, 2>(v, partials, tot) && threadIdx.x < SP) {
-        SysState &q = sys[threadIdx.x];
-        if (first) q.cnt = 0;
-        if (q.status == kRun) {
-            const double2 aw = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
-            if (fabs(aw.x) < 1e-40 && fabs(aw.y) < 1e-40) q.status = MTGPU_DIV_BY_ZERO;
-            else set_alpha(q, cdiv(q.zs, aw));
-        }
-    }
+    finish_alpha<SP, kB>(v, sys, partials, first);
 }
 
 // r -= alpha a, s -= alpha w, and the MRS smoothing of the residual
@@ -652,28 +688,25 @@ k_update(int n, const float4 *__restrict__ a, const float4 *__restrict__ w, floa
     }
     const tf v[4] = {tf_sum(su), tf_sum(uu), tf_sum(nn), tf_sum(rr)};
     __shared__ double tot[4][32];
-    if (sys_grid_sum<SP, 4>(v, partials, tot) && threadIdx.x < SP) {
-        SysState &q = sys[threadIdx.x];
-        if (q.status == kRun) {
-            const double s_u = tot[0][threadIdx.x], u_u = tot[1][threadIdx.x];
-            const double n_n = tot[2][threadIdx.x], r_r = tot[3][threadIdx.x];
-            const double wm = fabs(u_u) < 1e-100 ? 0.0 : -s_u / u_u;
-            if (wm < 0.0) {
-                q.mrs_mode = 0;
-                q.res_next = q.residual;
-            } else if (wm > 1.0) {
-                q.mrs_mode = 1;
-                q.res_next = r_r > 0.0 ? sqrt(r_r) : 0.0;
-            } else {
-                q.mrs_mode = 2;
-                set_mrs_w(q, wm);
-                const double m2 = n_n + 2.0 * wm * s_u + wm * wm * u_u;
-                q.res_next = m2 > 0.0 ? sqrt(m2) : 0.0;
-            }
-            const int c = min(q.cnt, kGroupIters - 1);
-            hist[2 * (threadIdx.x * kGroupIters + c)] = q.alpha_f;
-            hist[2 * (threadIdx.x * kGroupIters + c) + 1] = q.beta_f;
-            q.cnt = c + 1;
+    SysState &q = sys[threadIdx.x % SP];
+    const int status = q.status, c = min(q.cnt, kGroupIters - 1);
+    const float4 alpha_f = q.alpha_f, beta_f = q.beta_f;
+    if (sys_grid_sum<SP, 4>(v, partials, tot) && threadIdx.x < SP && status == kRun) {
+        const double s_u = tot[0][threadIdx.x], u_u = tot[1][threadIdx.x];
+        const double n_n = tot[2][threadIdx.x], r_r = tot[3][threadIdx.x];
+        hist[2 * (threadIdx.x * kGroupIters + c)] = alpha_f;
+        hist[2 * (threadIdx.x * kGroupIters + c) + 1] = beta_f;
+        q.cnt = c + 1;
+        const double wm = fabs(u_u) < 1e-100 ? 0.0 : -s_u / u_u;
+        if (wm < 0.0) {
+            q.mrs_mode = 0;
+        } else if (wm > 1.0) {
+            q.mrs_mode = 1;
+            q.res2_next = r_r;
+        } else {
+            q.mrs_mode = 2;
+            set_mrs_w(q, wm);
+            q.res2_next = n_n + 2.0 * wm * s_u + wm * wm * u_u;
         }
     }
 }
@@ -703,30 +736,31 @@ struct SpmvTail {
     }
     // the same from this thread's (z, s) re, im of system threadIdx.x % SP.
     // mode 1: the stop test on ||s_m|| of this iteration (k_update's
-    // res_next), then beta; mode 0 (set-up): (z, s) only
+    // res2_next), then beta; mode 0 (set-up): (z, s) only
     template <int SP, int NT = kB>
     static __device__ __forceinline__ void finish_v(const tf (&v)[2], SysState *sys,
                                                     float4 *partials, int mode)
     {
         __shared__ double tot[2][32];
-        if (sys_grid_sum<SP, 2, NT>(v, partials, tot) && threadIdx.x < SP) {
-            SysState &q = sys[threadIdx.x];
-            if (q.status == kRun) {
-                const double2 zs_new = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
-                if (mode == 0) {
-                    q.zs = zs_new;
-                } else {
-                    q.residual = q.res_next;
-                    q.residual_rel = q.residual / q.r_old;
-                    set_beta(q, cdiv(zs_new, q.zs));
-                    q.zs = zs_new;
-                    if (q.residual_rel < q.eps_k) {
-                        q.status = MTGPU_OK;
-                    } else {
-                        q.iter += 1;
-                        if (q.iter > q.maxiter) q.status = MTGPU_MAXITER;
-                    }
-                }
+        SysState &q = sys[threadIdx.x % SP];
+        const double2 zs = q.zs;
+        const double r_old = q.r_old, eps_k = q.eps_k, res2 = q.res2_next, res = q.residual;
+        const int status = q.status, mrs = q.mrs_mode, iter = q.iter, maxiter = q.maxiter;
+        if (sys_grid_sum<SP, 2, NT>(v, partials, tot) && threadIdx.x < SP && status == kRun) {
+            const double2 zs_new = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
+            q.zs = zs_new;
+            if (mode == 0) return;
+            const double2 beta = cquot(zs_new, zs);
+            const double residual = mrs == 0 ? res : (res2 > 0.0 ? sqrt(res2) : 0.0);
+            const double rel = residual / r_old;
+            set_beta(q, beta);
+            q.residual = residual;
+            q.residual_rel = rel;
+            if (rel < eps_k) {
+                q.status = MTGPU_OK;
+            } else {
+                q.iter = iter + 1;
+                if (iter + 1 > maxiter) q.status = MTGPU_MAXITER;
             }
         }
     }
