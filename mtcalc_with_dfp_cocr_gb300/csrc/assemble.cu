@@ -195,7 +195,9 @@ __global__ void k_row_fill(int nb, int nslices, const int *ec_ptr, const int *ec
         double h[3];
         cell_h(xyz, nver, nver_stride, cell, h);
         const int mat = nvkat[cell];
-        const double muc = mu[mat], sc = sig[mat];
+        const double sc = sig[mat];
+        BrickRow brick;
+        brick.init(li, h, mu[mat]);
         for (int lj = 0; lj < 12; lj++) {
             const int j = ed[(long long)cell * ed_stride + lj];
             // binary search of column j
@@ -207,8 +209,8 @@ __global__ void k_row_fill(int nb, int nslices, const int *ec_ptr, const int *ec
             }
             if (q < 0) continue;
             double b, c;
-            brick_entry(li, lj, h, b, c);
-            K[q] = __dadd_rn(K[q], __ddiv_rn(b, muc));
+            brick.entry(lj, b, c);
+            K[q] = __dadd_rn(K[q], b);
             M[q] = __dadd_rn(M[q], __dmul_rn(c, sc));
         }
     }

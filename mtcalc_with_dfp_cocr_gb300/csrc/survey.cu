@@ -102,16 +102,26 @@ __global__ void k_g_lattice_check(MF M, int m, const int *__restrict__ gp, const
 __global__ void k_maxdiff(long long n, const float4 *__restrict__ a, const float4 *__restrict__ b,
                           unsigned long long *out)
 {
-    double dm = 0.0, bm = 0.0;
+    // in FP32, so 0 iff all values are equal and within 2^-23 of the largest
+    // difference otherwise, one atomic per block: FP64 values and an atomic
+    // per thread took 590 us for 19.5M complex values
+    float dm = 0.f, bm = 0.f;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
         const float4 u = a[i], v = b[i];
-        const double2 ud = to_d2(u), vd = to_d2(v);
-        dm = fmax(dm, fmax(fabs(ud.x - vd.x), fabs(ud.y - vd.y)));
-        bm = fmax(bm, fmax(fabs(vd.x), fabs(vd.y)));
+        dm = fmaxf(dm, fmaxf(fabsf((u.x - v.x) + (u.z - v.z)), fabsf((u.y - v.y) + (u.w - v.w))));
+        bm = fmaxf(bm, fmaxf(fabsf(v.x + v.z), fabsf(v.y + v.w)));
     }
-    atomicMax(out, (unsigned long long)__double_as_longlong(dm));
-    atomicMax(out + 1, (unsigned long long)__double_as_longlong(bm));
+    __shared__ unsigned int mx[2];
+    if (threadIdx.x < 2) mx[threadIdx.x] = 0u;
+    __syncthreads();
+    // the order of non-negative floats is that of their bits
+    atomicMax(&mx[0], __float_as_uint(dm));
+    atomicMax(&mx[1], __float_as_uint(bm));
+    __syncthreads();
+    if (threadIdx.x < 2)
+        atomicMax(out + threadIdx.x,
+                  (unsigned long long)__double_as_longlong((double)__uint_as_float(mx[threadIdx.x])));
 }
 
 // a fixed pseudo-random test vector (double-float values in [-1, 1))
@@ -207,22 +217,45 @@ k_tile_cols(int nslices, int T, const long long *pc, const long long *pr, const 
     }
 }
 
-// system-major FP64 [S][nb] <-> row-major FP64 [nb][SP]
-__global__ void k_in64(int nb, int S, int SP, const double2 *src, double2 *dst)
+// System-major [S][nb] FP64 <-> row-major [nb][SP], FP64 or double-float.  A
+// block moves 32 rows of all systems through shared memory, so that both
+// sides are read and written in whole lines: element by element in the
+// row-major order, a warp of 32 systems touched 32 lines of the system-major
+// side for 16 bytes of each (32 systems x 610k rows: 283 -> 150 us in, 345 -> 150 us out).
+constexpr int kTRows = 32;
+__device__ __forceinline__ void row_store(double2 *p, double2 v) { *p = v; }
+__device__ __forceinline__ void row_store(float4 *p, double2 v) { *p = to4(from_d2(v)); }
+__device__ __forceinline__ double2 row_load(const double2 *p) { return *p; }
+__device__ __forceinline__ double2 row_load(const float4 *p) { return to_d2(*p); }
+
+template <class T>
+__global__ void __launch_bounds__(kB)
+k_to_rows(int nb, int S, int SP, const double2 *__restrict__ src, T *__restrict__ dst)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)nb * SP) return;
-    const int k = (int)(i % SP);
-    dst[i] = k < S ? src[(long long)k * nb + i / SP] : make_double2(0.0, 0.0);
+    __shared__ double2 t[32][kTRows + 1];
+    const int r0 = blockIdx.x * kTRows, l = threadIdx.x % kTRows;
+    if (r0 + l < nb)
+        for (int k = threadIdx.x / kTRows; k < S; k += kB / kTRows) t[k][l] = src[(long long)k * nb + r0 + l];
+    __syncthreads();
+    for (int i = threadIdx.x; i < kTRows * SP; i += kB) {
+        const int k = i % SP, r = i / SP;
+        if (r0 + r < nb) row_store(dst + (long long)r0 * SP + i, k < S ? t[k][r] : make_double2(0.0, 0.0));
+    }
 }
 
-__global__ void k_out64(int nb, int S, int SP, const double2 *xacc, double2 *dst)
+template <class T>
+__global__ void __launch_bounds__(kB)
+k_from_rows(int nb, int S, int SP, const T *__restrict__ src, double2 *__restrict__ dst)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)nb * SP) return;
-    const int k = (int)(i % SP);
-    if (k >= S) return;
-    dst[(long long)k * nb + i / SP] = xacc[i];
+    __shared__ double2 t[32][kTRows + 1];
+    const int r0 = blockIdx.x * kTRows, l = threadIdx.x % kTRows;
+    for (int i = threadIdx.x; i < kTRows * SP; i += kB) {
+        const int k = i % SP, r = i / SP;
+        if (r0 + r < nb && k < S) t[k][r] = row_load(src + (long long)r0 * SP + i);
+    }
+    __syncthreads();
+    if (r0 + l < nb)
+        for (int k = threadIdx.x / kTRows; k < S; k += kB / kTRows) dst[(long long)k * nb + r0 + l] = t[k][l];
 }
 
 // ------------------------------------------------------- conversions
@@ -233,26 +266,6 @@ __global__ void k_to_df(long long n, const double *src, float2 *dst)
         const df v = from_double(src[i]);
         dst[i] = make_float2(v.h, v.l);
     }
-}
-
-// system-major FP64 [S][nb] -> row-major double-float [nb][SP]
-__global__ void k_in(int nb, int S, int SP, const double2 *src, float4 *dst)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)nb * SP) return;
-    const int k = (int)(i % SP);
-    const long long row = i / SP;
-    const double2 v = k < S ? src[(long long)k * nb + row] : make_double2(0.0, 0.0);
-    dst[i] = to4(from_d2(v));
-}
-
-__global__ void k_out(int nb, int S, int SP, const float4 *src, double2 *dst)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)nb * SP) return;
-    const int k = (int)(i % SP);
-    if (k >= S) return;
-    dst[(long long)k * nb + i / SP] = to_d2(src[i]);
 }
 
 // D_A[row][k] = 1 / (K_ii + i omega_k M_ii), computed in FP64
@@ -1414,11 +1427,10 @@ int survey_spmv(Survey &V, const double2 *x_sys_major, double2 *y_sys_major)
         init[k] = s;
     }
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
-    const long long tot = (long long)V.nb * V.SP;
-    const unsigned ge = (unsigned)((tot + kB - 1) / kB);
-    k_in<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, x_sys_major, V.s);
+    const unsigned gt = (unsigned)ceil_div(V.nb, kTRows);
+    k_to_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, x_sys_major, V.s);
     MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
-    k_out<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, V.z, y_sys_major);
+    k_from_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, V.z, y_sys_major);
     note_launches(2);
     MTGPU_TRY(cudaGetLastError());
     MTGPU_TRY(cudaStreamSynchronize(V.st));
@@ -1476,8 +1488,7 @@ void SurveyRun::release()
 int survey_begin(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, double eps,
                  int maxiter, int verify, int iters_per_launch, SurveyRun &R)
 {
-    const long long tot = (long long)V.nb * V.SP;
-    const unsigned ge = (unsigned)((tot + kB - 1) / kB);
+    const unsigned gt = (unsigned)ceil_div(V.nb, kTRows);
     R = SurveyRun{};
     R.x_out = x_sys_major;
     R.eps = eps;
@@ -1497,8 +1508,8 @@ int survey_begin(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, do
     }
     int rc;
     if ((rc = upload_sys(V))) return rc;
-    k_in64<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, b_sys_major, V.b64);
-    k_in64<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, x_sys_major, V.xacc);
+    k_to_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, b_sys_major, V.b64);
+    k_to_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, x_sys_major, V.xacc);
     note_launches(2);
     if ((rc = dev_alloc(&R.d_flag, 32))) return rc;
     // inner right-hand side r0 = b - A x0 (FP64), threshold relative to ||b||
@@ -1632,8 +1643,7 @@ int survey_collect(Survey &V, SurveyRun &R)
 
 int survey_finish(Survey &V, SurveyRun &R, mtgpu_survey_stats *stats, int stat_offset)
 {
-    const long long tot = (long long)V.nb * V.SP;
-    const unsigned ge = (unsigned)((tot + kB - 1) / kB);
+    const unsigned gt = (unsigned)ceil_div(V.nb, kTRows);
     int rc;
     // true residual of the systems that ended without a check
     bool any = false;
@@ -1646,7 +1656,7 @@ int survey_finish(Survey &V, SurveyRun &R, mtgpu_survey_stats *stats, int stat_o
         MTGPU_SP_DISPATCH(V.SP, res64(V, R.d_flag, 0));
         if ((rc = sync_sys(V))) return rc;
     }
-    k_out64<<<ge, kB, 0, V.st>>>(V.nb, V.S, V.SP, V.xacc, R.x_out);
+    k_from_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, V.xacc, R.x_out);
     note_launches(1);
     MTGPU_TRY(cudaGetLastError());
     MTGPU_TRY(cudaStreamSynchronize(V.st));
