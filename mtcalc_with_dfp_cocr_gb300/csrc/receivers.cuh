@@ -27,20 +27,21 @@ int locate_receivers(const ParamMatrix &P, int nrec, const double *d_rec, double
 struct Smoothing {
     int levels = 5;
     int nsub = 0;                    // [0]: curl A over all materials; [1..]: A per material
-    int npad = 0, ncell = 0, nblk = 0;
+    int npad = 0, ncell = 0;
     std::vector<int> sub_cells, sub_nodes, sub_material;
     int *d_cell = nullptr, *d_cell_sub = nullptr;     // [ncell] global brick, subdomain
     double *d_cell_g = nullptr;                       // [ncell] row sum of the brick mass matrix
     int *d_nc_ptr = nullptr, *d_nc = nullptr;         // padded node -> bricks (d_cell index)
-    int *d_mptr = nullptr, *d_mcol = nullptr;         // nodal mass matrix, padded rows
-    double *d_mval = nullptr, *d_mdiag = nullptr;
-    int *d_blk_sub = nullptr;                         // [nblk] subdomain of each node block
+    int2 *d_m32 = nullptr;                            // nodal mass matrix: column within the subdomain, FP32 value
+    double *d_m64 = nullptr;                          // ... FP64 value
+    float *d_dinv = nullptr;                          // 1 / diagonal
+    int *d_off = nullptr, *d_nn = nullptr;            // per subdomain: first padded node, nodes
     int *d_rn = nullptr;                              // [nrec][2][8] nodes (curl A, A); -1 none
     double *d_rw = nullptr;                           // [nrec][2][8] trilinear weights
     int S_cap = 0;
-    double *d_val = nullptr, *d_x = nullptr, *d_r = nullptr, *d_z = nullptr, *d_p = nullptr,
-           *d_q = nullptr, *d_scal = nullptr;
-    int *d_done = nullptr, *d_active = nullptr;
+    double *d_val = nullptr, *d_x = nullptr, *d_r = nullptr, *d_f = nullptr;
+    float *d_w = nullptr;                             // FP32 vectors of the projection
+    int *d_out = nullptr;
     int iterations = 0;
     void release();
 };

@@ -17,34 +17,45 @@
 //   * the receiver value is the trilinear interpolant of u in its brick.
 //
 // The reference factorises M with PARDISO and solves one value type at a
-// time.  Here every (subdomain, value type, system) is one column of a
-// batched Jacobi-preconditioned conjugate-gradient solve in FP64 to a
-// relative residual of 1e-14 (the diagonally scaled trilinear mass matrix
-// has a condition number below ~30, so 40-60 iterations), on all value
-// types of all systems at once.  The subdomains, the mass matrix and the
-// interpolation weights are built once per receiver set on the host; the
-// per-call work (centre values, right-hand sides, CG, interpolation) runs on
-// the device.
+// time.  Here every (subdomain, value type, system) is one column, solved by
+// iterative refinement: FP64 right-hand sides, solutions and residuals f - M u,
+// corrections by Jacobi-preconditioned conjugate gradients in FP32 (the
+// diagonally scaled trilinear mass matrix has a condition number below ~30,
+// so about 20 iterations gain five digits), until the FP64 residual is below
+// 1e-14 of the right-hand side: three to four rounds.  One block holds one
+// subdomain and two or four columns from the right-hand side to the solution:
+// no launches between iterations, and the matrix, read from L2, serves all of
+// its columns.  (CG in FP64, four launches an iteration, took 5.9 ms for 96
+// columns of 6,600 nodes; GB300 runs FP64 at 1/64 of FP32, and 27
+// multiply-adds a node, column and iteration are 27 us of its FP64 pipes.)
+// The subdomains, the mass matrix and the interpolation weights are built
+// once per receiver set on the host; the per-call work (centre values,
+// right-hand sides, projection, interpolation) runs on the device.
 //
 // Vector layout: [column][padded node], column = value * S + system with
-// values (x re, x im, y re, y im, z re, z im); every subdomain's node range
-// is padded to a multiple of the 256-thread block so that a block's rows
-// belong to one subdomain and its dot-product partials to one (subdomain,
-// column) problem.  Conforming (tensor) meshes only: no terminal nodes.
+// values (x re, x im, y re, y im, z re, z im); FP32 vectors [group
+// of columns][padded node][column].  Conforming (tensor) meshes only: no
+// terminal nodes.
 #include "rcv_eval.cuh"
 #include "receivers.cuh"
 
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
 
 namespace mtgpu {
 namespace {
 
-constexpr int kBlk = 256;            // nodes per block (padding unit)
+constexpr int kPad = 32;             // padding unit of a subdomain's nodes
+constexpr int kSolve = 512;          // threads of a solving block
 constexpr double kTol2 = 1e-28;      // (relative residual 1e-14)^2
-constexpr int kMaxIter = 2000;       // guard; the CG needs well under 100
-constexpr int kCheckEvery = 8;
+// A residual that has stopped falling is at FP64's own accuracy; accepted
+// below this square
+constexpr double kFloor2 = 1e-24;
+constexpr int kMaxOuter = 60;        // guards; four rounds of ~20 are needed
+constexpr int kMaxInner = 60;
+constexpr float kInner2 = 1e-10f;    // (a round's FP32 residual reduction)^2
 
 // brick-centre values: one thread per (brick of a subdomain, system)
 __global__ void k_sm_centre(int ncell, int S, const int *__restrict__ cell,
@@ -73,136 +84,253 @@ __global__ void k_sm_centre(int ncell, int S, const int *__restrict__ cell,
     }
 }
 
-template <int N>
-__device__ __forceinline__ void block_sum(double (&v)[N], double *out_addr[N])
+constexpr int kSlots = 27;           // matrix entries per node, padded
+
+// C FP32 values, one per column of the block
+template <int C>
+struct alignas(4 * C) vec {
+    float a[C];
+};
+template <int C>
+__device__ __forceinline__ vec<C> splat(float s)
 {
-    __shared__ double part[N][kBlk / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    vec<C> v;
 #pragma unroll
-    for (int n = 0; n < N; n++) {
-        double s = v[n];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) part[n][w] = s;
+    for (int c = 0; c < C; c++) v.a[c] = s;
+    return v;
+}
+template <int C>
+__device__ __forceinline__ vec<C> operator*(vec<C> x, vec<C> y)
+{
+#pragma unroll
+    for (int c = 0; c < C; c++) x.a[c] *= y.a[c];
+    return x;
+}
+template <int C>
+__device__ __forceinline__ vec<C> fma_(vec<C> x, vec<C> y, vec<C> z)
+{
+#pragma unroll
+    for (int c = 0; c < C; c++) z.a[c] = fmaf(x.a[c], y.a[c], z.a[c]);
+    return z;
+}
+// x / y where y > 0, else 0
+template <int C>
+__device__ __forceinline__ vec<C> quot(vec<C> x, vec<C> y)
+{
+#pragma unroll
+    for (int c = 0; c < C; c++) x.a[c] = y.a[c] > 0.f ? x.a[c] / y.a[c] : 0.f;
+    return x;
+}
+
+// Sums of C values per thread over the block, in a fixed order, to all
+// threads; buf: [warps] slots, alternated by the caller between calls.
+template <int C, class T>
+__device__ __forceinline__ void block_sum(T (&v)[C], T (*buf)[C])
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // halve the values a lane holds while lane bits are left to pick them,
+    // then add the lanes of each value
+    int o = 16, first = 0;
+#pragma unroll
+    for (int h = C / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+        first += up ? h : 0;
+#pragma unroll
+        for (int i = 0; i < h; i++) {
+            const T mine = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+            v[i] = mine + __shfl_xor_sync(0xffffffffu, give, o);
+        }
     }
+    const int rest = o;
+#pragma unroll
+    for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    if ((lane & (2 * rest - 1)) == 0) buf[w][first] = v[0];
     __syncthreads();
-    if (threadIdx.x < N) {
-        double s = 0.0;
-        for (int j = 0; j < kBlk / 32; j++) s += part[threadIdx.x][j];
-        atomicAdd(out_addr[threadIdx.x], s);
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        T s = buf[0][c];
+#pragma unroll
+        for (int q = 1; q < kSolve / 32; q++) s += buf[q][c];
+        v[c] = s;
     }
 }
 
-// problem scalars, [quantity][problem]
-enum { kRz = 0, kPq, kRz2, kRr, kFf, kBeta, kNq };
+struct SolveArgs {
+    int npad, ncol, ncell;
+    const int *off, *nn;                     // per subdomain: first padded node, nodes
+    const int *nc_ptr, *nc;                  // node -> bricks
+    const double *cell_g, *val;
+    // the mass matrix, kSlots entries a node (padded with zeros), slot by slot
+    // for every 32 nodes so that a warp reads whole lines: column within the
+    // subdomain and FP32 value, FP64 value
+    const int2 *m32;
+    const double *m64;
+    const float *dinv;                       // 1 / diagonal
+    double *x, *f, *r;                       // [column][padded node]
+    float *w;                                // FP32 vectors, 4 x [group][padded node][C]
+    int pcap;                                // bytes of shared memory for p
+    int *out;                                // columns that did not converge; largest iteration count
+};
 
-// f = sum over the node's bricks of g_c val_c; x = 0, r = f, z = f / diag,
-// p = z; (r, z) and (f, f) per problem
-__global__ void __launch_bounds__(kBlk)
-k_sm_init(int npad, int ncell, int nsub, const int *__restrict__ blk_sub,
-          const int *__restrict__ nc_ptr, const int *__restrict__ nc,
-          const double *__restrict__ cell_g, const double *__restrict__ val,
-          const double *__restrict__ diag, double *x, double *r, double *z, double *p,
-          double *scal, int nprob)
+// the projection of C columns (blockIdx.x) of one subdomain (blockIdx.y)
+template <int C>
+__global__ void __launch_bounds__(kSolve, 1)
+k_sm_solve(SolveArgs A)
 {
-    const int n = blockIdx.x * kBlk + threadIdx.x;
-    const int col = blockIdx.y;
-    const long long o = (long long)col * npad + n;
-    double f = 0.0;
-    for (int j = nc_ptr[n]; j < nc_ptr[n + 1]; j++) {
-        const int c = nc[j];
-        f += cell_g[c] * val[(long long)col * ncell + c];
+    using V = vec<C>;
+    extern __shared__ __align__(16) unsigned char psh[];
+    __shared__ double dbuf[2][kSolve / 32][C];
+    __shared__ float fbuf[2][kSolve / 32][C];
+    const int sub = blockIdx.y, n0 = A.off[sub], nn = A.nn[sub], tid = threadIdx.x;
+    const int c0 = C * blockIdx.x, nc = min(C, A.ncol - c0);
+    const long long nw = (long long)gridDim.x * A.npad;
+    V *const w = reinterpret_cast<V *>(A.w) + (long long)blockIdx.x * A.npad + n0;
+    V *const p = nn * (int)sizeof(V) <= A.pcap ? reinterpret_cast<V *>(psh) : w;
+    V *const r32 = w + nw, *const d32 = w + 2 * nw, *const q32 = w + 3 * nw;
+    const float *const dinv = A.dinv + n0;
+    const int2 *const m32 = A.m32 + (long long)n0 * kSlots;
+    const double *const m64 = A.m64 + (long long)n0 * kSlots;
+    auto slots = [](int n) { return (n >> 5) * (32 * kSlots) + (n & 31); };
+    double *x[C], *f[C], *r[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        const long long o = (long long)(c0 + min(c, nc - 1)) * A.npad + n0;
+        x[c] = A.x + o;
+        f[c] = A.f + o;
+        r[c] = A.r + o;
     }
-    const double zz = f / diag[n];
-    x[o] = 0.0;
-    r[o] = f;
-    z[o] = zz;
-    p[o] = zz;
-    const int pr = col * nsub + blk_sub[blockIdx.x];
-    double v[2] = {f * zz, f * f};
-    double *dst[2] = {scal + kRz * nprob + pr, scal + kFf * nprob + pr};
-    block_sum<2>(v, dst);
-}
-
-// a problem whose right-hand side is zero is done at the start
-__global__ void k_sm_start(int nprob, const double *scal, int *done)
-{
-    const int pr = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pr < nprob) done[pr] = !(scal[kFf * nprob + pr] > 0.0);
-}
-
-// q = M p, (p, q)
-__global__ void __launch_bounds__(kBlk)
-k_sm_spmv(int npad, int nsub, const int *__restrict__ blk_sub, const int *__restrict__ mptr,
-          const int *__restrict__ mcol, const double *__restrict__ mval,
-          const double *__restrict__ p, double *q, double *scal, const int *__restrict__ done,
-          int nprob)
-{
-    const int col = blockIdx.y;
-    const int pr = col * nsub + blk_sub[blockIdx.x];
-    if (done[pr]) return;   // uniform over the block
-    const int n = blockIdx.x * kBlk + threadIdx.x;
-    const double *pc = p + (long long)col * npad;
-    double s = 0.0;
-    for (int j = mptr[n]; j < mptr[n + 1]; j++) s += mval[j] * pc[mcol[j]];
-    q[(long long)col * npad + n] = s;
-    double v[1] = {pc[n] * s};
-    double *dst[1] = {scal + kPq * nprob + pr};
-    block_sum<1>(v, dst);
-}
-
-// x += alpha p, r -= alpha q, z = r / diag; (r, z), (r, r)
-__global__ void __launch_bounds__(kBlk)
-k_sm_update(int npad, int nsub, const int *__restrict__ blk_sub, const double *__restrict__ diag,
-            double *x, double *r, double *z, const double *__restrict__ p,
-            const double *__restrict__ q, double *scal, const int *__restrict__ done, int nprob)
-{
-    const int col = blockIdx.y;
-    const int pr = col * nsub + blk_sub[blockIdx.x];
-    if (done[pr]) return;
-    const int n = blockIdx.x * kBlk + threadIdx.x;
-    const long long o = (long long)col * npad + n;
-    const double pq = scal[kPq * nprob + pr];
-    const double al = pq > 0.0 ? scal[kRz * nprob + pr] / pq : 0.0;
-    x[o] += al * p[o];
-    const double rr = r[o] - al * q[o];
-    const double zz = rr / diag[n];
-    r[o] = rr;
-    z[o] = zz;
-    double v[2] = {rr * zz, rr * rr};
-    double *dst[2] = {scal + kRz2 * nprob + pr, scal + kRr * nprob + pr};
-    block_sum<2>(v, dst);
-}
-
-// per problem: beta, the stop test, reset of the partial sums; counts the
-// problems still running
-__global__ void k_sm_scalars(int nprob, double *scal, int *done, int *active)
-{
-    const int pr = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pr >= nprob || done[pr]) return;
-    const double rz = scal[kRz * nprob + pr], rz2 = scal[kRz2 * nprob + pr];
-    const bool stop = scal[kRr * nprob + pr] <= kTol2 * scal[kFf * nprob + pr] ||
-                      !(scal[kPq * nprob + pr] > 0.0) || !(rz > 0.0);
-    scal[kBeta * nprob + pr] = rz > 0.0 ? rz2 / rz : 0.0;
-    scal[kRz * nprob + pr] = rz2;
-    scal[kPq * nprob + pr] = 0.0;
-    scal[kRz2 * nprob + pr] = 0.0;
-    scal[kRr * nprob + pr] = 0.0;
-    if (stop)
-        done[pr] = 1;
-    else
-        atomicAdd(active, 1);
-}
-
-// p = z + beta p
-__global__ void __launch_bounds__(kBlk)
-k_sm_direction(int npad, int nsub, const int *__restrict__ blk_sub, const double *__restrict__ z,
-               double *p, const double *__restrict__ scal, const int *__restrict__ done, int nprob)
-{
-    const int col = blockIdx.y;
-    const int pr = col * nsub + blk_sub[blockIdx.x];
-    if (done[pr]) return;
-    const long long o = (long long)col * npad + blockIdx.x * kBlk + threadIdx.x;
-    p[o] = z[o] + scal[kBeta * nprob + pr] * p[o];
+    int flip = 0, total = 0;
+    auto sum = [&](V v) {
+        block_sum<C>(v.a, fbuf[flip]);
+        flip ^= 1;
+        return v;
+    };
+    // f = sum over the node's bricks of g_c val_c; x = 0, so r = f
+    double ff[C] = {}, rr[C], last[C] = {};
+    for (int n = tid; n < nn; n += kSolve)
+        for (int c = 0; c < nc; c++) {
+            double s = 0.0;
+            for (int j = A.nc_ptr[n0 + n]; j < A.nc_ptr[n0 + n + 1]; j++) {
+                const int e = A.nc[j];
+                s += A.cell_g[e] * A.val[(long long)(c0 + c) * A.ncell + e];
+            }
+            f[c][n] = s;
+            r[c][n] = s;
+            x[c][n] = 0.0;
+#pragma unroll
+            for (int q = 0; q < C; q++)
+                if (q == c) ff[q] += s * s;
+        }
+    block_sum<C>(ff, dbuf[flip]);
+    flip ^= 1;
+#pragma unroll
+    for (int c = 0; c < C; c++) rr[c] = ff[c];
+    bool done[C];
+    int open = 0;
+    for (int round = 0; round < kMaxOuter; round++) {
+        open = 0;
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            // (a NaN ends its column, as does a zero right-hand side)
+            done[c] = c >= nc || !(rr[c] > kTol2 * ff[c]) ||
+                      (round > 0 && rr[c] > 0.25 * last[c] && rr[c] <= kFloor2 * ff[c]);
+            open += !done[c];
+            last[c] = rr[c];
+        }
+        if (open == 0) break;
+        // FP32 correction M d = r / |r| of the open columns
+        double norm[C], scale[C];
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            norm[c] = done[c] ? 0.0 : sqrt(rr[c]);
+            scale[c] = norm[c] > 0.0 ? 1.0 / norm[c] : 0.0;
+        }
+        V rz = splat<C>(0.f);
+        for (int n = tid; n < nn; n += kSolve) {
+            V v;
+#pragma unroll
+            for (int c = 0; c < C; c++) v.a[c] = done[c] ? 0.f : (float)(r[c][n] * scale[c]);
+            const V z = v * splat<C>(dinv[n]);
+            r32[n] = v;
+            d32[n] = splat<C>(0.f);
+            p[n] = z;
+            rz = fma_(v, z, rz);
+        }
+        rz = sum(rz);
+        for (int it = 0; it < kMaxInner; it++) {
+            V pq = splat<C>(0.f);
+            for (int n = tid; n < nn; n += kSolve) {
+                V s = splat<C>(0.f);
+                const int2 *m = m32 + slots(n);
+#pragma unroll 9
+                for (int j = 0; j < kSlots; j++) {
+                    const int2 e = __ldg(m + 32 * j);
+                    s = fma_(splat<C>(__int_as_float(e.y)), p[e.x], s);
+                }
+                q32[n] = s;
+                pq = fma_(p[n], s, pq);
+            }
+            pq = sum(pq);
+            total++;
+            const V al = quot(rz, pq), nal = al * splat<C>(-1.f);
+            V rz2 = splat<C>(0.f), r2 = rz2;
+            for (int n = tid; n < nn; n += kSolve) {
+                d32[n] = fma_(al, p[n], d32[n]);
+                const V v = fma_(nal, q32[n], r32[n]);
+                r32[n] = v;
+                r2 = fma_(v, v, r2);
+                rz2 = fma_(v, v * splat<C>(dinv[n]), rz2);
+            }
+            r2 = sum(r2);
+            bool more = false;
+#pragma unroll
+            for (int c = 0; c < C; c++) more |= r2.a[c] > kInner2;
+            if (!more) break;
+            rz2 = sum(rz2);
+            const V be = quot(rz2, rz);
+            rz = rz2;
+            for (int n = tid; n < nn; n += kSolve) p[n] = fma_(be, p[n], r32[n] * splat<C>(dinv[n]));
+            __syncthreads();
+        }
+        // x += |r| d, r = f - M x in FP64
+        for (int n = tid; n < nn; n += kSolve) {
+            const V d = d32[n];
+#pragma unroll
+            for (int c = 0; c < C; c++)
+                if (!done[c]) x[c][n] += norm[c] * (double)d.a[c];
+        }
+        __syncthreads();
+        double s2[C] = {};
+        for (int n = tid; n < nn; n += kSolve) {
+            double s[C];
+#pragma unroll
+            for (int c = 0; c < C; c++) s[c] = done[c] ? 0.0 : f[c][n];
+            const int at = slots(n);
+#pragma unroll 3
+            for (int j = 0; j < kSlots; j++) {
+                const double m = m64[at + 32 * j];
+                const int col = m32[at + 32 * j].x;
+#pragma unroll
+                for (int c = 0; c < C; c++)
+                    if (!done[c]) s[c] -= m * x[c][col];
+            }
+#pragma unroll
+            for (int c = 0; c < C; c++)
+                if (!done[c]) {
+                    r[c][n] = s[c];
+                    s2[c] += s[c] * s[c];
+                }
+        }
+        block_sum<C>(s2, dbuf[flip]);
+        flip ^= 1;
+#pragma unroll
+        for (int c = 0; c < C; c++)
+            if (!done[c]) rr[c] = s2[c];
+    }
+    if (tid == 0) {
+        if (open > 0) atomicAdd(A.out, open);
+        atomicMax(A.out + 1, total);
+    }
 }
 
 // receiver values (trilinear interpolation of the nodal solutions) and the
@@ -303,22 +431,19 @@ void Smoothing::release()
     dev_free(d_cell_g);
     dev_free(d_nc_ptr);
     dev_free(d_nc);
-    dev_free(d_mptr);
-    dev_free(d_mcol);
-    dev_free(d_mval);
-    dev_free(d_mdiag);
-    dev_free(d_blk_sub);
+    dev_free(d_m64);
+    dev_free(d_off);
+    dev_free(d_nn);
+    dev_free(d_m32);
+    dev_free(d_dinv);
     dev_free(d_rn);
     dev_free(d_rw);
     dev_free(d_val);
     dev_free(d_x);
     dev_free(d_r);
-    dev_free(d_z);
-    dev_free(d_p);
-    dev_free(d_q);
-    dev_free(d_scal);
-    dev_free(d_done);
-    dev_free(d_active);
+    dev_free(d_f);
+    dev_free(d_w);
+    dev_free(d_out);
     S_cap = 0;
 }
 
@@ -394,23 +519,23 @@ int smoothing_build(Smoothing &sm, const ::mtgpu_assembly_s &a, int nrec, const 
     std::vector<int> node_off(sm.nsub + 1, 0), cell_off(sm.nsub + 1, 0);
     for (int s = 0; s < sm.nsub; s++) {
         const int nn = (int)subs[s].nodes.size();
-        node_off[s + 1] = node_off[s] + (nn + kBlk - 1) / kBlk * kBlk;
+        node_off[s + 1] = node_off[s] + (nn + kPad - 1) / kPad * kPad;
         cell_off[s + 1] = cell_off[s] + (int)subs[s].cells.size();
         sm.sub_cells.push_back((int)subs[s].cells.size());
         sm.sub_nodes.push_back(nn);
     }
     sm.npad = node_off[sm.nsub];
     sm.ncell = cell_off[sm.nsub];
-    sm.nblk = sm.npad / kBlk;
-    std::vector<int> cell(sm.ncell), cell_sub(sm.ncell), blk_sub(sm.nblk);
-    std::vector<double> cell_g(sm.ncell), mdiag(sm.npad, 1.0);
-    std::vector<int> mptr(sm.npad + 1, 0), mcol, nc_ptr(sm.npad + 1, 0), nc;
-    std::vector<double> mval;
+    std::vector<int> cell(sm.ncell), cell_sub(sm.ncell);
+    std::vector<double> cell_g(sm.ncell);
+    std::vector<float> dinv(sm.npad, 1.f);
+    std::vector<int2> m32((size_t)sm.npad * kSlots, make_int2(0, 0));
+    std::vector<double> m64((size_t)sm.npad * kSlots, 0.0);
+    std::vector<int> nc_ptr(sm.npad + 1, 0), nc;
     std::vector<int> loc(P.kuzlov, -1);
     for (int s = 0; s < sm.nsub; s++) {
         const SubBuild &B = subs[s];
         const int n0 = node_off[s], nn = (int)B.nodes.size();
-        for (int b = node_off[s] / kBlk; b < node_off[s + 1] / kBlk; b++) blk_sub[b] = s;
         for (int i = 0; i < nn; i++) loc[B.nodes[i]] = i;
         // rows of up to 27 (column, value) slots
         std::vector<int> rc(27 * (size_t)nn, -1), cnt(nn, 0);
@@ -456,19 +581,18 @@ int smoothing_build(Smoothing &sm, const ::mtgpu_assembly_s &a, int nrec, const 
             std::vector<std::pair<int, double>> row(cnt[i]);
             for (int q = 0; q < cnt[i]; q++) row[q] = {rc[base + q], rv[base + q]};
             std::sort(row.begin(), row.end());
-            for (auto &e : row) {
-                mcol.push_back(n0 + e.first);
-                mval.push_back(e.second);
-                if (e.first == i) mdiag[n0 + i] = e.second;
+            const size_t at = (size_t)n0 * kSlots + (size_t)(i >> 5) * (32 * kSlots) + (i & 31);
+            for (int q = 0; q < cnt[i]; q++) {
+                const float v32 = (float)row[q].second;
+                m32[at + 32 * q].x = row[q].first;
+                memcpy(&m32[at + 32 * q].y, &v32, sizeof(float));
+                m64[at + 32 * q] = row[q].second;
+                if (row[q].first == i) dinv[n0 + i] = (float)(1.0 / row[q].second);
             }
-            mptr[n0 + i + 1] = (int)mcol.size();
             for (int c : adj[i]) nc.push_back(c);
             nc_ptr[n0 + i + 1] = (int)nc.size();
         }
-        for (int i = nn; i < node_off[s + 1] - n0; i++) {   // padding rows
-            mptr[n0 + i + 1] = (int)mcol.size();
-            nc_ptr[n0 + i + 1] = (int)nc.size();
-        }
+        for (int i = nn; i < node_off[s + 1] - n0; i++) nc_ptr[n0 + i + 1] = (int)nc.size();   // padding rows
         for (int i = 0; i < nn; i++) loc[B.nodes[i]] = -1;
     }
     // receivers: padded nodes and trilinear weights of their brick, per type
@@ -494,11 +618,11 @@ int smoothing_build(Smoothing &sm, const ::mtgpu_assembly_s &a, int nrec, const 
     int rc;
     if ((rc = upload(&sm.d_cell, cell, st)) || (rc = upload(&sm.d_cell_sub, cell_sub, st)) ||
         (rc = upload(&sm.d_cell_g, cell_g, st)) || (rc = upload(&sm.d_nc_ptr, nc_ptr, st)) ||
-        (rc = upload(&sm.d_nc, nc, st)) || (rc = upload(&sm.d_mptr, mptr, st)) ||
-        (rc = upload(&sm.d_mcol, mcol, st)) || (rc = upload(&sm.d_mval, mval, st)) ||
-        (rc = upload(&sm.d_mdiag, mdiag, st)) || (rc = upload(&sm.d_blk_sub, blk_sub, st)) ||
+        (rc = upload(&sm.d_nc, nc, st)) || (rc = upload(&sm.d_m64, m64, st)) ||
+        (rc = upload(&sm.d_m32, m32, st)) || (rc = upload(&sm.d_dinv, dinv, st)) ||
+        (rc = upload(&sm.d_off, node_off, st)) || (rc = upload(&sm.d_nn, sm.sub_nodes, st)) ||
         (rc = upload(&sm.d_rn, rn, st)) || (rc = upload(&sm.d_rw, rw, st)) ||
-        (rc = dev_alloc(&sm.d_active, 1)))
+        (rc = dev_alloc(&sm.d_out, 2)))
         return rc;
     MTGPU_TRY(cudaStreamSynchronize(st));   // the host vectors go out of scope
     return MTGPU_OK;
@@ -511,61 +635,52 @@ int smoothing_fields(Smoothing &sm, const ParamMatrix &P, int nrec, int S, long 
                      cudaStream_t st)
 {
     // grow-only work arrays
-    const int ncol = 6 * S, nprob = ncol * sm.nsub;
+    const int ncol = 6 * S;
     if (S > sm.S_cap) {
-        for (double **p : {&sm.d_val, &sm.d_x, &sm.d_r, &sm.d_z, &sm.d_p, &sm.d_q, &sm.d_scal})
-            dev_free(*p);
-        dev_free(sm.d_done);
+        for (double **p : {&sm.d_val, &sm.d_x, &sm.d_r, &sm.d_f}) dev_free(*p);
+        dev_free(sm.d_w);
         sm.S_cap = 0;
         const size_t nv = (size_t)ncol * sm.npad;
         int rc;
         if ((rc = dev_alloc(&sm.d_val, (size_t)ncol * std::max(sm.ncell, 1))) ||
             (rc = dev_alloc(&sm.d_x, nv)) || (rc = dev_alloc(&sm.d_r, nv)) ||
-            (rc = dev_alloc(&sm.d_z, nv)) || (rc = dev_alloc(&sm.d_p, nv)) ||
-            (rc = dev_alloc(&sm.d_q, nv)) || (rc = dev_alloc(&sm.d_scal, (size_t)kNq * nprob)) ||
-            (rc = dev_alloc(&sm.d_done, (size_t)nprob)))
+            (rc = dev_alloc(&sm.d_f, nv)) || (rc = dev_alloc(&sm.d_w, (size_t)4 * (ncol + 3) * sm.npad)))
             return rc;
         sm.S_cap = S;
     }
-    MTGPU_TRY(cudaMemsetAsync(sm.d_scal, 0, sizeof(double) * kNq * nprob, st));
     unsigned long long launches = 0;
     sm.iterations = 0;
     if (sm.npad > 0) {
         k_sm_centre<<<dim3(ceil_div(sm.ncell, kThreads), S), kThreads, 0, st>>>(
             sm.ncell, S, sm.d_cell, sm.d_cell_sub, P.d_nver, P.nver_stride, P.d_ed, P.ed_stride,
             P.d_xyz, x_stride, d_x, sm.d_val);
-        const dim3 grid(sm.nblk, ncol);
-        k_sm_init<<<grid, kBlk, 0, st>>>(sm.npad, sm.ncell, sm.nsub, sm.d_blk_sub, sm.d_nc_ptr,
-                                         sm.d_nc, sm.d_cell_g, sm.d_val, sm.d_mdiag, sm.d_x,
-                                         sm.d_r, sm.d_z, sm.d_p, sm.d_scal, nprob);
-        const int gp = ceil_div(nprob, kThreads);
-        k_sm_start<<<gp, kThreads, 0, st>>>(nprob, sm.d_scal, sm.d_done);
-        launches += 3;
+        // four columns a block share the matrix's reads; two where four would
+        // leave more than a third of the SMs without a block
+        int dev = 0, nsm = 1;
+        MTGPU_TRY(cudaGetDevice(&dev));
+        MTGPU_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        const int C = 3LL * ceil_div(ncol, 4) * sm.nsub >= 2LL * nsm ? 4 : 2, groups = ceil_div(ncol, C);
+        // p of a subdomain in shared memory where it fits (12,800 nodes at
+        // four columns), else in L2
+        constexpr int kSmem = 200 * 1024;
+        int widest = 0;
+        for (int n : sm.sub_nodes) widest = std::max(widest, n);
+        const int smem = (int)std::min<long long>(kSmem, (long long)widest * 4 * C);
+        const SolveArgs A{sm.npad, ncol, sm.ncell, sm.d_off, sm.d_nn, sm.d_nc_ptr, sm.d_nc, sm.d_cell_g,
+                          sm.d_val, sm.d_m32, sm.d_m64, sm.d_dinv, sm.d_x, sm.d_f, sm.d_r, sm.d_w, smem,
+                          sm.d_out};
+        MTGPU_TRY(cudaMemsetAsync(sm.d_out, 0, 2 * sizeof(int), st));
+        const void *solve = C == 4 ? (const void *)k_sm_solve<4> : (const void *)k_sm_solve<2>;
+        MTGPU_TRY(cudaFuncSetAttribute(solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        if (C == 4) k_sm_solve<4><<<dim3(groups, sm.nsub), kSolve, smem, st>>>(A);
+        else k_sm_solve<2><<<dim3(groups, sm.nsub), kSolve, smem, st>>>(A);
+        launches += 2;
         MTGPU_TRY(cudaGetLastError());
-        int active = 1;
-        while (active > 0 && sm.iterations < kMaxIter) {
-            for (int it = 0; it < kCheckEvery; it++) {
-                // the count of running problems comes from the last scalars pass
-                if (it == kCheckEvery - 1)
-                    MTGPU_TRY(cudaMemsetAsync(sm.d_active, 0, sizeof(int), st));
-                k_sm_spmv<<<grid, kBlk, 0, st>>>(sm.npad, sm.nsub, sm.d_blk_sub, sm.d_mptr,
-                                                 sm.d_mcol, sm.d_mval, sm.d_p, sm.d_q, sm.d_scal,
-                                                 sm.d_done, nprob);
-                k_sm_update<<<grid, kBlk, 0, st>>>(sm.npad, sm.nsub, sm.d_blk_sub, sm.d_mdiag,
-                                                   sm.d_x, sm.d_r, sm.d_z, sm.d_p, sm.d_q,
-                                                   sm.d_scal, sm.d_done, nprob);
-                k_sm_scalars<<<gp, kThreads, 0, st>>>(nprob, sm.d_scal, sm.d_done, sm.d_active);
-                k_sm_direction<<<grid, kBlk, 0, st>>>(sm.npad, sm.nsub, sm.d_blk_sub, sm.d_z,
-                                                      sm.d_p, sm.d_scal, sm.d_done, nprob);
-                launches += 4;
-            }
-            sm.iterations += kCheckEvery;
-            MTGPU_TRY(cudaGetLastError());
-            MTGPU_TRY(cudaMemcpyAsync(&active, sm.d_active, sizeof(int), cudaMemcpyDeviceToHost,
-                                      st));
-            MTGPU_TRY(cudaStreamSynchronize(st));
-        }
-        if (active > 0) {
+        int out[2] = {0, 0};
+        MTGPU_TRY(cudaMemcpyAsync(out, sm.d_out, sizeof(out), cudaMemcpyDeviceToHost, st));
+        MTGPU_TRY(cudaStreamSynchronize(st));
+        sm.iterations = out[1];
+        if (out[0] > 0) {
             set_last_message("receiver smoothing: the projection solve did not converge");
             note_launches(launches);
             return MTGPU_MAXITER;
