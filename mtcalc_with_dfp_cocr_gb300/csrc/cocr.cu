@@ -19,7 +19,7 @@
 //   k_it_spmv   z = A s, MRS smoothing of s_m, |s_m|, (z,s)
 //               -> stop test, beta
 // Reductions are two-level (fixed per-block partials, then the last block
-// sums them in block order), so results do not change run to run.
+// sums them in a fixed order), so results do not change run to run.
 #include "mtgpu_internal.cuh"
 
 namespace mtgpu {
@@ -37,68 +37,92 @@ struct Ctl {
     double residual;     // ||s_m||
     double residual_rel;
     double2 alpha, beta, zs;
+    double2 *x;          // the solution being updated (the graph does not depend on it)
     double sums[4];      // scratch results of one-off reductions
     unsigned int ticket[4];
 };
 
 namespace {
 
-constexpr int kRedThreads = 256;
+constexpr int kRedThreads = 256;   // most threads of a reducing block
 
 // ---------------------------------------------------------- reductions
+// Sums of N <= 4 FP64 values over the block, totals in threads t < N: lanes
+// exchange halves until each holds one value (6 adds a warp for 3 or 4 values
+// instead of 15 or 20; GB300 issues an FP64 add of a warp once in 16 cycles),
+// then thread t adds the warps' sums.
 template <int N>
-__device__ inline void block_sum(double (&v)[N], double *smem /* N * 32 */)
+__device__ inline double block_sum(const double (&v)[N], double (*smem)[4] /* [32] */)
 {
+    constexpr int P = N <= 1 ? 1 : (N <= 2 ? 2 : 4);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double u[P];
 #pragma unroll
-    for (int k = 0; k < N; k++)
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0)
+    for (int k = 0; k < P; k++) u[k] = k < N ? v[k] : 0.0;
+    int first = 0, o = 16;
 #pragma unroll
-        for (int k = 0; k < N; k++) smem[k * 32 + warp] = v[k];
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
+    for (int h = P / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+        first += up ? h : 0;
 #pragma unroll
-        for (int k = 0; k < N; k++) {
-            v[k] = lane < nw ? smem[k * 32 + lane] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+        for (int i = 0; i < h; i++) {
+            const double mine = up ? u[i + h] : u[i], give = up ? u[i] : u[i + h];
+            u[i] = mine + __shfl_xor_sync(0xffffffffu, give, o);
         }
     }
+    const int rest = 2 * o;
+#pragma unroll
+    for (; o >= 1; o >>= 1) u[0] += __shfl_xor_sync(0xffffffffu, u[0], o);
+    if ((lane & (rest - 1)) == 0) smem[warp][first] = u[0];
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x < N)
+        for (int q = 0; q < nw; q++) s += smem[q][threadIdx.x];
+    return s;
 }
 
 // Publish this block's partial sums; returns true in the one block that
-// arrives last, which then holds the grid totals in v (thread 0).
+// arrives last, which then holds the grid totals in v (thread 0).  Each of
+// its threads adds whole partials, 12 loads in flight.
 template <int N>
 __device__ bool grid_sum(double (&v)[N], double *partials, unsigned int *ticket)
 {
-    __shared__ double smem[N * 32];
+    __shared__ double smem[2][32][4];
+    __shared__ double tot[4];
     __shared__ bool last;
-    block_sum<N>(v, smem);
+    const double s = block_sum<N>(v, smem[0]);
+    if (threadIdx.x < N) __stcg(partials + (size_t)blockIdx.x * 4 + threadIdx.x, s);
+    __syncthreads();
     if (threadIdx.x == 0) {
-#pragma unroll
-        for (int k = 0; k < N; k++) partials[(size_t)k * gridDim.x + blockIdx.x] = v[k];
-        __threadfence();
-        const unsigned int t = atomicAdd(ticket, 1u);
-        last = (t == gridDim.x - 1);
+        last = count_arrival(ticket) == gridDim.x - 1;
+        if (last) *ticket = 0u;
     }
     __syncthreads();
     if (!last) return false;
-    __threadfence();
-    double acc[N];
+    constexpr int U = 12;
+    double acc[N] = {};
+    for (int b0 = 0; b0 < (int)gridDim.x; b0 += U * blockDim.x) {
+        double2 l[U], h[U];
 #pragma unroll
-    for (int k = 0; k < N; k++) {
-        acc[k] = 0.0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-            acc[k] += __ldcg(&partials[(size_t)k * gridDim.x + b]);
-    }
-    block_sum<N>(acc, smem);
-    if (threadIdx.x == 0) {
+        for (int u = 0; u < U; u++) {
+            const int b = b0 + u * blockDim.x + threadIdx.x;
+            const double2 *q = reinterpret_cast<const double2 *>(partials) + 2 * (size_t)b;
+            const bool in = b < (int)gridDim.x;
+            l[u] = in ? __ldcg(q) : make_double2(0.0, 0.0);
+            if (N > 2) h[u] = in ? __ldcg(q + 1) : make_double2(0.0, 0.0);
+        }
 #pragma unroll
-        for (int k = 0; k < N; k++) v[k] = acc[k];
-        *ticket = 0u;
+        for (int u = 0; u < U; u++) {
+            acc[0] += l[u].x;
+            if (N > 1) acc[N > 1 ? 1 : 0] += l[u].y;
+            if (N > 2) acc[N > 2 ? 2 : 0] += h[u].x;
+        }
     }
+    const double r = block_sum<N>(acc, smem[1]);
+    if (threadIdx.x < N) tot[threadIdx.x] = r;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] = tot[k];
     return true;
 }
 
@@ -166,44 +190,90 @@ k_norm2(int nb, const double2 *__restrict__ r, const double2 *__restrict__ b, Ct
 }
 
 // ------------------------------------------------------- the iteration
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
 k_it_node(int m, const int *__restrict__ gp, const int *__restrict__ gj,
           const double *__restrict__ gv, const double2 *__restrict__ ds,
           const double2 *__restrict__ z, const double2 *__restrict__ a,
           double2 *__restrict__ h, const Ctl *ctl)
 {
+    pdl_wait();
     if (!running(ctl)) return;
     const double2 beta = ctl->beta;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < m; v += gridDim.x * blockDim.x) {
+        // up to six entries (all of a conforming mesh) with their loads in
+        // flight together; one at a time each waits for two
+        const int j0 = gp[v], n = gp[v + 1] - j0;
+        const double2 dsv = ds[v];
+        int e[6];
+        double g[6];
+        double2 zv[6], av[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+            e[q] = q < n ? gj[j0 + q] : 0;
+            g[q] = q < n ? gv[j0 + q] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+            if (q < n) {
+                zv[q] = z[e[q]];
+                av[q] = a[e[q]];
+            }
         double hr = 0.0, hi = 0.0;
-        for (int j = gp[v]; j < gp[v + 1]; j++) {
-            const int e = gj[j];
-            const double2 an = cadd(z[e], cmul(beta, a[e]));
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+            if (q < n) {
+                const double2 an = cadd(zv[q], cmul(beta, av[q]));
+                hr += g[q] * an.x;
+                hi += g[q] * an.y;
+            }
+        for (int j = j0 + 6; j < j0 + n; j++) {          // T-matrix rows only
+            const int k = gj[j];
+            const double2 an = cadd(z[k], cmul(beta, a[k]));
             hr += gv[j] * an.x;
             hi += gv[j] * an.y;
         }
-        h[v] = cmul(make_double2(hr, hi), ds[v]);
+        h[v] = cmul(make_double2(hr, hi), dsv);
     }
 }
 
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, 3)
 k_it_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj,
-          const double *__restrict__ tv, const double2 *__restrict__ da,
+          const double *__restrict__ tv, const int2 *__restrict__ tn, const double2 *__restrict__ da,
           const double2 *__restrict__ h, const double2 *__restrict__ s,
           const double2 *__restrict__ z, double2 *__restrict__ p, double2 *__restrict__ a,
           double2 *__restrict__ w, Ctl *ctl, double *partials)
 {
+    pdl_wait();
     if (!running(ctl)) return;
+    const double2 zs = ctl->zs;
     const double2 beta = ctl->beta;
     double v[2] = {0.0, 0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double2 pn = cadd(s[i], cmul(beta, p[i]));
-        const double2 an = cadd(z[i], cmul(beta, a[i]));
-        double2 wn = cmul(an, da[i]);
-        for (int j = tp[i]; j < tp[i + 1]; j++) {
-            const double2 hv = h[tj[j]];
-            wn.x += tv[j] * hv.x;
-            wn.y += tv[j] * hv.y;
+        // G^T row of a conforming mesh: its two nodes' rows (one dependent
+        // load), -1/2 and +1/2; else the CSR of T-matrix meshes
+        const int2 row = tn ? tn[i] : make_int2(-1, -1);
+        const double2 sv = s[i], po = p[i], zv = z[i], ao = a[i], dav = da[i];
+        double2 h0 = make_double2(0.0, 0.0), h1 = h0;
+        if (row.x >= 0) h0 = h[row.x];
+        if (row.y >= 0) h1 = h[row.y];
+        const double2 pn = cadd(sv, cmul(beta, po));
+        const double2 an = cadd(zv, cmul(beta, ao));
+        double2 wn = cmul(an, dav);
+        if (tn) {
+            if (row.x >= 0) {
+                wn.x += -0.5 * h0.x;
+                wn.y += -0.5 * h0.y;
+            }
+            if (row.y >= 0) {
+                wn.x += 0.5 * h1.x;
+                wn.y += 0.5 * h1.y;
+            }
+        } else {
+            for (int j = tp[i]; j < tp[i + 1]; j++) {
+                const double2 hv = h[tj[j]];
+                wn.x += tv[j] * hv.x;
+                wn.y += tv[j] * hv.y;
+            }
         }
         p[i] = pn;
         a[i] = an;
@@ -216,18 +286,19 @@ k_it_edge(int n, const int *__restrict__ tp, const int *__restrict__ tj,
         if (fabs(aw.x) < 1e-40 && fabs(aw.y) < 1e-40) {
             ctl->status = MTGPU_DIV_BY_ZERO;
         } else {
-            ctl->alpha = cdiv(ctl->zs, aw);
+            ctl->alpha = cquot(zs, aw);
         }
     }
 }
 
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, 3)
 k_it_update(int n, const double2 *__restrict__ p, const double2 *__restrict__ a,
             const double2 *__restrict__ w, const double2 *__restrict__ sm,
-            double2 *__restrict__ x, double2 *__restrict__ r, double2 *__restrict__ s, Ctl *ctl,
-            double *partials)
+            double2 *__restrict__ r, double2 *__restrict__ s, Ctl *ctl, double *partials)
 {
+    pdl_wait();
     if (!running(ctl)) return;
+    double2 *const x = ctl->x;
     const double2 al = ctl->alpha;
     double v[2] = {0.0, 0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -254,7 +325,7 @@ k_it_update(int n, const double2 *__restrict__ p, const double2 *__restrict__ a,
     }
 }
 
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, 3)
 k_it_spmv(int nb, const int *__restrict__ wc, const int *__restrict__ wr,
           const long long *__restrict__ pc, const long long *__restrict__ pr,
           const int *__restrict__ col_c, const double2 *__restrict__ val_c,
@@ -262,7 +333,11 @@ k_it_spmv(int nb, const int *__restrict__ wc, const int *__restrict__ wr,
           const double2 *__restrict__ s, const double2 *__restrict__ r,
           double2 *__restrict__ z, double2 *__restrict__ sm, Ctl *ctl, double *partials)
 {
+    pdl_wait();
     if (!running(ctl)) return;
+    const double2 zs = ctl->zs;
+    const double residual = ctl->residual, r_old = ctl->r_old, eps = ctl->eps;
+    const int iter = ctl->iter, maxiter = ctl->maxiter;
     const int mode = ctl->mrs_mode;
     const double wm = ctl->mrs_w;
     double v[3] = {0.0, 0.0, 0.0};
@@ -306,16 +381,20 @@ k_it_spmv(int nb, const int *__restrict__ wc, const int *__restrict__ wr,
         }
     }
     if (grid_sum<3>(v, partials, &ctl->ticket[3]) && threadIdx.x == 0) {
-        if (mode != 0) ctl->residual = sqrt(v[2]);
-        ctl->residual_rel = ctl->residual / ctl->r_old;
+        // (independent FP64 chains side by side)
         const double2 zs_new = make_double2(v[0], v[1]);
-        ctl->beta = cdiv(zs_new, ctl->zs);
+        const double2 beta = cquot(zs_new, zs);
+        const double res = mode != 0 ? sqrt(v[2]) : residual;
+        const double rel = res / r_old;
+        ctl->residual = res;
+        ctl->residual_rel = rel;
+        ctl->beta = beta;
         ctl->zs = zs_new;
-        if (ctl->residual_rel < ctl->eps) {
+        if (rel < eps) {
             ctl->status = MTGPU_OK;
         } else {
-            ctl->iter += 1;
-            if (ctl->iter > ctl->maxiter) ctl->status = MTGPU_MAXITER;
+            ctl->iter = iter + 1;
+            if (iter + 1 > maxiter) ctl->status = MTGPU_MAXITER;
         }
     }
 }
@@ -342,17 +421,20 @@ int cocr_alloc(CocrSolver &S)
     int dev = 0, nsm = 0;
     MTGPU_TRY(cudaGetDevice(&dev));
     MTGPU_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    // as many blocks as are resident at once (the loops are grid-stride), so
-    // no block waits for a second wave
+    // Blocks of 64 threads where all rows are resident at once, so that the
+    // FP64 pipes get even shares (45,000 rows: 10 warps on the busiest SM
+    // against 16 in blocks of 256, 9.3 on average); else blocks of 256, as many
+    // as are resident (the loops are grid-stride)
+    S.threads = nb <= nsm * 1024 ? 64 : kRedThreads;
     int occ = 64;
     const void *fs[] = {(const void *)k_it_edge, (const void *)k_it_update, (const void *)k_it_spmv,
                         (const void *)k_init_norms};
     for (const void *f : fs) {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kRedThreads, 0) == cudaSuccess && b > 0)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, S.threads, 0) == cudaSuccess && b > 0)
             occ = std::min(occ, b);
     }
-    S.grid = std::max(1, std::min(ceil_div(nb, kRedThreads), occ * nsm));
+    S.grid = std::max(1, std::min(ceil_div(nb, S.threads), occ * nsm));
     int rc;
     if ((rc = dev_alloc(&S.r, nb)) || (rc = dev_alloc(&S.p, nb)) || (rc = dev_alloc(&S.s, nb)) ||
         (rc = dev_alloc(&S.z, nb)) || (rc = dev_alloc(&S.a, nb)) || (rc = dev_alloc(&S.w, nb)) ||
@@ -364,37 +446,34 @@ int cocr_alloc(CocrSolver &S)
     return MTGPU_OK;
 }
 
-static void launch_iteration(CocrSolver &S, double2 *x)
+static void launch_iteration(CocrSolver &S)
 {
     const Folded &P = S.P;
     const SellMatrix &A = S.A;
-    const int nb = S.nb, g = S.grid;
+    const int nb = S.nb, g = S.grid, th = S.threads;
     if (P.m > 0)
-        k_it_node<<<std::max(1, std::min(ceil_div(P.m, kThreads), g)), kThreads, 0, S.st>>>(
-            P.m, P.d_gp, P.d_gj, P.d_gv, P.d_ds, S.z, S.a, P.d_h, S.ctl);
-    k_it_edge<<<g, kRedThreads, 0, S.st>>>(nb, P.d_tp, P.d_tj, P.d_tv, P.d_da, P.d_h, S.s, S.z,
-                                           S.p, S.a, S.w, S.ctl, S.partials);
-    k_it_update<<<g, kRedThreads, 0, S.st>>>(nb, S.p, S.a, S.w, S.sm, x, S.r, S.s, S.ctl,
-                                             S.partials);
-    k_it_spmv<<<g, kRedThreads, 0, S.st>>>(nb, A.d_wc, A.d_wr, A.d_pc, A.d_pr, A.d_col_c,
-                                           A.d_val_c, A.d_col_r, A.d_val_r, S.s, S.r, S.z, S.sm,
-                                           S.ctl, S.partials);
+        pdl(k_it_node, std::max(1, std::min(ceil_div(P.m, th), g)), th, 0, S.st, P.m, P.d_gp, P.d_gj,
+            P.d_gv, P.d_ds, S.z, S.a, P.d_h, S.ctl);
+    pdl(k_it_edge, g, th, 0, S.st, nb, P.d_tp, P.d_tj, P.d_tv, P.d_tn, P.d_da, P.d_h, S.s, S.z, S.p, S.a, S.w,
+        S.ctl, S.partials);
+    pdl(k_it_update, g, th, 0, S.st, nb, S.p, S.a, S.w, S.sm, S.r, S.s, S.ctl, S.partials);
+    pdl(k_it_spmv, g, th, 0, S.st, nb, A.d_wc, A.d_wr, A.d_pc, A.d_pr, A.d_col_c, A.d_val_c, A.d_col_r,
+        A.d_val_r, S.s, S.r, S.z, S.sm, S.ctl, S.partials);
 }
 
 static int kernels_per_iteration(const CocrSolver &S) { return S.P.m > 0 ? 4 : 3; }
 
-static int build_graph(CocrSolver &S, double2 *x, int iters)
+static int build_graph(CocrSolver &S, int iters)
 {
     if (S.graph) cudaGraphExecDestroy(S.graph);
     S.graph = nullptr;
     cudaGraph_t g;
     MTGPU_TRY(cudaStreamBeginCapture(S.st, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < iters; k++) launch_iteration(S, x);
+    for (int k = 0; k < iters; k++) launch_iteration(S);
     MTGPU_TRY(cudaStreamEndCapture(S.st, &g));
     cudaError_t e = cudaGraphInstantiate(&S.graph, g, 0);
     cudaGraphDestroy(g);
     MTGPU_TRY(e);
-    S.graph_x = x;
     S.graph_iters = iters;
     return MTGPU_OK;
 }
@@ -410,7 +489,7 @@ static int sync_ctl(CocrSolver &S)
 static int true_residual(CocrSolver &S, const double2 *b, const double2 *x, double *out)
 {
     sell_residual(S.A, b, x, S.w, S.st);
-    k_norm2<<<S.grid, kRedThreads, 0, S.st>>>(S.nb, S.w, b, S.ctl, S.partials);
+    k_norm2<<<S.grid, S.threads, 0, S.st>>>(S.nb, S.w, b, S.ctl, S.partials);
     note_launches(2);
     MTGPU_TRY(cudaGetLastError());
     int rc = sync_ctl(S);
@@ -429,23 +508,24 @@ int cocr_solve(CocrSolver &S, const double2 *b, double2 *x, double eps, int maxi
     init.status = kRunning;
     init.maxiter = maxiter;
     init.eps = eps;
+    init.x = x;
     MTGPU_TRY(cudaMemcpyAsync(S.ctl, &init, sizeof(Ctl), cudaMemcpyHostToDevice, S.st));
     // stages 1-4 of PCOCR_RCI::Run
     sell_residual(S.A, b, x, S.r, S.st);                                    // r = b - A x
-    k_init_norms<<<S.grid, kRedThreads, 0, S.st>>>(nb, b, S.r, S.sm, S.ctl, S.partials);
+    k_init_norms<<<S.grid, S.threads, 0, S.st>>>(nb, b, S.r, S.sm, S.ctl, S.partials);
     folded_apply(S.P, S.r, S.s, S.st);                                      // s = M^-1 r
     MTGPU_TRY(cudaMemsetAsync(S.p, 0, sizeof(double2) * nb, S.st));
     MTGPU_TRY(cudaMemsetAsync(S.a, 0, sizeof(double2) * nb, S.st));
     MTGPU_TRY(cudaMemsetAsync(S.w, 0, sizeof(double2) * nb, S.st));
     sell_spmv(S.A, S.s, S.z, S.st);                                         // z = A s
-    k_init_zs<<<S.grid, kRedThreads, 0, S.st>>>(nb, S.z, S.s, S.ctl, S.partials);
+    k_init_zs<<<S.grid, S.threads, 0, S.st>>>(nb, S.z, S.s, S.ctl, S.partials);
     note_launches(S.P.m > 0 ? 6 : 5);
     MTGPU_TRY(cudaGetLastError());
     int rc = sync_ctl(S);
     if (rc) return rc;
 
-    if (S.graph == nullptr || S.graph_x != (const void *)x || S.graph_iters != iters_per_launch)
-        if ((rc = build_graph(S, x, iters_per_launch))) return rc;
+    if (S.graph == nullptr || S.graph_iters != iters_per_launch)
+        if ((rc = build_graph(S, iters_per_launch))) return rc;
 
     const unsigned long long kpi = (unsigned long long)kernels_per_iteration(S);
     double true_rr = -1.0;

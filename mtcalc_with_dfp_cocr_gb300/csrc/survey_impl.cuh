@@ -180,10 +180,7 @@ __device__ bool sys_grid_sum(const tf (&v)[N], float4 *partials, double (*tot)[3
         if (threadIdx.x < W) __stcg(dst + threadIdx.x, s);
         __syncthreads();
         if (threadIdx.x == 0) {
-            // release: the block's stores, which the barrier ordered before
-            // this thread; acquire: those of the blocks counted before
-            unsigned int seen;
-            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(ticket) : "memory");
+            const unsigned int seen = count_arrival(ticket);
             last = seen == n - 1;
             if (last) *ticket = 0u;
         }
@@ -269,20 +266,6 @@ __device__ bool sys_grid_sum64(double (&v)[N], float4 *scratch, unsigned int *ti
     return true;
 }
 
-// Programmatic dependent launch: the iteration's kernels are launched with
-// the programmatic-serialization attribute, so the next grid is scheduled
-// while the one before it drains; each of them waits here, before its first
-// access to memory, until the grid before it has completed and its writes
-// are visible (a no-op for a kernel launched without the attribute).  Once
-// its own blocks run, the grid lets the next one be scheduled behind it:
-// launch latency then overlaps this grid's work (no grid has more blocks
-// than fit at once, so waiting blocks never keep running ones out).
-__device__ __forceinline__ void pdl_wait()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc)
 {
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
@@ -320,22 +303,6 @@ __device__ __forceinline__ void cp_async8(void *smem_dst, const void *gsrc)
 // still in L2 (a 58 MB vector of two systems against ~126 MB of L2); only
 // the order of the partial sums changes, and it is fixed.
 __device__ __forceinline__ int sweep(int i, int n, int rev) { return rev ? n - 1 - i : i; }
-
-template <typename... K, typename... A>
-void pdl(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-}
 
 struct Mat {
     const int *wc, *wr;
@@ -501,15 +468,6 @@ k_init(int nb, const float4 *__restrict__ r, float4 *__restrict__ sm, SysState *
             }
         }
     }
-}
-
-// a / b of FP64 values that come from FP32 sums: |b|^2 is far inside FP64's
-// range, so the quotient is formed from it directly, one divide deep instead
-// of the two of a division scaled against overflow
-__device__ __forceinline__ double2 cquot(double2 a, double2 b)
-{
-    const double d = b.x * b.x + b.y * b.y;
-    return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
 }
 
 // (a, w) -> alpha, by the block that finishes last.  Here and in the other
