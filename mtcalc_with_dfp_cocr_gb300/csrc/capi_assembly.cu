@@ -309,11 +309,12 @@ int mtgpu_survey_create_multi(int nmesh, mtgpu_assembly *const *a, const int *S,
 {
     MTGPU_CHECK_ARG(a && S && nu && out && nmesh >= 1, "null argument");
     *out = nullptr;
-    int total = 0;
+    int total = 0, batches = 0;
     for (int m = 0; m < nmesh; m++) {
         MTGPU_CHECK_ARG(a[m] != nullptr, "null assembly");
         MTGPU_CHECK_ARG(S[m] >= 1, "every mesh needs at least one system");
         total += S[m];
+        batches += ceil_div(S[m], 32);
     }
     MTGPU_CHECK_ARG(total <= MTGPU_SURVEY_MAX_SYSTEMS, "a survey holds at most "
                     "MTGPU_SURVEY_MAX_SYSTEMS (256) systems");
@@ -343,6 +344,7 @@ int mtgpu_survey_create_multi(int nmesh, mtgpu_assembly *const *a, const int *S,
                 return MTGPU_ERR_CUDA;
             }
             s->groups.push_back(std::make_unique<mtgpu::Survey>());
+            s->groups.back()->alone = batches == 1;
             s->g_st.push_back(st);
             s->g_first.push_back(k0 + f);
             std::vector<double> om(n);

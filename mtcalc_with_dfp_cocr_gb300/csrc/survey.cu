@@ -1301,10 +1301,12 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
             MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
             float ms = 0.f;
             if ((rc = survey_iter_timed(V, 1, &ms))) return rc;   // warm-up
-            if ((rc = survey_iter_timed(V, 3, &ms))) return rc;
-            V.tune_ms[c] = ms / 3.f;
-            if (ms < best) {
-                best = ms;
+            // (a whole group where its launch serves all of it)
+            const int reps = small_used(V) ? V.group : 3;
+            if ((rc = survey_iter_timed(V, reps, &ms))) return rc;
+            V.tune_ms[c] = ms / (float)reps;
+            if (V.tune_ms[c] < best) {
+                best = V.tune_ms[c];
                 best_ch = cand[c];
             }
         }
@@ -1401,8 +1403,8 @@ int survey_iter_timed(Survey &V, int reps, float *ms)
     MTGPU_TRY(cudaEventCreate(&e0));
     MTGPU_TRY(cudaEventCreate(&e1));
     MTGPU_TRY(cudaEventRecord(e0, V.st));
-    for (int q = 0; q < reps; q++) MTGPU_SP_DISPATCH(V.SP, iteration(V, q, INT_MAX));
-    note_launches((unsigned long long)reps * iteration_launches(V));
+    for (int q = 0; q < reps; q++) MTGPU_SP_DISPATCH(V.SP, iteration(V, q, small_used(V) ? reps : INT_MAX));
+    note_launches((unsigned long long)reps * iteration_launches(V) + (small_used(V) ? 2u * ceil_div(reps, V.group) : 0u));
     MTGPU_TRY(cudaEventRecord(e1, V.st));
     MTGPU_TRY(cudaEventSynchronize(e1));
     MTGPU_TRY(cudaEventElapsedTime(ms, e0, e1));
@@ -1507,6 +1509,8 @@ int survey_begin(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, do
         V.hsys[k] = s;
     }
     int rc;
+    // (the ticket slots: a launch that gave up leaves its counters behind)
+    MTGPU_TRY(cudaMemsetAsync(V.partials, 0, sizeof(float4) * kTicketSlots, V.st));
     if ((rc = upload_sys(V))) return rc;
     k_to_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, b_sys_major, V.b64);
     k_to_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, x_sys_major, V.xacc);
@@ -1563,7 +1567,7 @@ int survey_launch(Survey &V, SurveyRun &R)
         return MTGPU_ERR_CUDA;
     }
     const unsigned long long kpi = iteration_launches(V);
-    note_launches(kpi * (unsigned long long)R.ipl + ceil_div(R.ipl, V.group));
+    note_launches(kpi * (unsigned long long)R.ipl + (small_used(V) ? 2u : 1u) * ceil_div(R.ipl, V.group));
     R.guard += R.ipl;
     // the state arrives with the launch's end (read in survey_collect)
     MTGPU_TRY(cudaMemcpyAsync(V.hsys, V.sys, sizeof(SysState) * 32, cudaMemcpyDeviceToHost, V.st));
@@ -1586,6 +1590,10 @@ int survey_collect(Survey &V, SurveyRun &R)
         bool changed = false;
         for (int k = 0; k < V.S; k++) {
             SysState &q = V.hsys[k];
+            if (q.status == MTGPU_ERR_TIMEOUT) {
+                set_last_message("survey solve: a grid barrier did not complete");
+                return MTGPU_ERR_TIMEOUT;
+            }
             if (q.status != kRun) continue;
             if (q.residual_rel < 0.5 * R.best[k]) {
                 R.best[k] = q.residual_rel;

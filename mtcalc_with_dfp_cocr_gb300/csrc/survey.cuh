@@ -86,6 +86,9 @@ struct Survey {
     float tune_ms[kSpmvVariants] = {};   // SpMV times of the variants 0, 1, 2, 4, 8, 18, 20, 32, 33, 34, 35
     bool autotuned = false;              // the variant was chosen by this set-up's timing
     MatFree mf;
+    // k_small's launch grid (0: separate kernels), threads with rows, rows x systems per thread
+    int g_small = 0, small_threads = 0, small_items = 0;
+    bool alone = true;             // no other batch of the survey runs beside this one
     int g_mff = 0, g_mfe = 0;                    // matrix-free launch grids (faces, edges)
     int g_mft = 0;                               // tiled matrix-free launch grid (variant 34)
     int g_mfg = 0, g_mfe3 = 0;                   // face-mass and edge grids (variant 35)
@@ -194,10 +197,13 @@ int survey_finish(Survey &V, SurveyRun &R, mtgpu_survey_stats *stats, int stat_o
 int survey_spmv_timed(Survey &V, int reps, float *ms);
 int survey_spmv(Survey &V, const double2 *x_sys_major, double2 *y_sys_major);
 int survey_iter_timed(Survey &V, int reps, float *ms);
-// kernels one iteration launches
+// whether groups of iterations run in k_small (not where the fused
+// preconditioner was asked for)
+inline bool small_used(const Survey &V) { return V.g_small > 0 && !V.prec_tile; }
+// kernels one iteration launches, those of its group's end aside
 inline int iteration_launches(const Survey &V)
 {
-    return (V.prec_tile ? 3 : (V.G.m > 0 ? 4 : 3)) + spmv_extra_launches(V.ch);
+    return small_used(V) ? 0 : (V.prec_tile ? 3 : (V.G.m > 0 ? 4 : 3)) + spmv_extra_launches(V.ch);
 }
 int survey_set_variant(Survey &V, int variant);
 // builds what `variant` needs beyond the set-up (on its first request);

@@ -988,8 +988,7 @@ __device__ __forceinline__ int mf_edge_in(const MF &M, int d, int i, int j, int 
 
 // x of the +d edge of node (i, j, kk) for system k, 0 on Dirichlet edges
 template <int SP>
-__device__ __forceinline__ cdf mf_x(const MF &M, const float4 *__restrict__ x, int d, int i, int j,
-                                    int kk, int k)
+__device__ __forceinline__ cdf mf_x(const MF &M, const float4 *x, int d, int i, int j, int kk, int k)
 {
     if (mf_dirichlet(M, d, i, j, kk)) return czero();
     return cdf_of(__ldg(x + mf_edge_in(M, d, i, j, kk) * SP + k));
@@ -1094,48 +1093,58 @@ __device__ __forceinline__ df scale(df a, float s) { return df{a.h * s, a.l * s}
 struct Pos {
     int x, y, z;
 };
-// Index context of a non-Dirichlet edge of direction D at lattice position
-// p (p along D a cell index, along T1 = D+1 and T2 = D+2 (mod 3) node
-// indices): the cell, T1-normal face and T2-normal face at p, the edge, and
-// whether the node lines one below / above along T1 (T2) lie on the
-// surface.  Every neighbour the row reads is one of these plus strides.
-template <int D>
+__device__ __forceinline__ int coord(int a, Pos p) { return a == 0 ? p.x : (a == 1 ? p.y : p.z); }
+__device__ __forceinline__ int extent(int a, const MF &M) { return a == 0 ? M.nx : (a == 1 ? M.ny : M.nz); }
+// Index context of a non-Dirichlet edge of direction d at lattice position
+// p (p along d a cell index, along T1 = d+1 and T2 = d+2 (mod 3) node
+// indices): the cell, T1-normal face and T2-normal face at p, the edge, their
+// strides along the axes, and whether the node lines one below / above along
+// T1 (T2) lie on the surface.  Every neighbour the row reads is one of these
+// plus strides.
 struct MfRow {
-    static constexpr int T1 = (D + 1) % 3, T2 = (D + 2) % 3;
-    int cell, f1, f2, e;
+    int cell, c1, c2;          // cell, strides along T1, T2
+    int f1, n1, t1;            // T1-normal face, strides along T1, T2
+    int f2, n2, t2;            // T2-normal face, strides along T2, T1
+    int e, e1, e2;             // edge, strides along T1, T2
+    int w1, w2, wm;            // weights of the T1-, T2-normal faces and of the mass
     bool lo1, hi1, lo2, hi2;
 };
-template <int A>
-__device__ __forceinline__ int coord(Pos p) { return A == 0 ? p.x : (A == 1 ? p.y : p.z); }
-template <int A>
-__device__ __forceinline__ int extent(const MF &M) { return A == 0 ? M.nx : (A == 1 ? M.ny : M.nz); }
-template <int D>
-__device__ __forceinline__ MfRow<D> mf_rowctx(const MF &M, Pos p)
+__device__ __forceinline__ MfRow mf_rowctx(const MF &M, int d, Pos p)
 {
-    constexpr int T1 = MfRow<D>::T1, T2 = MfRow<D>::T2;
-    MfRow<D> r;
+    const int T1 = d == 2 ? 0 : d + 1, T2 = d == 0 ? 2 : d - 1;
+    MfRow r;
     r.cell = p.x * M.cs[0] + p.y * M.cs[1] + p.z * M.cs[2];
+    r.c1 = M.cs[T1];
+    r.c2 = M.cs[T2];
     r.f1 = M.fb[T1] + p.x * M.fs[T1][0] + p.y * M.fs[T1][1] + p.z * M.fs[T1][2];
+    r.n1 = M.fs[T1][T1];
+    r.t1 = M.fs[T1][T2];
     r.f2 = M.fb[T2] + p.x * M.fs[T2][0] + p.y * M.fs[T2][1] + p.z * M.fs[T2][2];
-    r.e = mf_edge_in(M, D, p.x, p.y, p.z);
-    const int t1 = coord<T1>(p), t2 = coord<T2>(p);
-    r.lo1 = t1 == 1;
-    r.hi1 = t1 == extent<T1>(M) - 2;
-    r.lo2 = t2 == 1;
-    r.hi2 = t2 == extent<T2>(M) - 2;
+    r.n2 = M.fs[T2][T2];
+    r.t2 = M.fs[T2][T1];
+    r.e = mf_edge_in(M, d, p.x, p.y, p.z);
+    r.e1 = M.es[T1];
+    r.e2 = M.es[T2];
+    const int nc = (int)M.ncell;
+    r.w1 = T1 * nc;
+    r.w2 = T2 * nc;
+    r.wm = (3 + d) * nc;
+    const int q1 = coord(T1, p), q2 = coord(T2, p);
+    r.lo1 = q1 == 1;
+    r.hi1 = q1 == extent(T1, M) - 2;
+    r.lo2 = q2 == 1;
+    r.hi2 = q2 == extent(T2, M) - 2;
     return r;
 }
 // the 3 x 3 parallel edges around the row (grid position (a, b) along
 // (T1, T2), the row at (1, 1)): Dirichlet, and the edge number otherwise
-template <int D>
-__device__ __forceinline__ bool mf_mass_dir(const MfRow<D> &r, int a, int b)
+__device__ __forceinline__ bool mf_mass_dir(const MfRow &r, int a, int b)
 {
     return (a == 0 && r.lo1) || (a == 2 && r.hi1) || (b == 0 && r.lo2) || (b == 2 && r.hi2);
 }
-template <int D>
-__device__ __forceinline__ int mf_mass_edge(const MF &M, const MfRow<D> &r, int a, int b)
+__device__ __forceinline__ int mf_mass_edge(const MfRow &r, int a, int b)
 {
-    return r.e + (a - 1) * M.es[MfRow<D>::T1] + (b - 1) * M.es[MfRow<D>::T2];
+    return r.e + (a - 1) * r.e1 + (b - 1) * r.e2;
 }
 
 // (a0 + b0, a1 + b1) of two double-float pairs, packed
@@ -1147,17 +1156,13 @@ __device__ __forceinline__ cdf pair_add(df a0, df a1, df b0, df b1)
     return t.get();
 }
 
-// weights w of the 4 cells around an edge of direction D, offsets (a - 1,
-// b - 1) along (T1, T2)
-template <int D>
-__device__ __forceinline__ void mf_weights(const MF &M, const MfRow<D> &r, int w, df (&out)[2][2])
+// the weights of table w at the 4 cells around a row, offsets (a - 1, b - 1) along (T1, T2)
+__device__ __forceinline__ void mf_weights(const MF &M, const MfRow &r, int w, df (&out)[2][2])
 {
-    const int base = w * (int)M.ncell + r.cell;
 #pragma unroll
     for (int a = 0; a < 2; a++)
 #pragma unroll
-        for (int b = 0; b < 2; b++)
-            out[a][b] = d2f(__ldg(M.w + base + (a - 1) * M.cs[MfRow<D>::T1] + (b - 1) * M.cs[MfRow<D>::T2]));
+        for (int b = 0; b < 2; b++) out[a][b] = d2f(__ldg(M.w + w + r.cell + (a - 1) * r.c1 + (b - 1) * r.c2));
 }
 
 // The mass part of a row for U systems k0, k0 + 1, ...: the 3 x 3 parallel
@@ -1166,13 +1171,13 @@ __device__ __forceinline__ void mf_weights(const MF &M, const MfRow<D> &r, int w
 // weight times 2 per axis on which A (B) is the edge's own position:
 // coefficients 4 (w00+w01+w10+w11), 2 (pair sums) and 1 (corner cells).
 // Then y = kk + i omega (mass part).  sv: the row's own x.
-template <int SP, int D, int U>
-__device__ __forceinline__ void mf_mass_row(const MF &M, const MfRow<D> &r, int k0, const df (&om)[U],
-                                            const float4 *__restrict__ x, const cdf (&sv)[U],
+template <int SP, int U>
+__device__ __forceinline__ void mf_mass_row(const MF &M, const MfRow &r, int k0, const df (&om)[U],
+                                            const float4 *x, const cdf (&sv)[U],
                                             acc2 (&kk)[U], cdf (&y)[U])
 {
     df wm[2][2];
-    mf_weights<D>(M, r, 3 + D, wm);
+    mf_weights(M, r, r.wm, wm);
     const cdf s = pair_add(wm[0][0], wm[1][0], wm[0][1], wm[1][1]);      // sums over b
     const cdf q = pair_add(wm[0][0], wm[0][1], wm[1][0], wm[1][1]);      // sums over a
     const df s0 = lane0(s), s1 = lane1(s), r0 = lane0(q), r1 = lane1(q);
@@ -1191,7 +1196,7 @@ __device__ __forceinline__ void mf_mass_row(const MF &M, const MfRow<D> &r, int 
                 if (a == 1 && b == 1)
                     xe = sv[u];
                 else if (!mf_mass_dir(r, a, b))
-                    xe = cdf_of(__ldg(x + mf_mass_edge(M, r, a, b) * SP + k0 + u));
+                    xe = cdf_of(__ldg(x + mf_mass_edge(r, a, b) * SP + k0 + u));
                 if (a == 0 && b == 0) mm[u].first(c, xe);
                 else mm[u].mac(c, xe);
             }
@@ -1228,32 +1233,31 @@ __device__ __forceinline__ void mf_face_group(const MF &M, int q, int step, int 
     }
 }
 
-// one non-Dirichlet edge of direction D at lattice position p for U systems:
-// (K + i omega M) s.  D, and with it the two transverse axes T1 = D+1,
-// T2 = D+2 (mod 3), are compile-time constants: the rows run direction by
+// one non-Dirichlet edge of direction d at lattice position p for U systems:
+// (K + i omega M) s.  With d a constant of the call the two transverse axes
+// and the strides are compile-time choices: the rows run direction by
 // direction, so warps are uniform.  The adjacent systems' values are
 // contiguous and share the index arithmetic, the weights and their
 // combinations.
-template <int SP, int D, int U>
-__device__ __forceinline__ void mf_row(const MF &M, Pos p, int k0, const df (&om)[U],
-                                       const float4 *__restrict__ x, const cdf (&sv)[U], cdf (&y)[U])
+template <int SP, int U>
+__device__ __forceinline__ void mf_row(const MF &M, int d, Pos p, int k0, const df (&om)[U],
+                                       const float4 *x, const cdf (&sv)[U], cdf (&y)[U])
 {
-    constexpr int T1 = (D + 1) % 3, T2 = (D + 2) % 3;
-    const MfRow<D> r = mf_rowctx<D>(M, p);
+    const MfRow r = mf_rowctx(M, d, p);
     df w1[2][2], w2[2][2];
-    mf_weights<D>(M, r, T1, w1);
-    mf_weights<D>(M, r, T2, w2);
+    mf_weights(M, r, r.w1, w1);
+    mf_weights(M, r, r.w2, w2);
     // D^T F D: faces of normal T1 through the edge (T2 cells b - 1 = -1: +1,
     // 0: -1), then faces of normal T2 (T1 cells -1: -1, 0: +1); each face's
     // F row over the cells before and after it along the normal
     acc2 kk[U];
     const cdf c1 = pair_add(w1[0][0], w1[0][1], w1[1][0], w1[1][1]);
-    mf_face_group<SP, U, true, true>(M, r.f1 - M.fs[T1][T2], M.fs[T1][T1], k0, w1[0][0], w1[1][0], lane0(c1), kk);
-    mf_face_group<SP, U, false, false>(M, r.f1, M.fs[T1][T1], k0, w1[0][1], w1[1][1], lane1(c1), kk);
+    mf_face_group<SP, U, true, true>(M, r.f1 - r.t1, r.n1, k0, w1[0][0], w1[1][0], lane0(c1), kk);
+    mf_face_group<SP, U, false, false>(M, r.f1, r.n1, k0, w1[0][1], w1[1][1], lane1(c1), kk);
     const cdf c2 = pair_add(w2[0][0], w2[1][0], w2[0][1], w2[1][1]);
-    mf_face_group<SP, U, false, false>(M, r.f2 - M.fs[T2][T1], M.fs[T2][T2], k0, w2[0][0], w2[0][1], lane0(c2), kk);
-    mf_face_group<SP, U, true, false>(M, r.f2, M.fs[T2][T2], k0, w2[1][0], w2[1][1], lane1(c2), kk);
-    mf_mass_row<SP, D, U>(M, r, k0, om, x, sv, kk, y);
+    mf_face_group<SP, U, false, false>(M, r.f2 - r.t2, r.n2, k0, w2[0][0], w2[0][1], lane0(c2), kk);
+    mf_face_group<SP, U, true, false>(M, r.f2, r.n2, k0, w2[1][0], w2[1][1], lane1(c2), kk);
+    mf_mass_row<SP, U>(M, r, k0, om, x, sv, kk, y);
 }
 
 // The matrix-free SpMV with two systems per thread (variant 33, SP >= 2):
@@ -1294,11 +1298,11 @@ k_mf_edges2(int nb, MF M, const float2 *__restrict__ omega, const float4 *__rest
                 y[0] = sv[0];
                 y[1] = sv[1];
             } else if (d == 0) {
-                mf_row<SP, 0, 2>(M, p, k0, om, s, sv, y);
+                mf_row<SP, 2>(M, 0, p, k0, om, s, sv, y);
             } else if (d == 1) {
-                mf_row<SP, 1, 2>(M, p, k0, om, s, sv, y);
+                mf_row<SP, 2>(M, 1, p, k0, om, s, sv, y);
             } else {
-                mf_row<SP, 2, 2>(M, p, k0, om, s, sv, y);
+                mf_row<SP, 2>(M, 2, p, k0, om, s, sv, y);
             }
 #pragma unroll
             for (int u = 0; u < 2; u++)
@@ -1352,11 +1356,11 @@ k_mf_edges(int nb, MF M, const float2 *__restrict__ omega, const float4 *__restr
         if (mf_dirichlet(M, d, p.x, p.y, p.z))
             y[0] = sv[0];
         else if (d == 0)
-            mf_row<SP, 0, 1>(M, p, k, om, s, sv, y);
+            mf_row<SP, 1>(M, 0, p, k, om, s, sv, y);
         else if (d == 1)
-            mf_row<SP, 1, 1>(M, p, k, om, s, sv, y);
+            mf_row<SP, 1>(M, 1, p, k, om, s, sv, y);
         else
-            mf_row<SP, 2, 1>(M, p, k, om, s, sv, y);
+            mf_row<SP, 1>(M, 2, p, k, om, s, sv, y);
         tail.row(i, y[0], sv[0], z);
     }
     tail.finish<SP>(sys, partials, mode);
@@ -1917,6 +1921,12 @@ k_group(long long n, float4 *__restrict__ s, float4 *__restrict__ p, double2 *__
     }
 }
 
+}  // namespace sv
+}  // namespace mtgpu
+#include "survey_small.cuh"
+namespace mtgpu {
+namespace sv {
+
 template <int SP>
 struct Impl {
     static Mat mat(const Survey &V)
@@ -2071,6 +2081,10 @@ struct Impl {
     static void iteration(Survey &V, int t, int n)
     {
         const int j = t % V.group;
+        if (small_used(V)) {
+            if (j == 0) small(V, std::min(V.group, n - t));
+            return;
+        }
         float4 *a = V.a;
         if (V.prec_tile) {
             a = (t & 1) ? V.a : V.a2;
@@ -2084,8 +2098,61 @@ struct Impl {
         if (j == V.group - 1 || t == n - 1)
             // (the iteration's sweep directions, and with them its sums, do not
             // depend on the group's length)
-            pdl(k_group<SP>, V.g_group, kB, 0, V.st, (long long)V.nb * SP, V.s, V.p, V.xacc, V.hist,
-                V.sys, V.dir ^ 1);
+            group(V);
+    }
+    static void group(Survey &V)
+    {
+        pdl(k_group<SP>, V.g_group, kB, 0, V.st, (long long)V.nb * SP, V.s, V.p, V.xacc, V.hist,
+            V.sys, V.dir ^ 1);
+    }
+    // n iterations (a group, or what is left of the sequence) in one launch
+    static void small(Survey &V, int n)
+    {
+        const SmallArgs A{V.nb, V.ds, V.da, V.G.d_tn, V.omega, V.r, V.a, V.w, V.sm,
+                          V.z, V.s, V.sys, V.hist, V.partials};
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = V.g_small;
+        cfg.blockDim = V.small_threads + 32;
+        cfg.dynamicSmemBytes = (size_t)V.small_items * kSmallItemBytes * V.small_threads;
+        cfg.stream = V.st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, k_small<SP>, mfd(V), A, n, V.small_items);
+        group(V);
+    }
+    // the grid of k_small and its rows x systems per thread; grid 0: not used.
+    // Variant 35 on a lattice mesh, one block per SM; the batches of a survey
+    // run side by side, which launches that need every SM would prevent
+    static void small_grid(Survey &V, int nsm)
+    {
+        V.g_small = 0;
+        const long long n = (long long)V.nb * SP;
+        if (V.ch != kMatFree + 3 || !V.mf.on || !V.mf.gface || !V.g_lat || !V.G.d_tn) return;
+        if (n > (long long)nsm * kSmallThreads * kSmallItems) return;
+        if (SP > kSmallSystems || !V.alone) return;
+        if ((size_t)nsm * 8 * SP > 2 * (partial_slots(V.pblocks, SP) - kTicketSlots)) return;
+        // as few rows per thread as fit, the rows even over the SMs
+        const int items = (int)((n + (long long)nsm * kSmallThreads - 1) / ((long long)nsm * kSmallThreads));
+        const int per = (int)((n + (long long)nsm * items - 1) / ((long long)nsm * items));
+        const int nt = std::max(kSmallMin, ceil_div(per, 32) * 32);
+        const int grid = (int)std::min<long long>(nsm, (n + nt - 1) / nt);
+        const int smem = items * kSmallItemBytes * nt;
+        int dev = 0, coop = 0, b = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+            cudaFuncSetAttribute((const void *)k_small<SP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kSmallItems * kSmallItemBytes * kSmallThreads) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void *)k_small<SP>, nt + 32, smem) !=
+                cudaSuccess || b < 1) {
+            cudaGetLastError();
+            return;
+        }
+        V.g_small = grid;
+        V.small_items = items;
+        V.small_threads = nt;
     }
     // one preconditioner step of the iteration (mode 1), unfused or fused
     static void precond_step(Survey &V, bool fused, float4 *ain, float4 *aout)
@@ -2224,6 +2291,7 @@ struct Impl {
             V.mft[0] = tx; V.mft[1] = ty; V.mft[2] = zc; V.mft[3] = grp; V.mft[4] = kz;
             V.g_mft = bxy * zc;
         }
+        small_grid(V, nsm);
         if constexpr (SP == 2) {
             if (V.ch == kRowVariant + 2 || V.ch == kRowVariant + 4) {
                 const void *fr = V.ch == kRowVariant + 2 ? (const void *)k_spmv_r2<2>

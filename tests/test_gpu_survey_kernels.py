@@ -112,3 +112,89 @@ def test_shorter_groups_where_memory_is_short(gpu):
     assert res[1][2] > res[0][2]
     A.close()
     torch.cuda.empty_cache()
+
+
+# cells and systems with 1, 2 and 3 rows x systems a thread in the one-kernel
+# iteration, single blocks, and one beyond its range (218,880 rows x systems)
+SMALL = [((2, 2, 2), 1), ((3, 2, 5), 8), ((4, 9, 3), 3), ((17, 16, 15), 5), ((31, 27, 22), 1),
+         ((24, 24, 25), 2), ((33, 31, 32), 2), ((33, 34, 32), 2)]
+
+
+def _ragged(torch, cells, S, seed):
+    rng = np.random.default_rng(seed)
+    x, y = _lines(rng, cells[0], -300.0), _lines(rng, cells[1], -500.0)
+    z = _lines(rng, cells[2], 0.0)
+    z -= z[max(1, cells[2] - 1)]
+    m = layered_model(x, y, z, [Layer(0.0, 0.01)],
+                      cell_sigma=10.0 ** rng.uniform(-3, 0, int(np.prod(cells))))
+    nus = list(10.0 ** rng.uniform(0, 2, S))
+    b = torch.from_numpy(rng.standard_normal((S, 2 * m.nb))).cuda()
+    return m, nus, b
+
+
+@pytest.mark.parametrize("cells,S", SMALL)
+def test_iterations_in_one_kernel(gpu, cells, S):
+    """Variant 35 of a small problem runs its iterations in one kernel.  After
+    5 iterations the residuals are those of variant 32's separate kernels: a
+    wrong or missing term shows at 1e-3; rounding (2^-46 an operation) stays
+    below 1e-7 unless the sums cancel by 2^20, and below 5 x 64 2^-46 of |b|
+    where nothing but rounding is left of the residual.  Solved to 1e-6 the
+    counts are variant 32's within the 3 that rounding moves them elsewhere, and
+    a second solve is the same to the last bit."""
+    torch = gpu
+    m, nus, b = _ragged(torch, cells, S, 7 * S + sum(cells))
+    A = assembly.Assembly(m)
+    sv = survey.Survey(A, nus)
+    res, its = {}, {}
+    for v in (32, 35):
+        sv.set_spmv_variant(v)
+        _, st = sv.solve(b, torch.zeros_like(b), eps=1e-13, maxiter=5, verify=False)
+        res[v] = np.array(st["residual_rel"])
+        _, st = sv.solve(b, torch.zeros_like(b), eps=1e-6, maxiter=2000, verify=False)
+        its[v] = np.array(st["iterations"])
+    assert np.all(np.abs(res[35] - res[32]) <= 1e-7 * res[32] + 320 * 2.0 ** -46)
+    runs = []
+    for _ in range(2):
+        x = torch.zeros_like(b)
+        code, st = sv.solve(b, x, eps=1e-6, maxiter=2000, verify=False)
+        assert code == 0 and np.all(np.abs(np.array(st["iterations"]) - its[32]) <= 3)
+        runs.append((st["iterations"], st["residual_rel"], x))
+    assert runs[0][:2] == runs[1][:2] and torch.equal(runs[0][2], runs[1][2])
+    sv.close()
+    A.close()
+
+
+def test_one_kernel_iterations_from_two_threads(gpu):
+    """Two surveys solved at the same time from two threads on their own
+    streams: each launch of the one-kernel iteration needs the whole chip, and
+    both end with what they give alone."""
+    import threading
+    torch = gpu
+    probs = []
+    for cells, S in (((24, 24, 25), 2), ((31, 27, 22), 1)):
+        m, nus, b = _ragged(torch, cells, S, 5)
+        A = assembly.Assembly(m)
+        sv = survey.Survey(A, nus)
+        sv.set_spmv_variant(35)
+        x = torch.zeros_like(b)
+        _, st = sv.solve(b, x, eps=1e-6, maxiter=2000, verify=False)
+        probs.append((A, sv, b, x, st["iterations"]))
+    ok = [0, 0]
+
+    def work(i):
+        A, sv, b, ref, its = probs[i]
+        for _ in range(4):
+            x = torch.zeros_like(b)
+            torch.cuda.synchronize()
+            code, st = sv.solve(b, x, eps=1e-6, maxiter=2000, verify=False)
+            ok[i] += code == 0 and st["iterations"] == its and bool(torch.equal(x, ref))
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert ok == [4, 4]
+    for A, sv, *_ in probs:
+        sv.close()
+        A.close()
