@@ -77,7 +77,8 @@ typedef struct {
      * 1: after that, keep iterating until the true residual ||b-Ax||/||b||
      *    is below eps as well (checked on the GPU in FP64). */
     int stop_on_true_residual;
-    /* iterations per CUDA-graph launch between host status checks (0: 16) */
+    /* iterations per launch between host status checks (0: 16, or 64 where one
+     * kernel runs them: FP64, up to 1,440 edges per SM) */
     int iterations_per_launch;
     /* 1: run the same algorithm in double-float arithmetic on the FP32 pipes
      * (the batched survey solver with one system; a system it cannot

@@ -7,7 +7,8 @@
 // (MRS.cpp:85-153, rci.cpp:66-75), REQ_DIV_BY_ZERO when (a,w) vanishes.
 //
 // One iteration is four kernels, captured into a CUDA graph several
-// iterations at a time; every decision (alpha, beta, the MRS weight, the
+// iterations at a time (up to 219,000 rows on 152 SMs: phases of one
+// cooperative kernel, cocr_small.cuh); every decision (alpha, beta, the MRS weight, the
 // stop test, the iteration limit) is taken on the device by the last block
 // of the kernel that finishes the reduction, so the host only looks at the
 // status word between graph launches.
@@ -40,11 +41,12 @@ struct Ctl {
     double2 *x;          // the solution being updated (the graph does not depend on it)
     double sums[4];      // scratch results of one-off reductions
     unsigned int ticket[4];
+    unsigned int bar, left;   // k_small64: barrier arrivals, blocks that left
 };
 
 namespace {
 
-constexpr int kRedThreads = 256;   // most threads of a reducing block
+constexpr int kRedThreads = 256;   // threads of a reducing block
 
 // ---------------------------------------------------------- reductions
 // Sums of N <= 4 FP64 values over the block, totals in threads t < N: lanes
@@ -400,6 +402,9 @@ k_it_spmv(int nb, const int *__restrict__ wc, const int *__restrict__ wr,
 }
 
 }  // namespace
+}  // namespace mtgpu
+#include "cocr_small.cuh"
+namespace mtgpu {
 
 // ---------------------------------------------------------------- solver
 void CocrSolver::release()
@@ -421,24 +426,21 @@ int cocr_alloc(CocrSolver &S)
     int dev = 0, nsm = 0;
     MTGPU_TRY(cudaGetDevice(&dev));
     MTGPU_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    // Blocks of 64 threads where all rows are resident at once, so that the
-    // FP64 pipes get even shares (45,000 rows: 10 warps on the busiest SM
-    // against 16 in blocks of 256, 9.3 on average); else blocks of 256, as many
-    // as are resident (the loops are grid-stride)
-    S.threads = nb <= nsm * 1024 ? 64 : kRedThreads;
+    // blocks of 256, as many as are resident (the loops are grid-stride)
     int occ = 64;
     const void *fs[] = {(const void *)k_it_edge, (const void *)k_it_update, (const void *)k_it_spmv,
                         (const void *)k_init_norms};
     for (const void *f : fs) {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, S.threads, 0) == cudaSuccess && b > 0)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kRedThreads, 0) == cudaSuccess && b > 0)
             occ = std::min(occ, b);
     }
-    S.grid = std::max(1, std::min(ceil_div(nb, S.threads), occ * nsm));
+    S.grid = std::max(1, std::min(ceil_div(nb, kRedThreads), occ * nsm));
+    small_grid(S, dev, nsm);
     int rc;
     if ((rc = dev_alloc(&S.r, nb)) || (rc = dev_alloc(&S.p, nb)) || (rc = dev_alloc(&S.s, nb)) ||
         (rc = dev_alloc(&S.z, nb)) || (rc = dev_alloc(&S.a, nb)) || (rc = dev_alloc(&S.w, nb)) ||
-        (rc = dev_alloc(&S.sm, nb)) || (rc = dev_alloc(&S.partials, (size_t)4 * S.grid)) ||
+        (rc = dev_alloc(&S.sm, nb)) || (rc = dev_alloc(&S.partials, (size_t)std::max(4 * S.grid, 7 * nsm))) ||
         (rc = dev_alloc(&S.ctl, 1)))
         return rc;
     MTGPU_TRY(cudaMallocHost((void **)&S.hctl, sizeof(Ctl)));
@@ -450,7 +452,7 @@ static void launch_iteration(CocrSolver &S)
 {
     const Folded &P = S.P;
     const SellMatrix &A = S.A;
-    const int nb = S.nb, g = S.grid, th = S.threads;
+    const int nb = S.nb, g = S.grid, th = kRedThreads;
     if (P.m > 0)
         pdl(k_it_node, std::max(1, std::min(ceil_div(P.m, th), g)), th, 0, S.st, P.m, P.d_gp, P.d_gj,
             P.d_gv, P.d_ds, S.z, S.a, P.d_h, S.ctl);
@@ -469,7 +471,9 @@ static int build_graph(CocrSolver &S, int iters)
     S.graph = nullptr;
     cudaGraph_t g;
     MTGPU_TRY(cudaStreamBeginCapture(S.st, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < iters; k++) launch_iteration(S);
+    if (S.g_small) launch_small(S, iters);
+    else
+        for (int k = 0; k < iters; k++) launch_iteration(S);
     MTGPU_TRY(cudaStreamEndCapture(S.st, &g));
     cudaError_t e = cudaGraphInstantiate(&S.graph, g, 0);
     cudaGraphDestroy(g);
@@ -489,7 +493,7 @@ static int sync_ctl(CocrSolver &S)
 static int true_residual(CocrSolver &S, const double2 *b, const double2 *x, double *out)
 {
     sell_residual(S.A, b, x, S.w, S.st);
-    k_norm2<<<S.grid, S.threads, 0, S.st>>>(S.nb, S.w, b, S.ctl, S.partials);
+    k_norm2<<<S.grid, kRedThreads, 0, S.st>>>(S.nb, S.w, b, S.ctl, S.partials);
     note_launches(2);
     MTGPU_TRY(cudaGetLastError());
     int rc = sync_ctl(S);
@@ -503,7 +507,7 @@ int cocr_solve(CocrSolver &S, const double2 *b, double2 *x, double eps, int maxi
                int stop_true, int iters_per_launch, mtgpu_solve_stats *stats)
 {
     const int nb = S.nb;
-    if (iters_per_launch <= 0) iters_per_launch = 16;
+    if (iters_per_launch <= 0) iters_per_launch = S.g_small ? kSmallIters : 16;
     Ctl init{};
     init.status = kRunning;
     init.maxiter = maxiter;
@@ -512,13 +516,13 @@ int cocr_solve(CocrSolver &S, const double2 *b, double2 *x, double eps, int maxi
     MTGPU_TRY(cudaMemcpyAsync(S.ctl, &init, sizeof(Ctl), cudaMemcpyHostToDevice, S.st));
     // stages 1-4 of PCOCR_RCI::Run
     sell_residual(S.A, b, x, S.r, S.st);                                    // r = b - A x
-    k_init_norms<<<S.grid, S.threads, 0, S.st>>>(nb, b, S.r, S.sm, S.ctl, S.partials);
+    k_init_norms<<<S.grid, kRedThreads, 0, S.st>>>(nb, b, S.r, S.sm, S.ctl, S.partials);
     folded_apply(S.P, S.r, S.s, S.st);                                      // s = M^-1 r
     MTGPU_TRY(cudaMemsetAsync(S.p, 0, sizeof(double2) * nb, S.st));
     MTGPU_TRY(cudaMemsetAsync(S.a, 0, sizeof(double2) * nb, S.st));
     MTGPU_TRY(cudaMemsetAsync(S.w, 0, sizeof(double2) * nb, S.st));
     sell_spmv(S.A, S.s, S.z, S.st);                                         // z = A s
-    k_init_zs<<<S.grid, S.threads, 0, S.st>>>(nb, S.z, S.s, S.ctl, S.partials);
+    k_init_zs<<<S.grid, kRedThreads, 0, S.st>>>(nb, S.z, S.s, S.ctl, S.partials);
     note_launches(S.P.m > 0 ? 6 : 5);
     MTGPU_TRY(cudaGetLastError());
     int rc = sync_ctl(S);
@@ -550,8 +554,12 @@ int cocr_solve(CocrSolver &S, const double2 *b, double2 *x, double eps, int maxi
             break;
         }
         MTGPU_TRY(cudaGraphLaunch(S.graph, S.st));
-        note_launches(kpi * (unsigned long long)iters_per_launch);
+        note_launches(S.g_small ? 1 : kpi * (unsigned long long)iters_per_launch);
         if ((rc = sync_ctl(S))) return rc;
+        if (S.hctl->status == MTGPU_ERR_TIMEOUT) {
+            set_last_message("COCR: a grid barrier did not complete");
+            return MTGPU_ERR_TIMEOUT;
+        }
     }
     if (S.hctl->status == kRunning) {
         set_last_message("COCR loop ended without a final status");

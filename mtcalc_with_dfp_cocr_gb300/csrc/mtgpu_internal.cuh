@@ -138,7 +138,9 @@ struct CocrSolver {
     Folded P;
     cudaStream_t st = nullptr;
     int nb = 0;
-    int grid = 0, threads = 256;  // blocks of the reduction kernels, and their threads
+    int grid = 0;                 // blocks of the reduction kernels
+    // one-kernel iterations (k_small64): blocks (0: not used), threads and rows per thread
+    int g_small = 0, small_threads = 0, small_items = 0;
     double2 *r = nullptr, *p = nullptr, *s = nullptr, *z = nullptr, *a = nullptr,
             *w = nullptr, *sm = nullptr;
     double *partials = nullptr;
@@ -205,6 +207,69 @@ __device__ __forceinline__ double2 cquot(double2 a, double2 b)
 {
     const double d = b.x * b.x + b.y * b.y;
     return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
+}
+
+// one component of cquot (c = 0 real, 1 imaginary), so that two lanes form the
+// quotient: a divide is 500 cycles, two of a thread 1000 even where they do not
+// depend on each other
+__device__ __forceinline__ double cquot_part(double2 a, double2 b, int c)
+{
+    const double d = b.x * b.x + b.y * b.y;
+    return (c == 0 ? a.x * b.x + a.y * b.y : a.y * b.x - a.x * b.y) / d;
+}
+
+// Barrier of all blocks of a cooperative launch on a counter that starts at 0.
+// Everything a block stored before arrive() is visible to all blocks after
+// wait() (to loads other than of the read-only path).  The wait is bounded:
+// the blocks of a cooperative launch are resident together, so it ends; if it
+// did not, the kernel gives up instead of hanging.
+constexpr int kBarPolls = 1 << 22;     // about 2 s
+struct GridBarrier {
+    unsigned int *ctr;
+    unsigned int target = 0;
+    __device__ __forceinline__ void arrive()
+    {
+        __syncthreads();
+        target += gridDim.x;
+        if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
+    }
+    // false: the other blocks did not arrive in time
+    __device__ __forceinline__ bool wait(int *late)
+    {
+        if (threadIdx.x == 0) {
+            unsigned int v = 0;
+            int q = 0;
+            for (; q < kBarPolls; q++) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+                if ((int)(v - target) >= 0) break;
+            }
+            if (q == kBarPolls) *late = 1;
+        }
+        __syncthreads();
+        return *late == 0;
+    }
+};
+// the total of output o of the blocks' partials part[output][block], from G
+// lanes of a warp (j: the lane among them), in all of them; 8 loads in flight
+template <int G>
+__device__ __forceinline__ double grid_total(const double *part, int o, int j)
+{
+    constexpr int U = 8;
+    const int B = gridDim.x;
+    double s = 0.0;
+    for (int q0 = j; q0 < B; q0 += U * G) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) v[u] = q0 + u * G < B ? __ldcg(part + (size_t)o * B + q0 + u * G) : 0.0;
+#pragma unroll
+        for (int h = 1; h < U; h <<= 1)
+#pragma unroll
+            for (int u = 0; u + h < U; u += 2 * h) v[u] += v[u + h];
+        s += v[0];
+    }
+#pragma unroll
+    for (int d = G / 2; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    return s;
 }
 
 // Counts this block on a ticket; the blocks that arrived before.  Called by

@@ -44,7 +44,6 @@ constexpr int kSmallSystems = 8;       // systems, at most
 constexpr int kSmallItems = 3;         // rows x systems per thread, at most
 constexpr int kSmallItemBytes = 6 * sizeof(float4) + sizeof(int4) + sizeof(unsigned);
 constexpr int kBarSlot = 992, kExitSlot = 1008;   // counters among the ticket slots
-constexpr int kBarPolls = 1 << 22;     // about 2 s
 
 struct SmallArgs {
     int nb;
@@ -55,32 +54,6 @@ struct SmallArgs {
     float4 *s;                         // the group's slots, nb * SP apart
     SysState *sys;
     float4 *hist, *partials;
-};
-
-struct GridBarrier {
-    unsigned int *ctr;
-    unsigned int target = 0;
-    __device__ __forceinline__ void arrive()
-    {
-        __syncthreads();
-        target += gridDim.x;
-        if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
-    }
-    // false: the other blocks did not arrive in time
-    __device__ __forceinline__ bool wait(int *late)
-    {
-        if (threadIdx.x == 0) {
-            unsigned int v = 0;
-            int q = 0;
-            for (; q < kBarPolls; q++) {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
-                if ((int)(v - target) >= 0) break;
-            }
-            if (q == kBarPolls) *late = 1;
-        }
-        __syncthreads();
-        return *late == 0;
-    }
 };
 
 // Sums over the grid for k_small: thread t carries N partial sums of system
@@ -137,34 +110,13 @@ struct SmallSum {
             if (t < W) __stcg(part + (size_t)t * gridDim.x + blockIdx.x, s);
         }
     }
-    // one output's total from G lanes of a warp, in all of them
-    template <int G>
-    static __device__ __forceinline__ double total(const double *part, int o, int j)
-    {
-        constexpr int U = 8;           // loads in flight
-        const int B = gridDim.x;
-        double s = 0.0;
-        for (int q0 = j; q0 < B; q0 += U * G) {
-            double v[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) v[u] = q0 + u * G < B ? __ldcg(part + (size_t)o * B + q0 + u * G) : 0.0;
-#pragma unroll
-            for (int h = 1; h < U; h <<= 1)
-#pragma unroll
-                for (int u = 0; u + h < U; u += 2 * h) v[u] += v[u + h];
-            s += v[0];
-        }
-#pragma unroll
-        for (int d = G / 2; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-        return s;
-    }
     // the grid's totals by the block's first kSmallMin threads
     static __device__ __forceinline__ void totals(const double *part, double (*tot)[32])
     {
         constexpr int G = kSmallMin / W < 32 ? kSmallMin / W : 32;
         const int o = threadIdx.x / G, j = threadIdx.x % G;
         if (o < W) {
-            const double s = total<G>(part, o, j);
+            const double s = grid_total<G>(part, o, j);
             if (j == 0) tot[o / SP][o % SP] = s;
         }
         __syncthreads();
@@ -175,7 +127,7 @@ struct SmallSum {
         constexpr int G = W < 32 ? 32 / W : 1;
         const int lane = threadIdx.x & 31;
         for (int o = lane / G; o < W; o += 32 / G) {
-            const double s = total<G>(part, o, lane % G);
+            const double s = grid_total<G>(part, o, lane % G);
             if (lane % G == 0) tot[o / SP][o % SP] = s;
         }
         __syncwarp();
@@ -264,13 +216,10 @@ __device__ __forceinline__ cdf small_row(const MF &M, int d, Pos p, int k, df om
     return kk.get();
 }
 
-// a / b (cquot) into a state's double and double-float forms, one component a
-// thread (c = 0 real, 1 imaginary): a divide is 500 cycles, two are 1000 even
-// where they do not depend on each other
+// a / b (cquot_part) into a state's double and double-float forms
 __device__ __forceinline__ void small_quot(double2 a, double2 b, int c, double2 &q, float4 &qf)
 {
-    const double d = b.x * b.x + b.y * b.y;
-    const double v = (c == 0 ? a.x * b.x + a.y * b.y : a.y * b.x - a.x * b.y) / d;
+    const double v = cquot_part(a, b, c);
     const df f = from_double(v);
     (c == 0 ? q.x : q.y) = v;
     (c == 0 ? qf.x : qf.y) = f.h;
