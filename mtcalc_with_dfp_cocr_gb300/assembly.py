@@ -97,13 +97,14 @@ class Assembly:
     def block2x2(self, nu, alfa, z1d, usin, ucos, eps=1e-8, maxiter=10000) -> BlockSLAE:
         inf = self.info()
         nb, nnz = self.nb, inf["nnz_lower"]
-        ig = np.zeros(nb + 1, np.int32)
-        jg = np.zeros(max(nnz, 1), np.int32)
-        idi = np.zeros(nb + 1, np.int32)
-        ijg = np.zeros(nnz + 1, np.int32)
-        di = np.zeros(2 * nb)
-        gg = np.zeros(max(inf["gg_len"], 1))
-        pr = np.zeros(2 * nb)
+        # every entry is written by the call
+        ig = np.empty(nb + 1, np.int32)
+        jg = np.empty(max(nnz, 1), np.int32)
+        idi = np.empty(nb + 1, np.int32)
+        ijg = np.empty(nnz + 1, np.int32)
+        di = np.empty(2 * nb)
+        gg = np.empty(max(inf["gg_len"], 1))
+        pr = np.empty(2 * nb)
         f = lambda v: np.ascontiguousarray(v, np.float64)
         rc = _lib.lib().mtgpu_assembly_block2x2(self._h, float(nu), int(alfa), len(z1d), f(z1d),
                                                 f(usin), f(ucos), ig, jg, idi, ijg, di, gg, pr)
