@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 namespace mtgpu {
 namespace sv {
@@ -1877,47 +1878,51 @@ k_res64(int nb, Mat64 A, const double *__restrict__ omega64, const double2 *__re
 // The same operations on the same values as one iteration at a time, so the
 // same p and x to the last bit; per iteration 1 + 6 / 16 vector passes instead
 // of the 5.4 of updating p and x in k_edge and folding x every 16 iterations
-// (1.8M edges x 2 systems: k_edge 95 -> 57 us, this kernel 11 us an iteration).
-// Four s values are in flight per thread.
+// (1.8M edges x 2 systems: k_edge 95 -> 57 us, this kernel 16 us an iteration,
+// two thirds of it arithmetic).  A whole group's s values are in flight per
+// thread (1.8M x 2: 260 us a group with 4, 251 with 16); the lanes' coefficients
+// lie side by side (512 bytes apart they met in one bank: 234,000 x 16 424 -> 258 us).
 template <int SP>
-__global__ void __launch_bounds__(kB)
+__global__ void __launch_bounds__(kB, 3)
 k_group(long long n, float4 *__restrict__ s, float4 *__restrict__ p, double2 *__restrict__ x,
         const float4 *__restrict__ hist, const SysState *sys, int rev)
 {
     pdl_wait();
-    __shared__ float4 ab[SP * kGroupIters * 2];
-    for (int i = threadIdx.x; i < SP * kGroupIters * 2; i += kB) ab[i] = hist[i];
+    __shared__ float4 ab[kGroupIters * 2][SP];
+    for (int i = threadIdx.x; i < SP * kGroupIters * 2; i += kB) ab[i % (kGroupIters * 2)][i / (kGroupIters * 2)] = hist[i];
     __syncthreads();
     const int k = threadIdx.x % SP;
     const int cnt = sys[k].cnt;
     if (cnt == 0) return;
-    const float4 *c = ab + 2 * kGroupIters * k;
     const long long stride = (long long)gridDim.x * kB;
     for (long long ii = (long long)blockIdx.x * kB + threadIdx.x; ii < n; ii += stride) {
         // n is a multiple of SP: a backward sweep by rows keeps the lane's system
         const long long i = rev ? n - SP - (ii - k) + k : ii;
         cdf pv = ldg(p + i), d = czero();
         const double2 xv = x[i];
+        const cdf last = ldg(s + cnt * n + i);
         int j = 0;
-        for (; j + 4 <= cnt; j += 4) {
-            cdf sv[4];
+        // U of the group's iterations, their loads in flight together
+        auto steps = [&](auto u_) {
+            constexpr int U = decltype(u_)::value;
+            for (; j + U <= cnt; j += U) {
+                cdf sv[U];
 #pragma unroll
-            for (int u = 0; u < 4; u++) sv[u] = ldg(s + (j + u) * n + i);
+                for (int u = 0; u < U; u++) sv[u] = ldg(s + (j + u) * n + i);
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                pv = caxpy(sv[u], cfac_of(from4(c[2 * (j + u) + 1])), pv);
-                d = caxpy(d, cfac_of(from4(c[2 * (j + u)])), pv);
+                for (int u = 0; u < U; u++) {
+                    pv = caxpy(sv[u], cfac_of(from4(ab[2 * (j + u) + 1][k])), pv);
+                    d = caxpy(d, cfac_of(from4(ab[2 * (j + u)][k])), pv);
+                }
             }
-        }
-        for (; j < cnt; j++) {
-            pv = caxpy(cdf_of(s[j * n + i]), cfac_of(from4(c[2 * j + 1])), pv);
-            d = caxpy(d, cfac_of(from4(c[2 * j])), pv);
-        }
-        const float4 last = s[cnt * n + i];
+        };
+        steps(std::integral_constant<int, 16>{});
+        steps(std::integral_constant<int, 4>{});
+        steps(std::integral_constant<int, 1>{});
         const double2 dv = to_d2(to4(d));
         x[i] = make_double2(xv.x + dv.x, xv.y + dv.y);
         p[i] = to4(pv);
-        s[i] = last;
+        s[i] = to4(last);
     }
 }
 
