@@ -341,7 +341,9 @@ int mtgpu_survey_spmv_timed(mtgpu_survey *s, int reps, float *ms);
  * re-initialises them. */
 int mtgpu_survey_spmv(mtgpu_survey *s, const double *d_x, double *d_y);
 
-/* The SpMV variant the set-up autotuning chose for the first batch (0: x segments and matrix
+/* The SpMV variant of the first batch, chosen at set-up by rule (35 where it is
+ * available and the batch has two systems or more, or iterates in one kernel)
+ * or by timing (0: x segments and matrix
  * slots staged in shared memory per tile of slices; 1: x segments staged
  * only; 2, 4, 8: slots in flight per thread, gathers from global memory;
  * 18, 20: two-system batches only, one thread per row for both systems with
@@ -358,7 +360,7 @@ int mtgpu_survey_spmv(mtgpu_survey *s, const double *d_x, double *d_y);
  * 34, 35 (ms[11]: ms
  * per whole iteration with that variant, so that each SpMV sees the cache as
  * the other kernels of an iteration leave it; 0 where a variant was not
- * available). */
+ * available or nothing was timed). */
 int mtgpu_survey_tuning(const mtgpu_survey *s, int *variant, float *ms);
 /* The environment variable MTGPU_SPMV_VARIANT, when it names a variant
  * available for the survey, replaces the autotuning at mtgpu_survey_create

@@ -1276,17 +1276,33 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
     const int pin_env = pin && *pin ? atoi(pin) : -1;
     if (pin_env >= 0 && (rc = survey_prepare_variant(V, pin_env))) return rc;
     if (pin_variant >= 0 && (rc = survey_prepare_variant(V, pin_variant))) return rc;
+    // Variant 35 without timing for two systems and more, and for one where its
+    // iterations run in one kernel.  Whole iterations, 32 / 33 / 35: 229,000 edges
+    // x systems at 2 lanes 43.2 / 42.5 / 43.2 us, 296,000 46.9 / 48.0 / 45.2, 1.6M
+    // 150 / 148 / 131; at 4 lanes 283,000 46.9 / 47.9 / 44.9, at 8 360,000 55.1 / 56.1 /
+    // 50.3, at 16 423,000 57.8 / 57.5 / 53.7, at 32 847,000 92.6 / 93.7 / 80.3, and
+    // further apart beyond.  For one system the sides change (346,000 edges 49.6
+    // / 52.1, 811,000 85.8 / 82.8): timed.  The timing took 1.6 of a forward
+    // model's 63 ms (126,000 edges x 8).
+    auto g_form = [&]() {
+        if (!V.mf.on || !V.mf.gface) return false;
+        V.ch = kMatFree + 3;
+        MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
+        return V.SP >= 2 || V.g_small > 0;
+    };
     if (pin_env >= 0 && spmv_variant_available(V, pin_env)) {
         V.ch = pin_env;
         MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
     } else if (pin_variant >= 0 && spmv_variant_available(V, pin_variant)) {
         V.ch = pin_variant;
         MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
+    } else if (g_form()) {
+        // (its grids are set)
     } else {
         // with the matrix-free operator the stored-matrix variants and the
         // tiled matrix-free one measured slower on every tensor mesh (whole
         // iterations on c2 at 2 systems: 0.67 ms and more against 0.57-0.60),
-        // so only the matrix-free forms 32, 33 and 35 are timed
+        // so only the matrix-free forms are timed
         const int cand[kSpmvVariants] = {0, 1, 2, 4, 8, kRowVariant + 2, kRowVariant + 4, kMatFree,
                                          kMatFree + 1, kMatFree + 2, kMatFree + 3};
         auto tried = [&](int v) {
@@ -1301,12 +1317,10 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
             MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
             float ms = 0.f;
             if ((rc = survey_iter_timed(V, 1, &ms))) return rc;   // warm-up
-            // (a whole group where its launch serves all of it)
-            const int reps = small_used(V) ? V.group : 3;
-            if ((rc = survey_iter_timed(V, reps, &ms))) return rc;
-            V.tune_ms[c] = ms / (float)reps;
-            if (V.tune_ms[c] < best) {
-                best = V.tune_ms[c];
+            if ((rc = survey_iter_timed(V, 3, &ms))) return rc;
+            V.tune_ms[c] = ms / 3.f;
+            if (ms < best) {
+                best = ms;
                 best_ch = cand[c];
             }
         }

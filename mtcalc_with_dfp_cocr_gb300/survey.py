@@ -79,8 +79,8 @@ class Survey:
                                                 C.c_void_p(y.data_ptr())), "mtgpu_survey_spmv")
 
     def tuning(self):
-        """(chosen SpMV variant, {variant: ms per launch}) of the set-up
-        autotuning; variants 0 and 1 stage x in shared memory per tile,
+        """(chosen SpMV variant, {variant: ms per iteration} where the set-up
+        timed them); variants 0 and 1 stage x in shared memory per tile,
         18 and 20 (two systems) run one thread per row for both systems, 32
         is the matrix-free SpMV of tensor meshes, 33 the same with two
         systems per thread, 34 the same in one tiled kernel with the edge
