@@ -425,8 +425,8 @@ int mtgpu_receivers_info(const mtgpu_receivers *r, int *nrec, int *n_unlocated, 
  *    the projection is interpolated at the receiver.  Receivers are located
  *    with boxes grown by 1e-6; a receiver with no non-air brick gets A = 0.
  *    The reference solves each projection with PARDISO; here all value types
- *    of all systems are solved together on the device by conjugate gradients
- *    to a relative residual of 1e-14.  Conforming hexahedral meshes only.
+ *    of all systems are solved together on the device by FP64 iterative
+ *    refinement to a relative residual of 1e-14.  Conforming hexahedral meshes only.
  * The assembly `a` must be the one the receivers were created on and must
  * outlive them while the output is smoothed.  The adjoint functions accept
  * the direct output only. */

@@ -166,7 +166,7 @@ __global__ void k_adj_gather(int n_touch, int S, int nrec, long long nb,
 // transverse axes, d the opposite edge), and only Im t is needed, 29
 // operations a direction; the table intervals of the edge midpoints are
 // looked up once per cell instead of once per system, table and edge.
-// 73,728 cells x 16 systems: 1,420 -> 300 us.
+// 73,728 cells x 16 systems: 1,420 -> 330 us.
 __global__ void __launch_bounds__(128)
 k_adj_grad(int kpar, int S, long long nb, const double2 *__restrict__ u,
            const double2 *__restrict__ lam, const double *__restrict__ omega,

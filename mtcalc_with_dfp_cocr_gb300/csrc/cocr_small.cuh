@@ -51,6 +51,13 @@ __device__ __forceinline__ double2 ld2(const double2 *p)
     return v;
 }
 
+// (re, im) += a b, unconjugated: two multiply-adds each
+__device__ __forceinline__ void dot_add(double &re, double &im, double2 a, double2 b)
+{
+    re = fma(-a.y, b.y, fma(a.x, b.x, re));
+    im = fma(a.y, b.x, fma(a.x, b.y, im));
+}
+
 // the sums of N <= 4 values over the block's first nw warps to part[value][block]
 template <int N>
 __device__ __forceinline__ void small_block(const double (&v)[N], int nw, double (*sm)[4], double *part)
@@ -195,8 +202,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
                 oa[u * NT] = an;
                 A.a[i] = an;
                 ow[u * NT] = wn;
-                v[0] += an.x * wn.x - an.y * wn.y;
-                v[1] += an.x * wn.y + an.y * wn.x;
+                dot_add(v[0], v[1], an, wn);
             }
             small_block<2>(v, nw, sums, part_e);
         }
@@ -231,8 +237,8 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
                 orr[u * NT] = rn;
                 const double2 sv = osm[u * NT];
                 const double ux = rn.x - sv.x, uy = rn.y - sv.y;
-                v[0] += sv.x * ux + sv.y * uy;
-                v[1] += ux * ux + uy * uy;
+                v[0] = fma(sv.y, uy, fma(sv.x, ux, v[0]));
+                v[1] = fma(uy, uy, fma(ux, ux, v[1]));
             }
             small_block<2>(v, nw, sums, part_u);
         }
@@ -286,8 +292,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
                 }
                 A.z[i] = make_double2(ar, ai);
                 const double2 si = os[u * NT];
-                v[0] += ar * si.x - ai * si.y;
-                v[1] += ar * si.y + ai * si.x;
+                dot_add(v[0], v[1], make_double2(ar, ai), si);
             }
             __syncthreads();
             const int mode = c.mrs_mode;
@@ -302,7 +307,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
                         smv = make_double2(old.x + wm * (smv.x - old.x), old.y + wm * (smv.y - old.y));
                     }
                     osm[u * NT] = smv;
-                    v[2] += smv.x * smv.x + smv.y * smv.y;
+                    v[2] = fma(smv.y, smv.y, fma(smv.x, smv.x, v[2]));
                 }
             }
             small_block<3>(v, nw, sums, part_r);

@@ -25,8 +25,9 @@
 // gather, the edge gather + (a, w), the updates + the MRS smoothing, and the
 // SpMV + (z, s) (one kernel for a stored matrix, two for the matrix-free
 // forms), captured in a CUDA graph several iterations at a time, with p and x
-// brought up to date once per group of iterations; all per-system decisions are taken on the
-// device by the block of each kernel that finishes last.
+// brought up to date once per group of iterations; all per-system decisions are
+// taken on the device by the block of each kernel that finishes last.  Small
+// problems run a group's iterations in one cooperative kernel (survey_small.cuh).
 #include "survey_impl.cuh"
 
 #include <algorithm>
