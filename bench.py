@@ -20,7 +20,7 @@ iterations.
 systems.  `e2e` goes through the reference-facing C ABI
 (mtgpu_pcocr_2x2_folded_ex, double-float) with the SLAE in host memory:
 upload, set-up, solve and download of x every solve.  `roofline` is the
-batched double-float SpMV, in the variant the set-up autotuning chose (on
+batched double-float SpMV, in the variant the set-up chose (on
 this tensor mesh the matrix-free one), against the measured HBM copy
 bandwidth.  The timed region is an NVTX range "timed" for ncu's
 --nvtx-include.
@@ -56,14 +56,14 @@ UNIT = "s/solve"
 WORKLOAD = "c2"
 # DRAM bytes of one matrix-free SpMV on c2 (two lanes, as the iteration
 # launches it), per variant: the sum of its kernels' ncu dram__bytes_read.sum
-# + dram__bytes_write.sum (profiles/bench_c2_launch_list.md,
-# profiles/spmv_matfree_c2_s2.md: variant 32's k_mf_faces + k_mf_edges,
-# variant 35's k_mf_gmarch + k_mf_edges_g)
-SPMV_MF_TRAFFIC_C2 = {32: 300.6e6, 35: 314.3e6}
+# + dram__bytes_write.sum (profiles/survey_iteration_kernels.md: variant 35's
+# k_mf_gmarch + k_mf_edges_g)
+SPMV_MF_TRAFFIC_C2 = {35: 264.7e6}
 # what bounds the matrix-free SpMV instead of HBM (ncu on c2, two lanes)
-SPMV_MF_BINDING = ("FP32 issue: k_mf_edges<2> 69 % issue-active, 51 % FMA pipe, 42 double-float "
-                   "multiply-adds of 12 FP32 instructions per edge and system "
-                   "(profiles/spmv_matfree_c2_s2.md)")
+SPMV_MF_BINDING = {
+    35: "FP32 arithmetic and load latency: k_mf_edges_g<2> FMA pipe 49 %, L1 77 %, 16 warps an SM "
+        "at 126 registers; k_mf_gmarch<2> FMA pipe 39 %, load latency "
+        "(profiles/survey_iteration_kernels.md)"}
 
 
 def load_peaks():
@@ -280,7 +280,7 @@ def gpu_arm(args):
     plain_value = (ms_plain / 1e3) / (plain_steps * S * world)
 
     # roofline of the dominant kernel: the batched double-float SpMV, in the
-    # variant the set-up autotuning chose
+    # variant the set-up chose
     peak, peak_kind = load_peaks()
     sv = survey.Survey(A, nus, stream)
     variant = sv.tuning()[0]
@@ -316,7 +316,7 @@ def gpu_arm(args):
             spmv_kernel = f"k_mf_faces + {edges} (matrix-free double-float SpMV, S systems)"
         traffic = SPMV_MF_TRAFFIC_C2.get(variant) if WORKLOAD == "c2" else None
         traffic_src = (f"ncu dram__bytes_read.sum + dram__bytes_write.sum of the variant-{variant} "
-                       f"kernels on c2 (profiles/bench_c2_launch_list.md)") if traffic else None
+                       f"kernels on c2 (profiles/survey_iteration_kernels.md)") if traffic else None
     else:
         spmv_bytes = nc * (4 + 8 + 8) + nr * (4 + 8) + meta + 2 * S * 16 * nb + tail
         spmv_kernel = f"k_spmv variant {variant} (batched double-float SELL-32 SpMV, S systems)"
@@ -324,13 +324,14 @@ def gpu_arm(args):
         traffic_src = None
     achieved = spmv_bytes / (spmv_ms * 1e-3) / 1e9
     # the whole iteration against HBM: the algorithmic bytes of its five
-    # kernels (node: z, a gathered, D_S read, h written; edge: s, p, z, a,
-    # D_A, x read, p, a, w, x written, h gathered, the compact G^T row;
-    # update: a, w, s_m, r, s read, r, s, s_m written; the SpMV as above)
+    # kernels (node: z, a gathered, D_S read, h written; edge: z, a, D_A
+    # read, a, w written, h gathered, the compact G^T row; update: a, w, s_m,
+    # r, s read, r, s, s_m written; the SpMV as above) and a sixteenth of the
+    # group's (17 s, p, x read, s, p, x written)
     # over the solve's time per iteration (its set-up and FP64 checks
     # included); m = the interior nodes, the rows of G on these meshes
     m_nodes = (m_.nx - 2) * (m_.ny - 2) * (m_.nz - 2)
-    iter_bytes = 16 * SP * (20 * nb + 3 * m_nodes) + 8 * nb + spmv_bytes
+    iter_bytes = 16 * SP * ((15 + 22 / 16) * nb + 3 * m_nodes) + 8 * nb + spmv_bytes
     iter_ms = 1e3 * batched["seconds"] / max(batched["iterations"])
     # the FP64 SpMV of the plain path (bound by the FP64 pipe on GB300)
     ctx = A.cocr(nus[0], stream)
@@ -418,7 +419,7 @@ def gpu_arm(args):
                      "frac": achieved / peak, "peak_kind": f"{peak_kind} hbm_gbs",
                      "bytes_per_launch": spmv_bytes, "ms_per_launch": spmv_ms,
                      "traffic": traffic, "traffic_source": traffic_src,
-                     "binding": SPMV_MF_BINDING if variant in (32, 33, 35) else None},
+                     "binding": SPMV_MF_BINDING.get(variant)},
         "roofline_iteration": {"bound": "hbm", "achieved": iter_bytes / (iter_ms * 1e-3) / 1e9,
                                "peak": peak, "unit": "GB/s",
                                "frac": iter_bytes / (iter_ms * 1e-3) / 1e9 / peak,
