@@ -42,6 +42,7 @@ struct Ctl {
     double sums[4];      // scratch results of one-off reductions
     unsigned int ticket[4];
     unsigned int bar, left;   // k_small64: barrier arrivals, blocks that left
+    int failed, polls;        // ... a wait ran out (set by kernels, cleared by the host); its bound
 };
 
 namespace {
@@ -513,6 +514,7 @@ int cocr_solve(CocrSolver &S, const double2 *b, double2 *x, double eps, int maxi
     init.maxiter = maxiter;
     init.eps = eps;
     init.x = x;
+    init.polls = barrier_polls();
     MTGPU_TRY(cudaMemcpyAsync(S.ctl, &init, sizeof(Ctl), cudaMemcpyHostToDevice, S.st));
     // stages 1-4 of PCOCR_RCI::Run
     sell_residual(S.A, b, x, S.r, S.st);                                    // r = b - A x
@@ -556,7 +558,7 @@ int cocr_solve(CocrSolver &S, const double2 *b, double2 *x, double eps, int maxi
         MTGPU_TRY(cudaGraphLaunch(S.graph, S.st));
         note_launches(S.g_small ? 1 : kpi * (unsigned long long)iters_per_launch);
         if ((rc = sync_ctl(S))) return rc;
-        if (S.hctl->status == MTGPU_ERR_TIMEOUT) {
+        if (S.hctl->failed) {
             set_last_message("COCR: a grid barrier did not complete");
             return MTGPU_ERR_TIMEOUT;
         }

@@ -107,13 +107,13 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
             *orr = ow + items * NT, *os = orr + items * NT, *osm = os + items * NT, *oda = osm + items * NT;
     int2 *otn = reinterpret_cast<int2 *>(own64 + 8 * items * NT) + tid;
     double *part_e = A.partials, *part_u = part_e + 2 * B, *part_r = part_u + 2 * B;
-    GridBarrier bar{&A.ctl->bar};
 
     if (tid == 0) {
         c = *A.ctl;
         late = 0;
     }
     __syncthreads();
+    GridBarrier bar{&A.ctl->bar, &A.ctl->failed, c.polls};
     double2 *const x = c.x;
     for (int u = 0; u < items; u++) {
         const int i = row0 + u * stride;
@@ -336,10 +336,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
         if (tid == 0) c.zs = zs_new;
     }
     __syncthreads();
-    if (late) {
-        if (tid == 0) A.ctl->status = MTGPU_ERR_TIMEOUT;
-        return;
-    }
+    if (late) return;
     if (any) {
         for (int u = 0; u < items; u++) {
             const int i = row0 + u * stride;
@@ -350,7 +347,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
             A.sm[i] = osm[u * NT];
         }
         if (blockIdx.x == 0 && tid == 0) {
-            Ctl *q = A.ctl;               // all but the counters
+            Ctl *q = A.ctl;               // all but the barrier's words
             q->status = c.status;
             q->iter = c.iter;
             q->mrs_mode = c.mrs_mode;

@@ -222,10 +222,17 @@ __device__ __forceinline__ double cquot_part(double2 a, double2 b, int c)
 // Everything a block stored before arrive() is visible to all blocks after
 // wait() (to loads other than of the read-only path).  The wait is bounded:
 // the blocks of a cooperative launch are resident together, so it ends; if it
-// did not, the kernel gives up instead of hanging.
+// did not, the block marks the solve as failed and leaves instead of hanging.
+// The other blocks may still pass that barrier (the late block had arrived at
+// it) and end the launch as if nothing had happened, so the mark is a word that
+// kernels only ever set: the launches after it end at their start, and the
+// host, which alone clears it (with the counters) when a solve begins, fails
+// the solve whatever its state says.
 constexpr int kBarPolls = 1 << 22;     // about 2 s
 struct GridBarrier {
     unsigned int *ctr;
+    int *failed;                       // the mark, in device memory
+    int polls;                         // ... after this many (0: kBarPolls)
     unsigned int target = 0;
     __device__ __forceinline__ void arrive()
     {
@@ -238,17 +245,28 @@ struct GridBarrier {
     {
         if (threadIdx.x == 0) {
             unsigned int v = 0;
+            const int n = polls > 0 ? polls : kBarPolls;
             int q = 0;
-            for (; q < kBarPolls; q++) {
+            for (; q < n; q++) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
                 if ((int)(v - target) >= 0) break;
             }
-            if (q == kBarPolls) *late = 1;
+            if (q == n) {
+                *late = 1;
+                *(volatile int *)failed = 1;
+            }
         }
         __syncthreads();
         return *late == 0;
     }
 };
+// MTGPU_BARRIER_POLLS (environment) lowers the bound of the waits, so that a
+// test makes one run out
+inline int barrier_polls()
+{
+    const char *e = getenv("MTGPU_BARRIER_POLLS");
+    return e ? std::max(0, atoi(e)) : 0;
+}
 // the total of output o of the blocks' partials part[output][block], from G
 // lanes of a warp (j: the lane among them), in all of them; 8 loads in flight
 template <int G>

@@ -466,7 +466,7 @@ const Ops &ops_of(int sp)
 
 int sync_sys(Survey &V)
 {
-    MTGPU_TRY(cudaMemcpyAsync(V.hsys, V.sys, sizeof(SysState) * 32, cudaMemcpyDeviceToHost, V.st));
+    MTGPU_TRY(cudaMemcpyAsync(V.hsys, V.sys, sizeof(SysState) * kSysSlots, cudaMemcpyDeviceToHost, V.st));
     MTGPU_TRY(cudaStreamSynchronize(V.st));
     return MTGPU_OK;
 }
@@ -1085,7 +1085,7 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
         (rc = dev_alloc(&V.kr, P.len_r)) || (rc = dev_alloc(&V.da, nv)) ||
         (rc = dev_alloc(&V.ds, (size_t)mm * V.SP)) || (rc = dev_alloc(&V.gkg, mm)) ||
         (rc = dev_alloc(&V.gmg, mm)) || (rc = dev_alloc(&V.omega, 32)) ||
-        (rc = dev_alloc(&V.omega64, 32)) || (rc = dev_alloc(&V.sys, 32)) ||
+        (rc = dev_alloc(&V.omega64, 32)) || (rc = dev_alloc(&V.sys, kSysSlots)) ||
         (rc = dev_alloc(&V.r, nv)) || (rc = dev_alloc(&V.p, nv)) || (rc = dev_alloc(&V.a, nv)) ||
         (rc = dev_alloc(&V.z, nv)) || (rc = dev_alloc(&V.w, nv)) || (rc = dev_alloc(&V.sm, nv)) ||
         (rc = dev_alloc(&V.h, (size_t)mm * V.SP)) || (rc = dev_alloc(&V.b64, nv)) ||
@@ -1101,7 +1101,8 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
     while (V.group > 1 && (size_t)(V.group + 1) * nv * sizeof(float4) > mem_free / 4) V.group /= 2;
     if ((rc = dev_alloc(&V.s, (size_t)(V.group + 1) * nv))) return rc;
     MTGPU_TRY(cudaMemsetAsync(V.partials, 0, sizeof(float4) * kTicketSlots, st));
-    MTGPU_TRY(cudaMallocHost((void **)&V.hsys, sizeof(SysState) * 32));
+    MTGPU_TRY(cudaMemsetAsync(V.sys, 0, sizeof(SysState) * kSysSlots, st));
+    MTGPU_TRY(cudaMallocHost((void **)&V.hsys, sizeof(SysState) * kSysSlots));
     trace.mark("allocations");
     std::vector<float2> omdf(32, make_float2(0.f, 0.f));
     std::vector<double> om64(32, 0.0);
@@ -1458,7 +1459,7 @@ namespace {
 
 int upload_sys(Survey &V)
 {
-    MTGPU_TRY(cudaMemcpyAsync(V.sys, V.hsys, sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
+    MTGPU_TRY(cudaMemcpyAsync(V.sys, V.hsys, sizeof(SysState) * kSysSlots, cudaMemcpyHostToDevice, V.st));
     return sync_sys(V);
 }
 
@@ -1523,6 +1524,8 @@ int survey_begin(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, do
         s.eps_k = eps;
         V.hsys[k] = s;
     }
+    V.hsys[kBarState] = SysState{};
+    V.hsys[kBarState].maxiter = barrier_polls();
     int rc;
     // (the ticket slots: a launch that gave up leaves its counters behind)
     MTGPU_TRY(cudaMemsetAsync(V.partials, 0, sizeof(float4) * kTicketSlots, V.st));
@@ -1585,7 +1588,7 @@ int survey_launch(Survey &V, SurveyRun &R)
     note_launches(kpi * (unsigned long long)R.ipl + (small_used(V) ? 2u : 1u) * ceil_div(R.ipl, V.group));
     R.guard += R.ipl;
     // the state arrives with the launch's end (read in survey_collect)
-    MTGPU_TRY(cudaMemcpyAsync(V.hsys, V.sys, sizeof(SysState) * 32, cudaMemcpyDeviceToHost, V.st));
+    MTGPU_TRY(cudaMemcpyAsync(V.hsys, V.sys, sizeof(SysState) * kSysSlots, cudaMemcpyDeviceToHost, V.st));
     R.launched = true;
     return MTGPU_OK;
 }
@@ -1602,13 +1605,13 @@ int survey_collect(Survey &V, SurveyRun &R)
             set_last_message("survey solve did not finish within its iteration guard");
             return MTGPU_ERR_TIMEOUT;
         }
+        if (V.hsys[kBarState].status != 0) {
+            set_last_message("survey solve: a grid barrier did not complete");
+            return MTGPU_ERR_TIMEOUT;
+        }
         bool changed = false;
         for (int k = 0; k < V.S; k++) {
             SysState &q = V.hsys[k];
-            if (q.status == MTGPU_ERR_TIMEOUT) {
-                set_last_message("survey solve: a grid barrier did not complete");
-                return MTGPU_ERR_TIMEOUT;
-            }
             if (q.status != kRun) continue;
             if (q.residual_rel < 0.5 * R.best[k]) {
                 R.best[k] = q.residual_rel;

@@ -27,6 +27,11 @@ struct SysState {
     unsigned int ticket[6];  // block-completion counters (system 0 only)
 };
 
+// The state slots: the systems' and one for the grid barrier of k_small, whose
+// status is set when a wait ran out (the host clears it) and whose maxiter
+// bounds the waits (0: the default)
+constexpr int kBarState = 32, kSysSlots = 33;
+
 // Iterations per group: p and x are needed by nothing in the iteration, so
 // the group's s vectors, alpha and beta are kept and p = s + beta p, x +=
 // alpha p applied for the whole group by one kernel (k_group)

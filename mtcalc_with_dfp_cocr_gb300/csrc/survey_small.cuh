@@ -35,9 +35,10 @@ namespace sv {
 // Phases read what other blocks wrote in the same launch: those loads go
 // through ldg (ld.global after the barrier's acquire), never the read-only path.
 //
-// Every wait is bounded: one that runs out ends the launch in all blocks with
-// status MTGPU_ERR_TIMEOUT for the running systems.  The launch is
-// cooperative, so all blocks are resident and the waits end.
+// Every wait is bounded; one that runs out fails the solve with
+// MTGPU_ERR_TIMEOUT (GridBarrier; the mark and the bound are the state slot
+// after the systems').  The launch is cooperative, so all blocks are resident
+// and the waits end.
 constexpr int kSmallThreads = 480;     // threads with rows, at most; one warp more for the stop test
 constexpr int kSmallMin = 256;         // ... at least
 constexpr int kSmallSystems = 8;       // systems, at most
@@ -249,7 +250,8 @@ k_small(const __grid_constant__ MF M, const __grid_constant__ SmallArgs A, int n
     unsigned int *tickets = reinterpret_cast<unsigned int *>(A.partials);
     double *part_e = reinterpret_cast<double *>(A.partials + kTicketSlots), *part_u = part_e + (size_t)B * 2 * SP,
            *part_r = part_u + (size_t)B * 4 * SP;
-    GridBarrier bar{tickets + kBarSlot};
+    SysState *const bs = A.sys + kBarState;
+    GridBarrier bar{tickets + kBarSlot, &bs->status, bs->maxiter};
     const df om = d2f(A.omega[k]);
 
     if (tid < SP) {
@@ -257,7 +259,9 @@ k_small(const __grid_constant__ MF M, const __grid_constant__ SmallArgs A, int n
         st[tid].cnt = 0;
         brk[tid] = 0;
     }
-    if (tid == 0) late = 0;
+    if (tid == 0) late = *(volatile const int *)&bs->status != 0;
+    __syncthreads();
+    if (late) return;                  // an earlier launch failed
     for (int u = 0; u < items; u++) {
         const int e = row0 + u * stride, i = e * SP + k;
         if (e >= A.nb) break;
@@ -459,10 +463,7 @@ k_small(const __grid_constant__ MF M, const __grid_constant__ SmallArgs A, int n
         }
     }
     __syncthreads();
-    if (late) {
-        if (tid < SP && st[tid].status == kRun) A.sys[tid].status = MTGPU_ERR_TIMEOUT;
-        return;
-    }
+    if (late) return;
     for (int u = 0; u < items; u++) {
         const int e = row0 + u * stride, i = e * SP + k;
         if (e >= A.nb) break;
