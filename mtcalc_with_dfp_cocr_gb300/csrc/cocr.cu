@@ -535,8 +535,9 @@ int cocr_solve(CocrSolver &S, const double2 *b, double2 *x, double eps, int maxi
 
     const unsigned long long kpi = (unsigned long long)kernels_per_iteration(S);
     double true_rr = -1.0;
-    // every launch advances at least one iteration until the status is final
-    for (long long guard = 0; guard <= (long long)maxiter + 2; guard += iters_per_launch) {
+    // a launch runs at least one iteration and the device stops at maxiter, so
+    // maxiter + 2 launches are enough; looking at a stop and going on is none
+    for (long long left = (long long)maxiter + 2;;) {
         if (S.hctl->status != kRunning) {
             if (S.hctl->status == MTGPU_OK && stop_true) {
                 if ((rc = true_residual(S, b, x, &true_rr))) return rc;
@@ -555,6 +556,10 @@ int cocr_solve(CocrSolver &S, const double2 *b, double2 *x, double eps, int maxi
             }
             break;
         }
+        if (left-- <= 0) {
+            set_last_message("COCR loop ended without a final status");
+            return MTGPU_ERR_TIMEOUT;
+        }
         MTGPU_TRY(cudaGraphLaunch(S.graph, S.st));
         note_launches(S.g_small ? 1 : kpi * (unsigned long long)iters_per_launch);
         if ((rc = sync_ctl(S))) return rc;
@@ -562,10 +567,6 @@ int cocr_solve(CocrSolver &S, const double2 *b, double2 *x, double eps, int maxi
             set_last_message("COCR: a grid barrier did not complete");
             return MTGPU_ERR_TIMEOUT;
         }
-    }
-    if (S.hctl->status == kRunning) {
-        set_last_message("COCR loop ended without a final status");
-        return MTGPU_ERR_TIMEOUT;
     }
     if (true_rr < 0.0 && (rc = true_residual(S, b, x, &true_rr))) return rc;
     if (stats) {
