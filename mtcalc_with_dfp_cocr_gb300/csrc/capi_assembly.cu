@@ -362,6 +362,14 @@ int mtgpu_survey_create_multi(int nmesh, mtgpu_assembly *const *a, const int *S,
         }
         k0 += S[m];
     }
+    // with the memory of all batches taken, what is left goes to longer groups
+    for (auto &g : s->groups) {
+        const int rc = batches > 1 ? survey_lengthen_group(*g) : MTGPU_OK;
+        if (rc) {
+            mtgpu_survey_destroy(s);
+            return rc;
+        }
+    }
     *out = s;
     return MTGPU_OK;
 }

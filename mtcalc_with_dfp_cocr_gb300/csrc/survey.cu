@@ -1042,6 +1042,36 @@ int prec_tile_setup(Survey &V, int nsm)
 
 }  // namespace
 
+namespace {
+// iterations per group: 16, fewer where their s vectors would take more than
+// a quarter of the free memory (1: no more memory than without groups)
+int group_length(const Survey &V, int *group)
+{
+    size_t mem_free = 0, mem_total = 0;
+    MTGPU_TRY(cudaMemGetInfo(&mem_free, &mem_total));
+    const size_t vec = sizeof(float4) * (size_t)V.nb * V.SP;
+    int g = kGroupIters;
+    while (g > 1 && (size_t)(g + 1) * vec > mem_free / 4) g /= 2;
+    *group = g;
+    return MTGPU_OK;
+}
+}  // namespace
+
+int survey_lengthen_group(Survey &V)
+{
+    int g = 1, rc;
+    if ((rc = group_length(V, &g)) || g <= V.group) return rc;
+    float4 *s = nullptr;
+    if (dev_alloc(&s, (size_t)(g + 1) * V.nb * V.SP)) {
+        cudaGetLastError();       // (other users of the GPU: the short group stays)
+        return MTGPU_OK;
+    }
+    dev_free(V.s);
+    V.s = s;
+    V.group = g;
+    return MTGPU_OK;
+}
+
 int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const double *omega,
                  Survey &V, cudaStream_t st, const mtgpu_assembly_s *a, const MatFreeMesh *mfm,
                  int pin_variant)
@@ -1093,12 +1123,11 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
         (rc = dev_alloc(&V.partials, partial_slots(std::max(gmax, nsm * 32), V.SP))))
         return rc;
     V.pblocks = std::max(gmax, nsm * 32);
-    // the s vectors of a group of iterations: 16, fewer where they would take
-    // more than a quarter of the free memory (1: no more than without groups)
-    size_t mem_free = 0, mem_total = 0;
-    MTGPU_TRY(cudaMemGetInfo(&mem_free, &mem_total));
-    V.group = kGroupIters;
-    while (V.group > 1 && (size_t)(V.group + 1) * nv * sizeof(float4) > mem_free / 4) V.group /= 2;
+    // the s vectors of a group of iterations.  Of a survey of several batches,
+    // 1 for now: the batches set up after this one need their memory first
+    // (survey_lengthen_group)
+    V.group = 1;
+    if (V.alone && (rc = group_length(V, &V.group))) return rc;
     if ((rc = dev_alloc(&V.s, (size_t)(V.group + 1) * nv))) return rc;
     MTGPU_TRY(cudaMemsetAsync(V.partials, 0, sizeof(float4) * kTicketSlots, st));
     MTGPU_TRY(cudaMemsetAsync(V.sys, 0, sizeof(SysState) * kSysSlots, st));

@@ -174,6 +174,9 @@ struct MatFreeMesh {
 int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const double *omega,
                  Survey &V, cudaStream_t st, const mtgpu_assembly_s *a = nullptr,
                  const MatFreeMesh *mfm = nullptr, int pin_variant = -1);
+// lengthens the group of iterations that a batch of a survey of several batches
+// was set up with, once all of them are
+int survey_lengthen_group(Survey &V);
 // b, x: system-major FP64 [S][nb] complex; x is the initial guess in and the
 // solution out.  verify: continue until the true residual is below eps too.
 int survey_solve(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, double eps,
