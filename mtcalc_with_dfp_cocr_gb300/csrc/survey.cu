@@ -98,32 +98,54 @@ __global__ void k_g_lattice_check(MF M, int m, const int *__restrict__ gp, const
     if (nbad) atomicAdd(bad, 1);
 }
 
-// largest |a - b| and |b| over n float4 double-float pairs (as ordered bits
-// of non-negative doubles)
-__global__ void k_maxdiff(long long n, const float4 *__restrict__ a, const float4 *__restrict__ b,
-                          unsigned long long *out)
+// Two row-major vectors of double-float values, the lanes of the batch's S
+// systems: out[0], out[1] the largest |a - b| and |b| (bits of a double),
+// out[2] whether any value differs, out[3] whether any is a NaN.
+// The magnitudes are FP32 (FP64 values and an atomic per thread took 590 us
+// for 19.5M complex values): |a - b| to 2^-47 |b| and 2^-23 of itself, for
+// the tolerances; equality is out[2]'s, word by word.
+__global__ void k_maxdiff(long long n, int S, int SP, const float4 *__restrict__ a,
+                          const float4 *__restrict__ b, unsigned long long *out)
 {
-    // in FP32, so 0 iff all values are equal and within 2^-23 of the largest
-    // difference otherwise, one atomic per block: FP64 values and an atomic
-    // per thread took 590 us for 19.5M complex values
     float dm = 0.f, bm = 0.f;
+    bool differs = false, nan = false;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
+        if ((int)(i & (SP - 1)) >= S) continue;       // lanes that nothing writes
         const float4 u = a[i], v = b[i];
-        dm = fmaxf(dm, fmaxf(fabsf((u.x - v.x) + (u.z - v.z)), fabsf((u.y - v.y) + (u.w - v.w))));
+        differs |= !(u.x == v.x && u.y == v.y && u.z == v.z && u.w == v.w);
+        const float re = (u.x - v.x) + (u.z - v.z), im = (u.y - v.y) + (u.w - v.w);
+        nan |= re != re || im != im;
+        dm = fmaxf(dm, fmaxf(fabsf(re), fabsf(im)));
         bm = fmaxf(bm, fmaxf(fabsf(v.x + v.z), fabsf(v.y + v.w)));
     }
-    __shared__ unsigned int mx[2];
-    if (threadIdx.x < 2) mx[threadIdx.x] = 0u;
+    __shared__ unsigned int mx[4];
+    if (threadIdx.x < 4) mx[threadIdx.x] = 0u;
     __syncthreads();
     // the order of non-negative floats is that of their bits
     atomicMax(&mx[0], __float_as_uint(dm));
     atomicMax(&mx[1], __float_as_uint(bm));
+    if (differs) mx[2] = 1u;
+    if (nan) mx[3] = 1u;
     __syncthreads();
     if (threadIdx.x < 2)
         atomicMax(out + threadIdx.x,
                   (unsigned long long)__double_as_longlong((double)__uint_as_float(mx[threadIdx.x])));
+    else if (threadIdx.x < 4 && mx[threadIdx.x])
+        atomicMax(out + threadIdx.x, 1ull);
 }
+struct MaxDiff {
+    unsigned long long w[4] = {0, 0, 1, 1};
+    bool equal() const { return w[2] == 0; }
+    // |a - b| / |b| by the largest of each; 1 where there is nothing to compare or a NaN
+    double relative() const
+    {
+        double d, m;
+        memcpy(&d, &w[0], sizeof(double));
+        memcpy(&m, &w[1], sizeof(double));
+        return m > 0.0 && w[3] == 0 ? d / m : 1.0;
+    }
+};
 
 // a fixed pseudo-random test vector (double-float values in [-1, 1))
 __global__ void k_pattern(long long n, float4 *v)
@@ -812,7 +834,7 @@ int matfree_build(Survey &V, const MatFreeMesh &a, const DevMesh &dm, int kuz, i
     }
     const long long n = (long long)V.nb * V.SP;
     unsigned long long *d_mx = nullptr;
-    if ((rc = dev_alloc(&d_mx, 2))) return rc;
+    if ((rc = dev_alloc(&d_mx, 4))) return rc;
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
     k_pattern<<<4 * nsm, kB, 0, V.st>>>(n, V.s);
     V.ch = 4;
@@ -823,13 +845,13 @@ int matfree_build(Survey &V, const MatFreeMesh &a, const DevMesh &dm, int kuz, i
     V.ch = kMatFree;
     MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
     MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
-    MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(unsigned long long) * 2, V.st));
-    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.z, V.w, d_mx);
+    MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(MaxDiff), V.st));
+    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.S, V.SP, V.z, V.w, d_mx);
     note_launches(5);
-    unsigned long long mx[2] = {0, 0};
+    MaxDiff mx;
     err = cudaGetLastError();
     if (err == cudaSuccess)
-        err = cudaMemcpyAsync(mx, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, V.st);
+        err = cudaMemcpyAsync(mx.w, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, V.st);
     if (err == cudaSuccess) err = cudaStreamSynchronize(V.st);
     dev_free(d_mx);
     V.ch = ch;
@@ -838,10 +860,7 @@ int matfree_build(Survey &V, const MatFreeMesh &a, const DevMesh &dm, int kuz, i
         set_last_error(err, "matrix-free SpMV set-up check", __FILE__, __LINE__);
         return MTGPU_ERR_CUDA;
     }
-    double dmax, bmax;
-    memcpy(&dmax, &mx[0], sizeof(double));
-    memcpy(&bmax, &mx[1], sizeof(double));
-    const double check = bmax > 0.0 ? dmax / bmax : 1.0;
+    const double check = mx.relative();
     if (!(check < 1e-9)) {
         F.release();   // not this matrix's operator: variant off, memory back
         F.check = check;
@@ -865,22 +884,20 @@ int matfree_build(Survey &V, const MatFreeMesh &a, const DevMesh &dm, int kuz, i
         MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
         V.ch = ch;
         MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
-        if ((rc = dev_alloc(&d_mx, 2))) return rc;
-        MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(unsigned long long) * 2, V.st));
-        k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.z, V.w, d_mx);
+        if ((rc = dev_alloc(&d_mx, 4))) return rc;
+        MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(MaxDiff), V.st));
+        k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.S, V.SP, V.z, V.w, d_mx);
         note_launches(4 + spmv_extra_launches(kMatFree) + spmv_extra_launches(kMatFree + 3));
         err = cudaGetLastError();
         if (err == cudaSuccess)
-            err = cudaMemcpyAsync(mx, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, V.st);
+            err = cudaMemcpyAsync(mx.w, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, V.st);
         if (err == cudaSuccess) err = cudaStreamSynchronize(V.st);
         dev_free(d_mx);
         if (err != cudaSuccess) {
             set_last_error(err, "face-mass matrix-free SpMV set-up check", __FILE__, __LINE__);
             return MTGPU_ERR_CUDA;
         }
-        memcpy(&dmax, &mx[0], sizeof(double));
-        memcpy(&bmax, &mx[1], sizeof(double));
-        F.gface = bmax > 0.0 && dmax / bmax < 1e-12;
+        F.gface = mx.relative() < 1e-12;
     }
     return MTGPU_OK;
 }
@@ -917,14 +934,14 @@ int matfree_tile_check(Survey &V, int nsm)
     V.ch = ch;
     MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
     unsigned long long *d_mx = nullptr;
-    int rc = dev_alloc(&d_mx, 2);
+    int rc = dev_alloc(&d_mx, 4);
     if (rc) return rc;
-    MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(unsigned long long) * 2, V.st));
-    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.z, V.w, d_mx);
+    MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(MaxDiff), V.st));
+    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.S, V.SP, V.z, V.w, d_mx);
     note_launches(4 + spmv_extra_launches(kMatFree));
-    unsigned long long mx[2] = {0, 0};
+    MaxDiff mx;
     cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess) err = cudaMemcpyAsync(mx, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, V.st);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(mx.w, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, V.st);
     if (err == cudaSuccess) err = cudaStreamSynchronize(V.st);
     dev_free(d_mx);
     if (err != cudaSuccess) {
@@ -932,9 +949,7 @@ int matfree_tile_check(Survey &V, int nsm)
         set_last_error(err, "tiled matrix-free SpMV set-up check", __FILE__, __LINE__);
         return MTGPU_ERR_CUDA;
     }
-    double dm;
-    memcpy(&dm, &mx[0], sizeof(double));
-    F.tiled = dm == 0.0;
+    F.tiled = mx.equal();
     return MTGPU_OK;
 }
 
@@ -992,7 +1007,7 @@ int prec_tile_setup(Survey &V, int nsm)
     }
     float4 *ref = nullptr;
     unsigned long long *d_mx = nullptr;
-    if ((rc = dev_alloc(&ref, (size_t)2 * n)) || (rc = dev_alloc(&d_mx, 2))) {
+    if ((rc = dev_alloc(&ref, (size_t)2 * n)) || (rc = dev_alloc(&d_mx, 4))) {
         dev_free(ref);
         return rc;
     }
@@ -1009,13 +1024,13 @@ int prec_tile_setup(Survey &V, int nsm)
     MTGPU_TRY(cudaMemcpyAsync(V.a2, V.a, sizeof(float4) * n, cudaMemcpyDeviceToDevice, V.st));
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
     MTGPU_SP_DISPATCH(V.SP, precond_step(V, true, V.p, V.a2));
-    MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(unsigned long long) * 2, V.st));
-    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.w, ref, d_mx);
-    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.a2, ref + n, d_mx);
+    MTGPU_TRY(cudaMemsetAsync(d_mx, 0, sizeof(MaxDiff), V.st));
+    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.S, V.SP, V.w, ref, d_mx);
+    k_maxdiff<<<4 * nsm, kB, 0, V.st>>>(n, V.S, V.SP, V.a2, ref + n, d_mx);
     note_launches(5);
-    unsigned long long mx[2] = {1, 1};
+    MaxDiff mx;
     cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess) err = cudaMemcpyAsync(mx, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, V.st);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(mx.w, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, V.st);
     if (err == cudaSuccess) err = cudaStreamSynchronize(V.st);
     dev_free(ref);
     dev_free(d_mx);
@@ -1023,9 +1038,7 @@ int prec_tile_setup(Survey &V, int nsm)
         set_last_error(err, "fused preconditioner set-up check", __FILE__, __LINE__);
         return MTGPU_ERR_CUDA;
     }
-    double dm;
-    memcpy(&dm, &mx[0], sizeof(double));
-    if (dm != 0.0) {   // not bit-equal: keep the two-kernel form
+    if (!mx.equal()) {   // not bit-equal: keep the two-kernel form
         dev_free(V.a2);
         return MTGPU_OK;
     }
@@ -1266,7 +1279,7 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
         }
         const long long n = (long long)V.nb * V.SP, nh = (long long)V.G.m * V.SP;
         unsigned long long *d_mx = nullptr;
-        if ((rc = dev_alloc(&d_mx, 2))) return rc;
+        if ((rc = dev_alloc(&d_mx, 4))) return rc;
         k_pattern<<<4 * nsm, kB, 0, st>>>(n, V.z);
         k_pattern<<<4 * nsm, kB, 0, st>>>(n, V.p);
         cudaError_t e = cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, st);
@@ -1277,22 +1290,22 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
         if (e == cudaSuccess) {
             V.g_lat = false;
             MTGPU_SP_DISPATCH(V.SP, node(V, V.z, V.p, 1));   // CSR form -> h
-            e = cudaMemsetAsync(d_mx, 0, sizeof(unsigned long long) * 2, st);
+            e = cudaMemsetAsync(d_mx, 0, sizeof(MaxDiff), st);
         }
         if (e == cudaSuccess) {
-            k_maxdiff<<<4 * nsm, kB, 0, st>>>(nh, V.h, V.w, d_mx);
+            k_maxdiff<<<4 * nsm, kB, 0, st>>>(nh, V.S, V.SP, V.h, V.w, d_mx);
             note_launches(5);
             e = cudaGetLastError();
         }
-        unsigned long long mx[2] = {1, 1};
-        if (e == cudaSuccess) e = cudaMemcpyAsync(mx, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, st);
+        MaxDiff mx;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(mx.w, d_mx, sizeof(mx), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         dev_free(d_mx);
         if (e != cudaSuccess) {
             set_last_error(e, "lattice G check", __FILE__, __LINE__);
             return MTGPU_ERR_CUDA;
         }
-        V.g_lat = mx[0] == 0;
+        V.g_lat = mx.equal();
     }
     trace.mark(!V.mf.on ? "no matrix-free tables" : (V.g_lat ? "matrix-free, lattice G" : "matrix-free tables"));
     // the stored matrix's tiles (variants 0, 1) where there is no
