@@ -200,13 +200,23 @@ void pdl(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t 
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
-// a / b where |b|^2 is far inside FP64's range (grid sums): the quotient is
-// formed from it directly, one divide (500 cycles here) deep instead of the
-// two of cdiv's scaling against overflow
+// the power of two that brings the larger component of b to [1, 2) (a zero,
+// infinite or NaN b stays one)
+__device__ __forceinline__ double pow2_of(double2 b)
+{
+    const int e = max(__double2hiint(b.x) & 0x7ff00000, __double2hiint(b.y) & 0x7ff00000);
+    return __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);
+}
+
+// a / b with b scaled by a power of two, so that |b|^2 neither overflows nor
+// underflows: one divide (500 cycles here) deep, where cdiv's scaling by a
+// quotient takes two
 __device__ __forceinline__ double2 cquot(double2 a, double2 b)
 {
+    const double s = pow2_of(b);
+    b = make_double2(b.x * s, b.y * s);
     const double d = b.x * b.x + b.y * b.y;
-    return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
+    return make_double2((a.x * b.x + a.y * b.y) / d * s, (a.y * b.x - a.x * b.y) / d * s);
 }
 
 // one component of cquot (c = 0 real, 1 imaginary), so that two lanes form the
@@ -214,8 +224,10 @@ __device__ __forceinline__ double2 cquot(double2 a, double2 b)
 // depend on each other
 __device__ __forceinline__ double cquot_part(double2 a, double2 b, int c)
 {
+    const double s = pow2_of(b);
+    b = make_double2(b.x * s, b.y * s);
     const double d = b.x * b.x + b.y * b.y;
-    return (c == 0 ? a.x * b.x + a.y * b.y : a.y * b.x - a.x * b.y) / d;
+    return (c == 0 ? a.x * b.x + a.y * b.y : a.y * b.x - a.x * b.y) / d * s;
 }
 
 // Barrier of all blocks of a cooperative launch on a counter that starts at 0.

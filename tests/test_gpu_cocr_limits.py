@@ -1,5 +1,5 @@
 """The FP64 solver where it runs out of something: iterations, when it stops
-on the true residual."""
+on the true residual; range, where the squares of its sums pass FP64's."""
 import pytest
 
 from mtcalc_with_dfp_cocr_gb300 import assembly
@@ -35,5 +35,30 @@ def test_true_residual_with_few_iterations(gpu, cells, eps):
                 assert (code, it, res) == (0, last[1], last[2]) and torch.equal(x, last[3])
             else:
                 assert code == -3 and it == maxiter + 1 and res >= eps
+    cx.close()
+    A.close()
+
+
+@pytest.mark.parametrize("cells", [(14, 13, 12), (33, 31, 32), (42, 42, 43)])
+@pytest.mark.parametrize("e", [-60, 300, 450])
+def test_right_hand_sides_of_any_size(gpu, cells, e):
+    """Every operation scales exactly with the right-hand side: b 2^e gives x
+    2^e, also where (a, w) and (z, s) are beyond 1e154 and their squares
+    beyond FP64's range.  Small ones end in the reference's breakdown test,
+    (a, w) < 1e-40, whose bound does not scale."""
+    torch = gpu
+    m, nus, b = _ragged(torch, cells, 1, 2)
+    A = assembly.Assembly(m)
+    cx = A.cocr(nus[0])
+    out = []
+    for scale in (1.0, 2.0 ** e):
+        x = torch.zeros_like(b[0])
+        code, st = cx.solve(b[0] * scale, x, eps=1e-5, maxiter=2000)
+        out.append((code, st.iterations, st.residual_rel, x / scale))
+    assert out[0][0] == 0
+    if e < 0:
+        assert out[1][0] == -2
+    else:
+        assert out[0][:3] == out[1][:3] and torch.equal(out[0][3], out[1][3])
     cx.close()
     A.close()
