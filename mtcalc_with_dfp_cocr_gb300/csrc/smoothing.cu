@@ -40,6 +40,7 @@
 #include "receivers.cuh"
 
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -224,14 +225,20 @@ k_sm_solve(SolveArgs A)
     block_sum<C>(ff, dbuf[flip]);
     flip ^= 1;
 #pragma unroll
-    for (int c = 0; c < C; c++) rr[c] = ff[c];
+    for (int c = 0; c < C; c++) {
+        rr[c] = ff[c];
+        // no projection of an infinity or a NaN (or of squares beyond FP64): the
+        // column is done at once, and not with x = 0
+        if (c < nc && !(ff[c] <= DBL_MAX))
+            for (int n = tid; n < nn; n += kSolve) x[c][n] = nan("");
+    }
     bool done[C];
     int open = 0;
     for (int round = 0; round < kMaxOuter; round++) {
         open = 0;
 #pragma unroll
         for (int c = 0; c < C; c++) {
-            // (a NaN ends its column, as does a zero right-hand side)
+            // (an infinity or a NaN ends its column, as does a zero right-hand side)
             done[c] = c >= nc || !(rr[c] > kTol2 * ff[c]) ||
                       (round > 0 && rr[c] > 0.25 * last[c] && rr[c] <= kFloor2 * ff[c]);
             open += !done[c];
