@@ -327,7 +327,8 @@ __device__ __forceinline__ cdf cmul(const cfac &a, cdf y)
 // ---- sums across threads
 // A partial sum as three FP32 numbers a + b + c.  Adding two of them with
 // two-sums on a and b keeps more than 60 bits (the error is that of c, about
-// 2^-70 of the larger operand), more than FP64's 53, in 21 FP32 operations:
+// 2^-70 of the larger operand; below 2^-89 c leaves FP32's range and it is
+// 2^-149), more than FP64's 53, in 21 FP32 operations:
 // GB300 issues an FP64 add of a warp once in 16 cycles, so the FP64 trees
 // over 256 threads that these sums replace took most of a small kernel.
 // FP32's range is the limit of a and not FP64's: sums that could overflow are
@@ -356,14 +357,22 @@ __device__ __forceinline__ tf tf_diff(const acc2 &x)
 {
     return tf_add(tf_of(lane0(cdf{x.h, x.l})), tf_neg(tf_of(lane1(cdf{x.h, x.l}))));
 }
-__device__ __forceinline__ tf tf_of(double v)
-{
-    const float a = (float)v;
-    const double r = v - (double)a;
-    const float b = (float)r;
-    return tf{a, b, (float)(r - (double)b)};
-}
 constexpr float kTfBig = 0x1p100f, kTfDown = 0x1p-64f;
+// FP64 sums as three FP32 numbers each; true where they are scaled by 2^-64
+// to stay in FP32's range (up to 2^192)
+__device__ __forceinline__ bool tf_of(const double (&d)[2], tf (&v)[2])
+{
+    const bool down = fmax(fabs(d[0]), fabs(d[1])) >= kTfBig;
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+        const double s = down ? d[n] * kTfDown : d[n];
+        const float a = (float)s;
+        const double r = s - (double)a;
+        const float b = (float)r;
+        v[n] = tf{a, b, (float)(r - (double)b)};
+    }
+    return down;
+}
 __device__ __forceinline__ float4 tf_pack(tf x, float w) { return make_float4(x.a, x.b, x.c, w); }
 __device__ __forceinline__ float4 tf4_add(float4 x, float4 y)
 {

@@ -364,6 +364,7 @@ k_mf_tile(MF M, MfTileGrid G, const float2 *__restrict__ omega, const float4 *__
             for (int n = 0; n < 2; n++)
                 for (int t = u * CPS; t < (u + 1) * CPS; t++) d[n] += red[n * NT + t];
     }
-    const tf v[2] = {tf_of(d[0]), tf_of(d[1])};
-    SpmvTail::finish_v<SP, NT>(v, sys, partials, mode);
+    tf v[2];
+    const bool down = tf_of(d, v);
+    SpmvTail::finish_v<SP, NT>(v, sys, partials, mode, down);
 }

@@ -201,6 +201,7 @@ k_prec_tile(MF M, PrecGrid G, const float4 *__restrict__ ds, const float4 *__res
                 d[1] += red[NT + t];
             }
     }
-    const tf v[2] = {tf_of(d[0]), tf_of(d[1])};
-    finish_alpha<SP, NT>(v, sys, partials, first);
+    tf v[2];
+    const bool down = tf_of(d, v);
+    finish_alpha<SP, NT>(v, sys, partials, first, down);
 }

@@ -79,17 +79,18 @@ struct GridSum {
     }
     // the block's totals in threads t < W: a warp halves the number of values
     // per lane while it halves the lanes per value (N + log2 adds instead of
-    // N log2), then thread t < W adds the warps' sums
-    static __device__ __forceinline__ float4 block(const tf (&v)[N], float4 *sm)
+    // N log2), then thread t < W adds the warps' sums.  down: this thread's
+    // values are scaled by 2^-64 already
+    static __device__ __forceinline__ float4 block(const tf (&v)[N], float4 *sm, bool down)
     {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        bool big = false;
+        bool big = down;
 #pragma unroll
         for (int n = 0; n < N; n++) big |= fabsf(v[n].a) >= kTfBig;
         big = __any_sync(0xffffffffu, big);
         tf u[N];
 #pragma unroll
-        for (int n = 0; n < N; n++) u[n] = big ? tf_scale(v[n], kTfDown) : v[n];
+        for (int n = 0; n < N; n++) u[n] = big && !down ? tf_scale(v[n], kTfDown) : v[n];
         int cnt = N, first = 0, dup = 0;
 #pragma unroll
         for (int o = 16; o >= SP; o >>= 1) {
@@ -167,7 +168,7 @@ inline size_t partial_slots(int blocks, int SP)
 // Per-system sums over the grid: true in the block that finishes last, with
 // the totals in tot[n][k].
 template <int SP, int N, int NT = kB>
-__device__ bool sys_grid_sum(const tf (&v)[N], float4 *partials, double (*tot)[32])
+__device__ bool sys_grid_sum(const tf (&v)[N], float4 *partials, double (*tot)[32], bool down = false)
 {
     using S = GridSum<SP, N, NT>;
     constexpr int W = S::W;
@@ -175,7 +176,7 @@ __device__ bool sys_grid_sum(const tf (&v)[N], float4 *partials, double (*tot)[3
     __shared__ bool last;
     unsigned int *tickets = reinterpret_cast<unsigned int *>(partials);
     float4 *part = partials + kTicketSlots;
-    float4 s = S::block(v, sm);
+    float4 s = S::block(v, sm, down);
     // one level: this block's sums to dst; whether it is the last of n blocks
     auto arrive = [&](float4 *dst, unsigned int *ticket, unsigned int n) {
         if (threadIdx.x < W) __stcg(dst + threadIdx.x, s);
@@ -484,13 +485,14 @@ k_init(int nb, const float4 *__restrict__ r, float4 *__restrict__ sm, SysState *
 // behind the sum's, and independent FP64 chains (a divide or a square root is
 // 500 cycles) run side by side.
 template <int SP, int NT>
-__device__ __forceinline__ void finish_alpha(const tf (&v)[2], SysState *sys, float4 *partials, int first)
+__device__ __forceinline__ void finish_alpha(const tf (&v)[2], SysState *sys, float4 *partials, int first,
+                                             bool down = false)
 {
     __shared__ double tot[2][32];
     SysState &q = sys[threadIdx.x % SP];
     const double2 zs = q.zs;
     const int status = q.status;
-    if (sys_grid_sum<SP, 2, NT>(v, partials, tot) && threadIdx.x < SP) {
+    if (sys_grid_sum<SP, 2, NT>(v, partials, tot, down) && threadIdx.x < SP) {
         if (first) q.cnt = 0;
         if (status == kRun) {
             const double2 aw = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
@@ -706,14 +708,14 @@ struct SpmvTail {
     // res2_next), then beta; mode 0 (set-up): (z, s) only
     template <int SP, int NT = kB>
     static __device__ __forceinline__ void finish_v(const tf (&v)[2], SysState *sys,
-                                                    float4 *partials, int mode)
+                                                    float4 *partials, int mode, bool down = false)
     {
         __shared__ double tot[2][32];
         SysState &q = sys[threadIdx.x % SP];
         const double2 zs = q.zs;
         const double r_old = q.r_old, eps_k = q.eps_k, res2 = q.res2_next, res = q.residual;
         const int status = q.status, mrs = q.mrs_mode, iter = q.iter, maxiter = q.maxiter;
-        if (sys_grid_sum<SP, 2, NT>(v, partials, tot) && threadIdx.x < SP && status == kRun) {
+        if (sys_grid_sum<SP, 2, NT>(v, partials, tot, down) && threadIdx.x < SP && status == kRun) {
             const double2 zs_new = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
             q.zs = zs_new;
             if (mode == 0) return;

@@ -198,3 +198,35 @@ def test_one_kernel_iterations_from_two_threads(gpu):
     for A, sv, *_ in probs:
         sv.close()
         A.close()
+
+
+@pytest.mark.parametrize("unit,S,e", [(1e4, 2, 57), (1e4, 4, 57), (1e6, 2, 54), (1e6, 4, 54)])
+@pytest.mark.parametrize("form", ["32", "34", "fused preconditioner"])
+def test_block_sums_beyond_fp32_range(gpu, monkeypatch, form, unit, S, e):
+    """The forms that add a block's threads in FP64 pass the sum on in FP32
+    numbers: at these sizes (length unit, right-hand side 2^e) it is beyond
+    2^128 while each thread's is not, and the solutions still scale exactly."""
+    torch = gpu
+    rng = np.random.default_rng(5)
+    cells = (20, 19, 24)
+    x, y = unit * _lines(rng, cells[0], -300.0), unit * _lines(rng, cells[1], -500.0)
+    z = _lines(rng, cells[2], 0.0)
+    z = unit * (z - z[cells[2] - 1])
+    m = layered_model(x, y, z, [Layer(0.0, 0.01 / unit ** 2)],
+                      cell_sigma=10.0 ** rng.uniform(-3, 0, int(np.prod(cells))) / unit ** 2)
+    nus = list(10.0 ** rng.uniform(0, 2, S))
+    b = torch.from_numpy(rng.standard_normal((S, 2 * m.nb))).cuda()
+    monkeypatch.setenv("MTGPU_PREC_TILE", "1" if form == "fused preconditioner" else "0")
+    A = assembly.Assembly(m)
+    sv = survey.Survey(A, nus)
+    sv.set_spmv_variant(34 if form == "34" else 32)
+    assert sv.preconditioner()[0] == (form == "fused preconditioner")
+    out = []
+    for scale in (1.0, 2.0 ** e):
+        u = torch.zeros_like(b)
+        code, st = sv.solve(b * scale, u, eps=1e-4, maxiter=300, verify=False)
+        assert code == 0 and st["fp64_iterations"] == [0] * S
+        out.append((st["iterations"], u / scale))
+    assert out[0][0] == out[1][0] and torch.equal(out[0][1], out[1][1])
+    sv.close()
+    A.close()
