@@ -1337,11 +1337,11 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
     if (pin_env >= 0 && spmv_variant_available(V, pin_env)) {
         V.ch = pin_env;
         MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
+    } else if (g_form()) {
+        // (its grids are set)
     } else if (pin_variant >= 0 && spmv_variant_available(V, pin_variant)) {
         V.ch = pin_variant;
         MTGPU_SP_DISPATCH(V.SP, grids(V, nsm));
-    } else if (g_form()) {
-        // (its grids are set)
     } else {
         // with the matrix-free operator the stored-matrix variants and the
         // tiled matrix-free one measured slower on every tensor mesh (whole

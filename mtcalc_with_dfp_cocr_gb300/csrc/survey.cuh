@@ -169,8 +169,9 @@ struct MatFreeMesh {
 // a: the assembly (host mesh copies) when the survey is built from one, or
 // mfm: the mesh of a host SLAE; on a tensor mesh either enables the
 // matrix-free SpMV variant
-// pin_variant >= 0 (and available): that SpMV variant instead of the
-// set-up autotuning
+// pin_variant >= 0 (and available): that SpMV variant where the set-up would
+// time the variants (not where its rule names one: the rule depends on the
+// batch, a kept choice does not)
 int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const double *omega,
                  Survey &V, cudaStream_t st, const mtgpu_assembly_s *a = nullptr,
                  const MatFreeMesh *mfm = nullptr, int pin_variant = -1);
