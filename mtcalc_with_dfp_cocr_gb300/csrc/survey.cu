@@ -240,11 +240,15 @@ k_tile_cols(int nslices, int T, const long long *pc, const long long *pr, const 
     }
 }
 
-// System-major [S][nb] FP64 <-> row-major [nb][SP], FP64 or double-float.  A
-// block moves 32 rows of all systems through shared memory, so that both
-// sides are read and written in whole lines: element by element in the
-// row-major order, a warp of 32 systems touched 32 lines of the system-major
-// side for 16 bytes of each (32 systems x 610k rows: 283 -> 150 us in, 345 -> 150 us out).
+// System-major [S][nb] FP64 <-> row-major [nb][SP], FP64 or double-float.
+// With more than kFewLanes lanes a block moves 32 rows of all systems through
+// shared memory, so that both sides are read and written in whole lines:
+// element by element in the row-major order, a warp of 32 systems touched 32
+// lines of the system-major side for 16 bytes of each (32 systems x 610k rows:
+// 283 -> 150 us in, 345 -> 150 us out).  With few lanes a warp's elements are whole
+// lines on both sides as they are, and a block of 32 rows leaves most of its
+// threads idle: a product with both transposes on 1.8M rows took 190 us that way
+// against 129 at 1 lane, 247 against 204 at 2, 390 against 374 at 4; 704 both at 8.
 constexpr int kTRows = 32;
 __device__ __forceinline__ void row_store(double2 *p, double2 v) { *p = v; }
 __device__ __forceinline__ void row_store(float4 *p, double2 v) { *p = to4(from_d2(v)); }
@@ -279,6 +283,47 @@ k_from_rows(int nb, int S, int SP, const T *__restrict__ src, double2 *__restric
     __syncthreads();
     if (r0 + l < nb)
         for (int k = threadIdx.x / kTRows; k < S; k += kB / kTRows) dst[(long long)k * nb + r0 + l] = t[k][l];
+}
+
+// element by element in the row-major order; SP = 1 << lg
+template <class T>
+__global__ void __launch_bounds__(kB)
+k_to_rows_few(int nb, int S, int lg, const double2 *__restrict__ src, T *__restrict__ dst)
+{
+    const long long i = (long long)blockIdx.x * kB + threadIdx.x, row = i >> lg;
+    const int k = (int)i & ((1 << lg) - 1);
+    if (row < nb) row_store(dst + i, k < S ? src[(long long)k * nb + row] : make_double2(0.0, 0.0));
+}
+
+template <class T>
+__global__ void __launch_bounds__(kB)
+k_from_rows_few(int nb, int S, int lg, const T *__restrict__ src, double2 *__restrict__ dst)
+{
+    const long long i = (long long)blockIdx.x * kB + threadIdx.x, row = i >> lg;
+    const int k = (int)i & ((1 << lg) - 1);
+    if (row < nb && k < S) dst[(long long)k * nb + row] = row_load(src + i);
+}
+
+constexpr int kFewLanes = 4;
+template <class T>
+void to_rows(const Survey &V, const double2 *src, T *dst)
+{
+    const int lg = __builtin_ctz(V.SP);
+    if (V.SP <= kFewLanes)
+        k_to_rows_few<<<(unsigned)((((long long)V.nb << lg) + kB - 1) / kB), kB, 0, V.st>>>(V.nb, V.S, lg, src, dst);
+    else
+        k_to_rows<<<(unsigned)ceil_div(V.nb, kTRows), kB, 0, V.st>>>(V.nb, V.S, V.SP, src, dst);
+    note_launches(1);
+}
+template <class T>
+void from_rows(const Survey &V, const T *src, double2 *dst)
+{
+    const int lg = __builtin_ctz(V.SP);
+    if (V.SP <= kFewLanes)
+        k_from_rows_few<<<(unsigned)((((long long)V.nb << lg) + kB - 1) / kB), kB, 0, V.st>>>(V.nb, V.S, lg, src, dst);
+    else
+        k_from_rows<<<(unsigned)ceil_div(V.nb, kTRows), kB, 0, V.st>>>(V.nb, V.S, V.SP, src, dst);
+    note_launches(1);
 }
 
 // ------------------------------------------------------- conversions
@@ -1487,11 +1532,9 @@ int survey_spmv(Survey &V, const double2 *x_sys_major, double2 *y_sys_major)
         init[k] = s;
     }
     MTGPU_TRY(cudaMemcpyAsync(V.sys, init.data(), sizeof(SysState) * 32, cudaMemcpyHostToDevice, V.st));
-    const unsigned gt = (unsigned)ceil_div(V.nb, kTRows);
-    k_to_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, x_sys_major, V.s);
+    to_rows(V, x_sys_major, V.s);
     MTGPU_SP_DISPATCH(V.SP, spmv_only(V, 0));
-    k_from_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, V.z, y_sys_major);
-    note_launches(2);
+    from_rows(V, V.z, y_sys_major);
     MTGPU_TRY(cudaGetLastError());
     MTGPU_TRY(cudaStreamSynchronize(V.st));
     return MTGPU_OK;
@@ -1548,7 +1591,6 @@ void SurveyRun::release()
 int survey_begin(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, double eps,
                  int maxiter, int verify, int iters_per_launch, SurveyRun &R)
 {
-    const unsigned gt = (unsigned)ceil_div(V.nb, kTRows);
     R = SurveyRun{};
     R.x_out = x_sys_major;
     R.eps = eps;
@@ -1572,9 +1614,8 @@ int survey_begin(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, do
     // (the ticket slots: a launch that gave up leaves its counters behind)
     MTGPU_TRY(cudaMemsetAsync(V.partials, 0, sizeof(float4) * kTicketSlots, V.st));
     if ((rc = upload_sys(V))) return rc;
-    k_to_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, b_sys_major, V.b64);
-    k_to_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, x_sys_major, V.xacc);
-    note_launches(2);
+    to_rows(V, b_sys_major, V.b64);
+    to_rows(V, x_sys_major, V.xacc);
     if ((rc = dev_alloc(&R.d_flag, 32))) return rc;
     // inner right-hand side r0 = b - A x0 (FP64), threshold relative to ||b||
     for (int k = 0; k < 32; k++) R.flag[k] = k < V.S;
@@ -1711,7 +1752,6 @@ int survey_collect(Survey &V, SurveyRun &R)
 
 int survey_finish(Survey &V, SurveyRun &R, mtgpu_survey_stats *stats, int stat_offset)
 {
-    const unsigned gt = (unsigned)ceil_div(V.nb, kTRows);
     int rc;
     // true residual of the systems that ended without a check
     bool any = false;
@@ -1724,8 +1764,7 @@ int survey_finish(Survey &V, SurveyRun &R, mtgpu_survey_stats *stats, int stat_o
         MTGPU_SP_DISPATCH(V.SP, res64(V, R.d_flag, 0));
         if ((rc = sync_sys(V))) return rc;
     }
-    k_from_rows<<<gt, kB, 0, V.st>>>(V.nb, V.S, V.SP, V.xacc, R.x_out);
-    note_launches(1);
+    from_rows(V, V.xacc, R.x_out);
     MTGPU_TRY(cudaGetLastError());
     MTGPU_TRY(cudaStreamSynchronize(V.st));
     int worst = MTGPU_OK;
