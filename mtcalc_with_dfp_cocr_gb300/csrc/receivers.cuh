@@ -42,6 +42,7 @@ struct Smoothing {
     double *d_val = nullptr, *d_x = nullptr, *d_r = nullptr, *d_f = nullptr;
     float *d_w = nullptr;                             // FP32 vectors of the projection
     int *d_out = nullptr;
+    int clusters[9] = {};                             // [q]: clusters of q blocks that run side by side
     int iterations = 0;
     void release();
 };

@@ -25,9 +25,11 @@
 // 1e-14 of the right-hand side: three to four rounds.  One block holds one
 // subdomain and two or four columns from the right-hand side to the solution:
 // no launches between iterations, and the matrix, read from L2, serves all of
-// its columns.  (CG in FP64, four launches an iteration, took 5.9 ms for 96
-// columns of 6,600 nodes; GB300 runs FP64 at 1/64 of FP32, and 27
-// multiply-adds a node, column and iteration are 27 us of its FP64 pipes.)
+// its columns; where few columns leave SMs idle, a cluster of up to eight
+// blocks shares the subdomain's nodes.  (CG in FP64, four launches an
+// iteration, took 5.9 ms for 96 columns of 6,600 nodes; GB300 runs FP64 at 1/64
+// of FP32, and 27 multiply-adds a node, column and iteration are 27 us of its
+// FP64 pipes.)
 // The subdomains, the mass matrix and the interpolation weights are built
 // once per receiver set on the host; the per-call work (centre values,
 // right-hand sides, projection, interpolation) runs on the device.
@@ -123,10 +125,35 @@ __device__ __forceinline__ vec<C> quot(vec<C> x, vec<C> y)
     return x;
 }
 
+// Q blocks that share a subdomain are a cluster (CL): barriers of all its
+// threads, after which each sees what the others stored before theirs, and
+// stores into the other blocks' shared memory.
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_addr(const void *own, int rank)
+{
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(own)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cluster_store(unsigned a, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_store(unsigned a, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+constexpr int kMaxCluster = 8;
+
 // Sums of C values per thread over the block, in a fixed order, to all
-// threads; buf: [warps] slots, alternated by the caller between calls.
-template <int C, class T>
-__device__ __forceinline__ void block_sum(T (&v)[C], T (*buf)[C])
+// threads; buf: [warps] slots, alternated by the caller between calls.  Of a
+// cluster, block `rank` of Q then gives its sums to all blocks (all: [block]
+// slots, alternated likewise), and every thread adds them in block order.
+template <int C, bool CL, class T>
+__device__ __forceinline__ void block_sum(T (&v)[C], T (*buf)[C], T (*all)[C], int Q, int rank)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     // halve the values a lane holds while lane bits are left to pick them,
@@ -154,6 +181,19 @@ __device__ __forceinline__ void block_sum(T (&v)[C], T (*buf)[C])
         for (int q = 1; q < kSolve / 32; q++) s += buf[q][c];
         v[c] = s;
     }
+    if (CL) {
+        if (threadIdx.x < Q) {
+            const unsigned a = cluster_addr(all[rank], threadIdx.x);
+#pragma unroll
+            for (int c = 0; c < C; c++) cluster_store(a + c * (unsigned)sizeof(T), v[c]);
+        }
+        cluster_barrier();
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            v[c] = 0;
+            for (int q = 0; q < Q; q++) v[c] += all[q][c];
+        }
+    }
 }
 
 struct SolveArgs {
@@ -170,11 +210,13 @@ struct SolveArgs {
     double *x, *f, *r;                       // [column][padded node]
     float *w;                                // FP32 vectors, 4 x [group][padded node][C]
     int pcap;                                // bytes of shared memory for p
+    int q;                                   // blocks a subdomain (a cluster)
     int *out;                                // columns that did not converge; largest iteration count
 };
 
-// the projection of C columns (blockIdx.x) of one subdomain (blockIdx.y)
-template <int C>
+// the projection of C columns of one subdomain (blockIdx.y); CL: by a cluster of
+// A.q blocks, each a range of the nodes, with p in global memory
+template <int C, bool CL>
 __global__ void __launch_bounds__(kSolve, 1)
 k_sm_solve(SolveArgs A)
 {
@@ -182,11 +224,17 @@ k_sm_solve(SolveArgs A)
     extern __shared__ __align__(16) unsigned char psh[];
     __shared__ double dbuf[2][kSolve / 32][C];
     __shared__ float fbuf[2][kSolve / 32][C];
-    const int sub = blockIdx.y, n0 = A.off[sub], nn = A.nn[sub], tid = threadIdx.x;
-    const int c0 = C * blockIdx.x, nc = min(C, A.ncol - c0);
-    const long long nw = (long long)gridDim.x * A.npad;
-    V *const w = reinterpret_cast<V *>(A.w) + (long long)blockIdx.x * A.npad + n0;
-    V *const p = nn * (int)sizeof(V) <= A.pcap ? reinterpret_cast<V *>(psh) : w;
+    __shared__ double dall[2][CL ? kMaxCluster : 1][C];
+    __shared__ float fall[2][CL ? kMaxCluster : 1][C];
+    const int Q = CL ? A.q : 1, rank = CL ? blockIdx.x % Q : 0, group = CL ? blockIdx.x / Q : blockIdx.x;
+    const int sub = blockIdx.y, n0 = A.off[sub], nn = A.nn[sub];
+    // this block's nodes
+    const int share = CL ? (nn + 32 * Q - 1) / (32 * Q) * 32 : nn;
+    const int first = share * rank + threadIdx.x, end = min(nn, share * (rank + 1));
+    const int c0 = C * group, nc = min(C, A.ncol - c0);
+    const long long nw = (long long)(gridDim.x / Q) * A.npad;
+    V *const w = reinterpret_cast<V *>(A.w) + (long long)group * A.npad + n0;
+    V *const p = !CL && nn * (int)sizeof(V) <= A.pcap ? reinterpret_cast<V *>(psh) : w;
     V *const r32 = w + nw, *const d32 = w + 2 * nw, *const q32 = w + 3 * nw;
     const float *const dinv = A.dinv + n0;
     const int2 *const m32 = A.m32 + (long long)n0 * kSlots;
@@ -201,14 +249,19 @@ k_sm_solve(SolveArgs A)
         r[c] = A.r + o;
     }
     int flip = 0, total = 0;
+    auto everyone = [&] {
+        if (CL) cluster_barrier();
+        else __syncthreads();
+    };
     auto sum = [&](V v) {
-        block_sum<C>(v.a, fbuf[flip]);
+        block_sum<C, CL>(v.a, fbuf[flip], fall[flip], Q, rank);
         flip ^= 1;
         return v;
     };
+    if (CL) cluster_barrier();               // the other blocks have started
     // f = sum over the node's bricks of g_c val_c; x = 0, so r = f
     double ff[C] = {}, rr[C], last[C] = {};
-    for (int n = tid; n < nn; n += kSolve)
+    for (int n = first; n < end; n += kSolve)
         for (int c = 0; c < nc; c++) {
             double s = 0.0;
             for (int j = A.nc_ptr[n0 + n]; j < A.nc_ptr[n0 + n + 1]; j++) {
@@ -222,7 +275,7 @@ k_sm_solve(SolveArgs A)
             for (int q = 0; q < C; q++)
                 if (q == c) ff[q] += s * s;
         }
-    block_sum<C>(ff, dbuf[flip]);
+    block_sum<C, CL>(ff, dbuf[flip], dall[flip], Q, rank);
     flip ^= 1;
 #pragma unroll
     for (int c = 0; c < C; c++) {
@@ -230,7 +283,7 @@ k_sm_solve(SolveArgs A)
         // no projection of an infinity or a NaN (or of squares beyond FP64): the
         // column is done at once, and not with x = 0
         if (c < nc && !(ff[c] <= DBL_MAX))
-            for (int n = tid; n < nn; n += kSolve) x[c][n] = nan("");
+            for (int n = first; n < end; n += kSolve) x[c][n] = nan("");
     }
     bool done[C];
     int open = 0;
@@ -253,7 +306,7 @@ k_sm_solve(SolveArgs A)
             scale[c] = norm[c] > 0.0 ? 1.0 / norm[c] : 0.0;
         }
         V rz = splat<C>(0.f);
-        for (int n = tid; n < nn; n += kSolve) {
+        for (int n = first; n < end; n += kSolve) {
             V v;
 #pragma unroll
             for (int c = 0; c < C; c++) v.a[c] = done[c] ? 0.f : (float)(r[c][n] * scale[c]);
@@ -266,7 +319,7 @@ k_sm_solve(SolveArgs A)
         rz = sum(rz);
         for (int it = 0; it < kMaxInner; it++) {
             V pq = splat<C>(0.f);
-            for (int n = tid; n < nn; n += kSolve) {
+            for (int n = first; n < end; n += kSolve) {
                 V s = splat<C>(0.f);
                 const int2 *m = m32 + slots(n);
 #pragma unroll 9
@@ -281,7 +334,7 @@ k_sm_solve(SolveArgs A)
             total++;
             const V al = quot(rz, pq), nal = al * splat<C>(-1.f);
             V rz2 = splat<C>(0.f), r2 = rz2;
-            for (int n = tid; n < nn; n += kSolve) {
+            for (int n = first; n < end; n += kSolve) {
                 d32[n] = fma_(al, p[n], d32[n]);
                 const V v = fma_(nal, q32[n], r32[n]);
                 r32[n] = v;
@@ -296,19 +349,19 @@ k_sm_solve(SolveArgs A)
             rz2 = sum(rz2);
             const V be = quot(rz2, rz);
             rz = rz2;
-            for (int n = tid; n < nn; n += kSolve) p[n] = fma_(be, p[n], r32[n] * splat<C>(dinv[n]));
-            __syncthreads();
+            for (int n = first; n < end; n += kSolve) p[n] = fma_(be, p[n], r32[n] * splat<C>(dinv[n]));
+            everyone();
         }
         // x += |r| d, r = f - M x in FP64
-        for (int n = tid; n < nn; n += kSolve) {
+        for (int n = first; n < end; n += kSolve) {
             const V d = d32[n];
 #pragma unroll
             for (int c = 0; c < C; c++)
                 if (!done[c]) x[c][n] += norm[c] * (double)d.a[c];
         }
-        __syncthreads();
+        everyone();
         double s2[C] = {};
-        for (int n = tid; n < nn; n += kSolve) {
+        for (int n = first; n < end; n += kSolve) {
             double s[C];
 #pragma unroll
             for (int c = 0; c < C; c++) s[c] = done[c] ? 0.0 : f[c][n];
@@ -328,13 +381,13 @@ k_sm_solve(SolveArgs A)
                     s2[c] += s[c] * s[c];
                 }
         }
-        block_sum<C>(s2, dbuf[flip]);
+        block_sum<C, CL>(s2, dbuf[flip], dall[flip], Q, rank);
         flip ^= 1;
 #pragma unroll
         for (int c = 0; c < C; c++)
             if (!done[c]) rr[c] = s2[c];
     }
-    if (tid == 0) {
+    if (rank == 0 && threadIdx.x == 0) {
         if (open > 0) atomicAdd(A.out, open);
         atomicMax(A.out + 1, total);
     }
@@ -375,6 +428,31 @@ __global__ void k_sm_receivers(int nrec, int S, int npad, const int *__restrict_
 }
 
 // ------------------------------------------------------------- host set-up
+// Blocks a subdomain: where the groups of columns leave SMs without a block, 2, 4
+// or 8 (a portable cluster), as many as run side by side (76 clusters of 2, 36 of
+// 4, 15 of 8 here) and with at least this many nodes each.  The GPU's time at
+// 1, 2, 4, 8 blocks: 59,904 nodes, one system 26.4 / 12.3 / 6.6 / 3.7 ms, eight 31.3 / 14.7
+// (and 8.4 in two waves of 4); 8,112 nodes, one 3.0 / 2.0 / 1.3 / 0.94, with four
+// systems 3.0 / 2.0 / 1.3 and 1.6 beyond what fits; 3,072 nodes 1.23 / 1.11 / 0.84 / 0.69; 343
+// nodes 0.39 / 0.61 / 0.62 / 0.63.  (Conjugate gradients in FP64 over the whole grid: 7.8 ms for one
+// system on 59,904 nodes, 13.4 for two, 47.7 for eight.)
+constexpr int kClusterNodes = 1024;
+
+// launch of the projection by clusters of q blocks
+cudaLaunchConfig_t cluster_config(cudaLaunchAttribute *at, int q, int groups, int nsub)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(groups * q, nsub);
+    cfg.blockDim = kSolve;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = q;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 struct SubBuild {
     std::vector<int> cells, nodes;   // ascending global indices
 };
@@ -632,6 +710,16 @@ int smoothing_build(Smoothing &sm, const ::mtgpu_assembly_s &a, int nrec, const 
         (rc = dev_alloc(&sm.d_out, 2)))
         return rc;
     MTGPU_TRY(cudaStreamSynchronize(st));   // the host vectors go out of scope
+    // clusters of q blocks that run side by side
+    for (int q = 2; q <= kMaxCluster; q *= 2) {
+        cudaLaunchAttribute at[1];
+        cudaLaunchConfig_t cfg = cluster_config(at, q, 1, 1);
+        sm.clusters[q] = 0;
+        if (cudaOccupancyMaxActiveClusters(&sm.clusters[q], k_sm_solve<2, true>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            sm.clusters[q] = 0;
+        }
+    }
     return MTGPU_OK;
 }
 
@@ -672,15 +760,25 @@ int smoothing_fields(Smoothing &sm, const ParamMatrix &P, int nrec, int S, long 
         constexpr int kSmem = 200 * 1024;
         int widest = 0;
         for (int n : sm.sub_nodes) widest = std::max(widest, n);
-        const int smem = (int)std::min<long long>(kSmem, (long long)widest * 4 * C);
+        int q = 1;
+        if (C == 2)
+            while (q < kMaxCluster && widest >= kClusterNodes * 2 * q && groups * sm.nsub <= sm.clusters[2 * q]) q *= 2;
+        const int smem = q > 1 ? 0 : (int)std::min<long long>(kSmem, (long long)widest * 4 * C);
         const SolveArgs A{sm.npad, ncol, sm.ncell, sm.d_off, sm.d_nn, sm.d_nc_ptr, sm.d_nc, sm.d_cell_g,
                           sm.d_val, sm.d_m32, sm.d_m64, sm.d_dinv, sm.d_x, sm.d_f, sm.d_r, sm.d_w, smem,
-                          sm.d_out};
+                          q, sm.d_out};
         MTGPU_TRY(cudaMemsetAsync(sm.d_out, 0, 2 * sizeof(int), st));
-        const void *solve = C == 4 ? (const void *)k_sm_solve<4> : (const void *)k_sm_solve<2>;
-        MTGPU_TRY(cudaFuncSetAttribute(solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-        if (C == 4) k_sm_solve<4><<<dim3(groups, sm.nsub), kSolve, smem, st>>>(A);
-        else k_sm_solve<2><<<dim3(groups, sm.nsub), kSolve, smem, st>>>(A);
+        if (q > 1) {
+            cudaLaunchAttribute at[1];
+            cudaLaunchConfig_t cfg = cluster_config(at, q, groups, sm.nsub);
+            cfg.stream = st;
+            MTGPU_TRY(cudaLaunchKernelEx(&cfg, k_sm_solve<2, true>, A));
+        } else {
+            const void *solve = C == 4 ? (const void *)k_sm_solve<4, false> : (const void *)k_sm_solve<2, false>;
+            MTGPU_TRY(cudaFuncSetAttribute(solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+            if (C == 4) k_sm_solve<4, false><<<dim3(groups, sm.nsub), kSolve, smem, st>>>(A);
+            else k_sm_solve<2, false><<<dim3(groups, sm.nsub), kSolve, smem, st>>>(A);
+        }
         launches += 2;
         MTGPU_TRY(cudaGetLastError());
         int out[2] = {0, 0};
