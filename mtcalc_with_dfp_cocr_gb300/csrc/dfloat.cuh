@@ -88,13 +88,6 @@ __device__ __forceinline__ df add(df a, df b)
     return t.get();
 }
 
-__device__ __forceinline__ df mul(df a, df b)
-{
-    acc t;
-    t.mac(a, b);
-    return t.get();
-}
-
 // complex double-float; in memory a float4 (re.h, im.h, re.l, im.l), so that
 // the high and the low parts of both components are register pairs for the
 // packed operations below
@@ -345,7 +338,6 @@ __device__ __forceinline__ tf tf_add(tf x, tf y)
     return tf{s, u, __fadd_rn(__fadd_rn(x.c, y.c), __fadd_rn(f, g))};
 }
 __device__ __forceinline__ tf tf_scale(tf x, float s) { return tf{x.a * s, x.b * s, x.c * s}; }
-__device__ __forceinline__ tf tf_of(const acc &x) { return tf{x.h, x.l, 0.f}; }
 __device__ __forceinline__ tf tf_of(df x) { return tf{x.h, x.l, 0.f}; }
 __device__ __forceinline__ tf tf_neg(tf x) { return tf{-x.a, -x.b, -x.c}; }
 // the sum of both components of an accumulator, and its first minus its second

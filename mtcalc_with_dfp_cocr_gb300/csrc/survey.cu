@@ -1181,6 +1181,7 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
         (rc = dev_alloc(&V.partials, partial_slots(std::max(gmax, nsm * 32), V.SP))))
         return rc;
     V.pblocks = std::max(gmax, nsm * 32);
+    MTGPU_CHECK_ARG(ceil_div(V.pblocks, kGroupBlocks) <= kMaxGroups, "more blocks than the grid sums have tickets");
     // the s vectors of a group of iterations.  Of a survey of several batches,
     // 1 for now: the batches set up after this one need their memory first
     // (survey_lengthen_group)

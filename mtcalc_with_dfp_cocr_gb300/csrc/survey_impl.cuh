@@ -154,7 +154,9 @@ struct GridSum {
 // on one SM (456 x 32 x 4: 14 us in FP64), so the last block of every group of
 // 24 adds the group's, and the last group's adds the groups'.
 constexpr int kGroupBlocks = 24;
-constexpr int kTicketSlots = 256;     // float4 slots before the partials: up to 1023 groups
+// float4 slots before the partials: the grid's ticket, the groups', and k_small's
+// two counters (kBarSlot, kExitSlot)
+constexpr int kTicketSlots = 256, kMaxGroups = 990;
 template <int SP>
 constexpr int group_blocks()
 {
@@ -1056,7 +1058,7 @@ __device__ __forceinline__ cdf mf_circ(cdf a, cdf b, cdf c, cdf d)
 // One thread per node and system forms the x-, y- and z-normal faces at the
 // node (those that exist): 9 edge values instead of 12 (the node's own
 // three edges are shared), one position decode instead of three; each sum
-// is mf_face_f's, so f is the same to the last bit.
+// is mf_circ's, so f is the same to the last bit.
 template <int SP>
 __global__ void __launch_bounds__(kB)
 k_mf_faces(MF M, const float4 *__restrict__ x, const SysState *sys, int rev)
@@ -1377,7 +1379,7 @@ k_mf_edges(int nb, MF M, const float2 *__restrict__ omega, const float4 *__restr
 // edge's curl-curl row is then the signed sum of g over its 4 faces, 8 adds
 // instead of the 24 multiply-adds of mf_row.  g is needed only on faces
 // whose position along the normal is interior (the faces of non-Dirichlet
-// edges); the others get 0.
+// edges); no row reads the others, and nothing forms them.
 
 // g = F f straight from x, each circulation formed once (variant 35): a
 // thread owns a column of faces along their normal and a chunk of len

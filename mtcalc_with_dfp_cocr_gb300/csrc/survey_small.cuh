@@ -45,6 +45,7 @@ constexpr int kSmallSystems = 8;       // systems, at most
 constexpr int kSmallItems = 3;         // rows x systems per thread, at most
 constexpr int kSmallItemBytes = 6 * sizeof(float4) + sizeof(int4) + sizeof(unsigned);
 constexpr int kBarSlot = 992, kExitSlot = 1008;   // counters among the ticket slots
+static_assert(kMaxGroups < kBarSlot && kExitSlot < 4 * kTicketSlots, "the counters lie behind the groups' tickets");
 
 struct SmallArgs {
     int nb;
