@@ -113,7 +113,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
         late = 0;
     }
     __syncthreads();
-    GridBarrier bar{&A.ctl->bar, &A.ctl->failed, c.polls};
+    GridBarrier bar{&A.ctl->bar};
     double2 *const x = c.x;
     for (int u = 0; u < items; u++) {
         const int i = row0 + u * stride;
@@ -165,7 +165,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
             A.h[v] = cmul(make_double2(hr, hi), dsv);
         }
         bar.arrive();
-        if (!bar.wait(&late)) break;
+        if (!bar.wait(&late, &A.ctl->failed, c.polls)) break;
 
         // p = s + beta p, a = z + beta a, w = D_A a + G^T h, (a, w) (k_it_edge)
         {
@@ -207,7 +207,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
             small_block<2>(v, nw, sums, part_e);
         }
         bar.arrive();
-        if (!bar.wait(&late)) break;
+        if (!bar.wait(&late, &A.ctl->failed, c.polls)) break;
         if (warp < 2) {
             const double q = grid_total<32>(part_e, warp, lane);
             if (lane == 0) tot[warp] = q;
@@ -243,7 +243,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
             small_block<2>(v, nw, sums, part_u);
         }
         bar.arrive();
-        if (!bar.wait(&late)) break;
+        if (!bar.wait(&late, &A.ctl->failed, c.polls)) break;
 
         // z = A s, (z, s); beside it the MRS weight; then s_m and its norm (k_it_spmv)
         {
@@ -313,7 +313,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
             small_block<3>(v, nw, sums, part_r);
         }
         bar.arrive();
-        if (!bar.wait(&late)) break;
+        if (!bar.wait(&late, &A.ctl->failed, c.polls)) break;
         if (warp < 3) {
             const double q = grid_total<32>(part_r, warp, lane);
             if (lane == 0) tot[warp] = q;

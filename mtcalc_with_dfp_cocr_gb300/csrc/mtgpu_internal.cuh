@@ -200,34 +200,29 @@ void pdl(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t 
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
-// the power of two that brings the larger component of b to [1, 2) (a zero,
-// infinite or NaN b stays one)
-__device__ __forceinline__ double pow2_of(double2 b)
-{
-    const int e = max(__double2hiint(b.x) & 0x7ff00000, __double2hiint(b.y) & 0x7ff00000);
-    return __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);
-}
-
-// a / b with b scaled by a power of two, so that |b|^2 neither overflows nor
-// underflows: one divide (500 cycles here) deep, where cdiv's scaling by a
-// quotient takes two
-__device__ __forceinline__ double2 cquot(double2 a, double2 b)
-{
-    const double s = pow2_of(b);
-    b = make_double2(b.x * s, b.y * s);
-    const double d = b.x * b.x + b.y * b.y;
-    return make_double2((a.x * b.x + a.y * b.y) / d * s, (a.y * b.x - a.x * b.y) / d * s);
-}
-
-// one component of cquot (c = 0 real, 1 imaginary), so that two lanes form the
-// quotient: a divide is 500 cycles, two of a thread 1000 even where they do not
-// depend on each other
+// One component of a / b (c = 0 real, 1 imaginary): one divide (500 cycles here)
+// deep, where cdiv's scaling by a quotient takes two.  |b|^2 as it stands where
+// a and b are far inside FP64's range; else b is scaled by the power of two
+// that brings its larger component to [1, 2), which changes no bit of a
+// quotient that needs none (a zero, infinite or NaN b stays one).
 __device__ __forceinline__ double cquot_part(double2 a, double2 b, int c)
 {
-    const double s = pow2_of(b);
-    b = make_double2(b.x * s, b.y * s);
+    const int ea = max(__double2hiint(a.x) & 0x7ff00000, __double2hiint(a.y) & 0x7ff00000),
+              eb = max(__double2hiint(b.x) & 0x7ff00000, __double2hiint(b.y) & 0x7ff00000);
+    double s = 1.0;
+    if (ea > (1023 + 500) << 20 || abs(eb - (1023 << 20)) > 400 << 20) {
+        s = __hiloint2double(max(0x7fe00000 - eb, 0x00100000), 0);
+        b = make_double2(b.x * s, b.y * s);
+    }
     const double d = b.x * b.x + b.y * b.y;
-    return (c == 0 ? a.x * b.x + a.y * b.y : a.y * b.x - a.x * b.y) / d * s;
+    const double q = (c == 0 ? a.x * b.x + a.y * b.y : a.y * b.x - a.x * b.y) / d;
+    return s == 1.0 ? q : q * s;
+}
+// both components, their divides side by side (two lanes with one each take
+// 500 cycles, one lane with both 1000)
+__device__ __forceinline__ double2 cquot(double2 a, double2 b)
+{
+    return make_double2(cquot_part(a, b, 0), cquot_part(a, b, 1));
 }
 
 // Barrier of all blocks of a cooperative launch on a counter that starts at 0.
@@ -243,8 +238,6 @@ __device__ __forceinline__ double cquot_part(double2 a, double2 b, int c)
 constexpr int kBarPolls = 1 << 22;     // about 2 s
 struct GridBarrier {
     unsigned int *ctr;
-    int *failed;                       // the mark, in device memory
-    int polls;                         // ... after this many (0: kBarPolls)
     unsigned int target = 0;
     __device__ __forceinline__ void arrive()
     {
@@ -252,18 +245,18 @@ struct GridBarrier {
         target += gridDim.x;
         if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
     }
-    // false: the other blocks did not arrive in time
-    __device__ __forceinline__ bool wait(int *late)
+    // false: the other blocks did not arrive in `polls` polls, and *failed, the
+    // mark in device memory, is set
+    __device__ __forceinline__ bool wait(int *late, int *failed, int polls)
     {
         if (threadIdx.x == 0) {
             unsigned int v = 0;
-            const int n = polls > 0 ? polls : kBarPolls;
             int q = 0;
-            for (; q < n; q++) {
+            for (; q < polls; q++) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
                 if ((int)(v - target) >= 0) break;
             }
-            if (q == n) {
+            if (q == polls) {
                 *late = 1;
                 *(volatile int *)failed = 1;
             }
@@ -272,12 +265,15 @@ struct GridBarrier {
         return *late == 0;
     }
 };
-// MTGPU_BARRIER_POLLS (environment) lowers the bound of the waits, so that a
-// test makes one run out
+// MTGPU_BARRIER_POLLS (environment) makes a wait run out in a test: it lowers
+// the bound of the FP64 solver's waits, and leaves a survey's counter one short
+// (there the bound is a constant: the loop without one costs up to 2 % of an
+// iteration)
 inline int barrier_polls()
 {
     const char *e = getenv("MTGPU_BARRIER_POLLS");
-    return e ? std::max(0, atoi(e)) : 0;
+    const int n = e ? atoi(e) : 0;
+    return n > 0 ? n : kBarPolls;
 }
 // the total of output o of the blocks' partials part[output][block], from G
 // lanes of a warp (j: the lane among them), in all of them; 8 loads in flight

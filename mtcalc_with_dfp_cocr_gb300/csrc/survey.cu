@@ -1610,10 +1610,11 @@ int survey_begin(Survey &V, const double2 *b_sys_major, double2 *x_sys_major, do
         V.hsys[k] = s;
     }
     V.hsys[kBarState] = SysState{};
-    V.hsys[kBarState].maxiter = barrier_polls();
     int rc;
     // (the ticket slots: a launch that gave up leaves its counters behind)
     MTGPU_TRY(cudaMemsetAsync(V.partials, 0, sizeof(float4) * kTicketSlots, V.st));
+    if (barrier_polls() != kBarPolls)
+        MTGPU_TRY(cudaMemsetAsync((unsigned int *)V.partials + kBarSlot, 0xff, sizeof(unsigned int), V.st));
     if ((rc = upload_sys(V))) return rc;
     to_rows(V, b_sys_major, V.b64);
     to_rows(V, x_sys_major, V.xacc);

@@ -28,8 +28,7 @@ struct SysState {
 };
 
 // The state slots: the systems' and one for the grid barrier of k_small, whose
-// status is set when a wait ran out (the host clears it) and whose maxiter
-// bounds the waits (0: the default)
+// status is set when a wait ran out (the host clears it)
 constexpr int kBarState = 32, kSysSlots = 33;
 
 // Iterations per group: p and x are needed by nothing in the iteration, so

@@ -36,8 +36,8 @@ namespace sv {
 // through ldg (ld.global after the barrier's acquire), never the read-only path.
 //
 // Every wait is bounded; one that runs out fails the solve with
-// MTGPU_ERR_TIMEOUT (GridBarrier; the mark and the bound are the state slot
-// after the systems').  The launch is cooperative, so all blocks are resident
+// MTGPU_ERR_TIMEOUT (GridBarrier; the mark is the state slot after the
+// systems').  The launch is cooperative, so all blocks are resident
 // and the waits end.
 constexpr int kSmallThreads = 480;     // threads with rows, at most; one warp more for the stop test
 constexpr int kSmallMin = 256;         // ... at least
@@ -218,10 +218,12 @@ __device__ __forceinline__ cdf small_row(const MF &M, int d, Pos p, int k, df om
     return kk.get();
 }
 
-// a / b (cquot_part) into a state's double and double-float forms
+// a component of a / b into a state's double and double-float forms.  (cquot_part
+// without its look at the range, which these sums of FP32 products cannot leave:
+// they lie between 2^-149 and 2^192; it took 0.5 us of a 17 us iteration)
 __device__ __forceinline__ void small_quot(double2 a, double2 b, int c, double2 &q, float4 &qf)
 {
-    const double v = cquot_part(a, b, c);
+    const double v = (c == 0 ? a.x * b.x + a.y * b.y : a.y * b.x - a.x * b.y) / (b.x * b.x + b.y * b.y);
     const df f = from_double(v);
     (c == 0 ? q.x : q.y) = v;
     (c == 0 ? qf.x : qf.y) = f.h;
@@ -251,8 +253,7 @@ k_small(const __grid_constant__ MF M, const __grid_constant__ SmallArgs A, int n
     unsigned int *tickets = reinterpret_cast<unsigned int *>(A.partials);
     double *part_e = reinterpret_cast<double *>(A.partials + kTicketSlots), *part_u = part_e + (size_t)B * 2 * SP,
            *part_r = part_u + (size_t)B * 4 * SP;
-    SysState *const bs = A.sys + kBarState;
-    GridBarrier bar{tickets + kBarSlot, &bs->status, bs->maxiter};
+    GridBarrier bar{tickets + kBarSlot};
     const df om = d2f(A.omega[k]);
 
     if (tid < SP) {
@@ -260,7 +261,7 @@ k_small(const __grid_constant__ MF M, const __grid_constant__ SmallArgs A, int n
         st[tid].cnt = 0;
         brk[tid] = 0;
     }
-    if (tid == 0) late = *(volatile const int *)&bs->status != 0;
+    if (tid == 0) late = *(volatile const int *)&A.sys[kBarState].status != 0;
     __syncthreads();
     if (late) return;                  // an earlier launch failed
     for (int u = 0; u < items; u++) {
@@ -343,7 +344,7 @@ k_small(const __grid_constant__ MF M, const __grid_constant__ SmallArgs A, int n
             S2::block(v, nw, sums, part_e);
         }
         bar.arrive();
-        if (!bar.wait(&late)) break;
+        if (!bar.wait(&late, &A.sys[kBarState].status, kBarPolls)) break;
         S2::totals(part_e, tot);
         if (tid < 2 * SP && st[k].status == kRun) {
             const double2 aw = make_double2(tot[0][k], tot[1][k]);
@@ -395,7 +396,7 @@ k_small(const __grid_constant__ MF M, const __grid_constant__ SmallArgs A, int n
             S4::block(v, nw, sums, part_u);
         }
         bar.arrive();
-        if (!bar.wait(&late)) break;
+        if (!bar.wait(&late, &A.sys[kBarState].status, kBarPolls)) break;
 
         // z = A s, (z, s); meanwhile the last warp adds the update's
         // sums and prepares the stop test
@@ -447,7 +448,7 @@ k_small(const __grid_constant__ MF M, const __grid_constant__ SmallArgs A, int n
             S2::block(v, nw, sums, part_r);
         }
         bar.arrive();
-        if (!bar.wait(&late)) break;
+        if (!bar.wait(&late, &A.sys[kBarState].status, kBarPolls)) break;
         S2::totals(part_r, tot);
         if (tid < 2 * SP && st[k].status == kRun)
             small_quot(make_double2(tot[0][k], tot[1][k]), st[k].zs, tid / SP, st[k].beta, st[k].beta_f);
