@@ -370,7 +370,7 @@ k_small64(const __grid_constant__ Small64 A, int n, int items)
 void small_grid(CocrSolver &S, int dev, int nsm)
 {
     S.g_small = 0;
-    if (S.nb < 1 || S.nb > (long long)nsm * kSmallThreads * kSmallItems) return;
+    if (S.nb < 1 || S.nb > (long long)nsm * kSmallThreads * kSmallItems || !one_kernel_wanted()) return;
     const int items = ceil_div(S.nb, nsm * kSmallThreads);
     const int nt = std::max(kSmallMin, ceil_div(ceil_div(S.nb, nsm * items), 32) * 32);
     const int smem = items * kSmallItemBytes * nt;

@@ -275,6 +275,17 @@ inline int barrier_polls()
     const int n = e ? atoi(e) : 0;
     return n > 0 ? n : kBarPolls;
 }
+// A one-kernel launch needs its blocks resident together, so small solves from
+// several threads follow one another where the separate kernels' overlap:
+// MTGPU_ONE_KERNEL=0 (environment, read when a solver is set up) is for programs
+// that run many.  Milliseconds a solve from 1, 2, 4, 8 threads, in one kernel and in
+// separate ones: 45,000 edges x 2 systems 7.3 6.9 6.8 6.7 and 8.9 5.5 3.6 3.5; 26,500 x 1 4.1
+// 3.6 3.6 3.6 and 6.3 3.3 1.9 1.3; FP64 on 45,000 8.9 8.8 8.7 8.7 and 14.2 8.5 6.1 4.8.
+inline bool one_kernel_wanted()
+{
+    const char *e = getenv("MTGPU_ONE_KERNEL");
+    return !(e && *e == '0');
+}
 // the total of output o of the blocks' partials part[output][block], from G
 // lanes of a warp (j: the lane among them), in all of them; 8 loads in flight
 template <int G>

@@ -2141,7 +2141,7 @@ struct Impl {
         const long long n = (long long)V.nb * SP;
         if (V.ch != kMatFree + 3 || !V.mf.on || !V.mf.gface || !V.g_lat || !V.G.d_tn) return;
         if (n > (long long)nsm * kSmallThreads * kSmallItems) return;
-        if (SP > kSmallSystems || !V.alone) return;
+        if (SP > kSmallSystems || !V.alone || !one_kernel_wanted()) return;
         if ((size_t)nsm * 8 * SP > 2 * (partial_slots(V.pblocks, SP) - kTicketSlots)) return;
         // as few rows per thread as fit, the rows even over the SMs
         const int items = (int)((n + (long long)nsm * kSmallThreads - 1) / ((long long)nsm * kSmallThreads));

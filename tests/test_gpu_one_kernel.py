@@ -56,3 +56,12 @@ def test_fp64(gpu, cells):
         assert n >= 4 * its
     else:
         assert n <= -(-its // 64) + 16
+
+
+def test_separate_kernels_on_request(gpu, monkeypatch):
+    """For programs that run many small solves from several threads."""
+    monkeypatch.setenv("MTGPU_ONE_KERNEL", "0")
+    n, groups = _survey_launches(gpu, (17, 16, 15), 5)
+    assert n >= 81 * groups
+    n, its = _fp64_launches(gpu, (14, 13, 12))
+    assert n >= 4 * its
