@@ -420,6 +420,18 @@ __device__ __forceinline__ cdf chalf(cdf x, float t) { return cdf{mul2(x.h, pk(t
 
 // ------------------------------------------------------------ set-up
 // the scalars that the row kernels read, in both forms
+// (a / b of these sums: cquot_part without its look at the range, which sums of
+// FP32 products, 2^-149 to 2^192 with their scaling, cannot leave; it took 0.5 us
+// of a 17 us one-kernel iteration and 0.4 of the separate kernels' 30)
+__device__ __forceinline__ double sum_quot_part(double2 a, double2 b, int c)
+{
+    const double d = b.x * b.x + b.y * b.y;
+    return (c == 0 ? a.x * b.x + a.y * b.y : a.y * b.x - a.x * b.y) / d;
+}
+__device__ __forceinline__ double2 sum_quot(double2 a, double2 b)
+{
+    return make_double2(sum_quot_part(a, b, 0), sum_quot_part(a, b, 1));
+}
 __device__ __forceinline__ void set_alpha(SysState &q, double2 v) { q.alpha = v; q.alpha_f = to4(from_d2(v)); }
 __device__ __forceinline__ void set_beta(SysState &q, double2 v) { q.beta = v; q.beta_f = to4(from_d2(v)); }
 __device__ __forceinline__ void set_mrs_w(SysState &q, double v)
@@ -499,7 +511,7 @@ __device__ __forceinline__ void finish_alpha(const tf (&v)[2], SysState *sys, fl
         if (status == kRun) {
             const double2 aw = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
             if (fabs(aw.x) < 1e-40 && fabs(aw.y) < 1e-40) q.status = MTGPU_DIV_BY_ZERO;
-            else set_alpha(q, cquot(zs, aw));
+            else set_alpha(q, sum_quot(zs, aw));
         }
     }
 }
@@ -721,7 +733,7 @@ struct SpmvTail {
             const double2 zs_new = make_double2(tot[0][threadIdx.x], tot[1][threadIdx.x]);
             q.zs = zs_new;
             if (mode == 0) return;
-            const double2 beta = cquot(zs_new, zs);
+            const double2 beta = sum_quot(zs_new, zs);
             const double residual = mrs == 0 ? res : (res2 > 0.0 ? sqrt(res2) : 0.0);
             const double rel = residual / r_old;
             set_beta(q, beta);

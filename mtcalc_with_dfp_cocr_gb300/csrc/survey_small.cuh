@@ -218,12 +218,10 @@ __device__ __forceinline__ cdf small_row(const MF &M, int d, Pos p, int k, df om
     return kk.get();
 }
 
-// a component of a / b into a state's double and double-float forms.  (cquot_part
-// without its look at the range, which these sums of FP32 products cannot leave:
-// they lie between 2^-149 and 2^192; it took 0.5 us of a 17 us iteration)
+// a component of a / b into a state's double and double-float forms
 __device__ __forceinline__ void small_quot(double2 a, double2 b, int c, double2 &q, float4 &qf)
 {
-    const double v = (c == 0 ? a.x * b.x + a.y * b.y : a.y * b.x - a.x * b.y) / (b.x * b.x + b.y * b.y);
+    const double v = sum_quot_part(a, b, c);
     const df f = from_double(v);
     (c == 0 ? q.x : q.y) = v;
     (c == 0 ? qf.x : qf.y) = f.h;
