@@ -56,14 +56,12 @@ UNIT = "s/solve"
 WORKLOAD = "c2"
 # DRAM bytes of one matrix-free SpMV on c2 (two lanes, as the iteration
 # launches it), per variant: the sum of its kernels' ncu dram__bytes_read.sum
-# + dram__bytes_write.sum (profiles/survey_iteration_kernels.md: variant 35's
-# k_mf_gmarch + k_mf_edges_g)
+# + dram__bytes_write.sum (variant 35's k_mf_gmarch + k_mf_edges_g)
 SPMV_MF_TRAFFIC_C2 = {35: 264.7e6}
 # what bounds the matrix-free SpMV instead of HBM (ncu on c2, two lanes)
 SPMV_MF_BINDING = {
     35: "FP32 arithmetic and load latency: k_mf_edges_g<2> FMA pipe 49 %, L1 77 %, 16 warps an SM "
-        "at 126 registers; k_mf_gmarch<2> FMA pipe 39 %, load latency "
-        "(profiles/survey_iteration_kernels.md)"}
+        "at 126 registers; k_mf_gmarch<2> FMA pipe 39 %, load latency"}
 
 
 def load_peaks():
@@ -316,7 +314,7 @@ def gpu_arm(args):
             spmv_kernel = f"k_mf_faces + {edges} (matrix-free double-float SpMV, S systems)"
         traffic = SPMV_MF_TRAFFIC_C2.get(variant) if WORKLOAD == "c2" else None
         traffic_src = (f"ncu dram__bytes_read.sum + dram__bytes_write.sum of the variant-{variant} "
-                       f"kernels on c2 (profiles/survey_iteration_kernels.md)") if traffic else None
+                       "kernels on c2") if traffic else None
     else:
         spmv_bytes = nc * (4 + 8 + 8) + nr * (4 + 8) + meta + 2 * S * 16 * nb + tail
         spmv_kernel = f"k_spmv variant {variant} (batched double-float SELL-32 SpMV, S systems)"

@@ -363,12 +363,12 @@ int mtgpu_survey_spmv(mtgpu_survey *s, const double *d_x, double *d_y);
  * available or nothing was timed). */
 int mtgpu_survey_tuning(const mtgpu_survey *s, int *variant, float *ms);
 /* The environment variable MTGPU_SPMV_VARIANT, when it names a variant
- * available for the survey, replaces the autotuning at mtgpu_survey_create
+ * available for the survey, replaces the set-up's choice at mtgpu_survey_create
  * (for profiler runs: a profiler serialises and cold-starts every launch, and
- * would make the autotuning choose differently from a plain run). */
+ * would make a timing choose differently from a plain run). */
 
 /* Pins the SpMV variant (0, 1, 2, 4, 8, 18, 20, 32, 33, 34 or 35) instead of the
- * autotuned choice.  The stored-matrix variants sum the same products in the
+ * set-up's choice.  The stored-matrix variants sum the same products in the
  * same order; the matrix-free one computes the same operator in another
  * order (it is enabled only where a set-up product agrees with the stored
  * matrix's to 1e-9).  MTGPU_ERR_ARG if the variant is unknown or unavailable

@@ -161,12 +161,13 @@ __global__ void k_adj_gather(int n_touch, int S, int nrec, long long nb,
 // a0_k on an edge: (h_d / 2) times the 1-D potential at the edge midpoint
 // times (alfa, 1 - alfa, 0), as in the right-hand side assembly.
 //
-// Bound by GB300's FP64 pipe: C's rows are (h_t1 h_t2 / h_d) / 9 times
-// 4 u_i + 2 (u_a + u_b) + u_d (a, b the neighbours of edge i along the
-// transverse axes, d the opposite edge), and only Im t is needed, 29
-// operations a direction; the table intervals of the edge midpoints are
-// looked up once per cell instead of once per system, table and edge.
-// 73,728 cells x 16 systems: 1,420 -> 330 us.
+// C's rows are (h_t1 h_t2 / h_d) / 9 times 4 u_i + 2 (u_a + u_b) + u_d (a, b
+// the neighbours of edge i along the transverse axes, d the opposite edge),
+// and only Im t is needed, 29 FP64 operations a direction; the table
+// intervals of the edge midpoints are looked up once per cell instead of
+// once per system, table and edge.  73,728 cells x 16 systems: 1,420 -> 330 us, of
+// which the FP64 operations are 165; the rest is the latency of the 24
+// gathers of one system after the other.
 __global__ void __launch_bounds__(128)
 k_adj_grad(int kpar, int S, long long nb, const double2 *__restrict__ u,
            const double2 *__restrict__ lam, const double *__restrict__ omega,

@@ -70,8 +70,7 @@ struct mtgpu_assembly_s {
     std::vector<double> sigflag;
     std::vector<int> ig_t;
     int nver_stride = 14;
-    // the SpMV variant the first survey set-up on this mesh chose, per batch
-    // width (lanes): the choice depends on the mesh and the width only, so
-    // later surveys on the assembly skip the autotuning
+    // the SpMV variant that a survey set-up's timing on this mesh chose, per
+    // batch width (lanes); later set-ups that would time use it instead
     std::map<int, int> tuned;
 };

@@ -1358,7 +1358,7 @@ int survey_setup(const ParamMatrix &P, const mtgpu_mesh_desc &mesh, int S, const
     // matrix-free operator; with one they are built only on request
     if (!V.mf.on && (rc = survey_prepare_variant(V, 0))) return rc;
     trace.mark("SpMV tiles");
-    // autotune the SpMV variant: time each candidate, keep the fastest.
+    // the SpMV variant: by rule (below), a kept timing, or timing each candidate.
     // MTGPU_SPMV_VARIANT (environment) pins an available variant instead:
     // runs under a profiler, which serialises and cold-starts every launch,
     // would otherwise tune to other variants than plain runs do

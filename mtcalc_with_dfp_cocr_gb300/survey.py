@@ -104,7 +104,7 @@ class Survey:
     def set_spmv_variant(self, variant):
         """Pin the SpMV variant (0 x and matrix staged, 1 x staged, 2, 4, 8
         slots in flight, 18, 20 row per thread for two systems, 32-35
-        matrix-free) instead of the autotuned one."""
+        matrix-free) instead of the set-up's choice."""
         _lib.check(_lib.lib().mtgpu_survey_set_spmv_variant(self._h, int(variant)),
                    "mtgpu_survey_set_spmv_variant")
 
